@@ -528,7 +528,7 @@ velo_status stage_impl(velo_ctx* c, const uint8_t* buf, const uint64_t* offsets,
   if ((st = ensure(c, c->d_ev_valid, 4ull * n, "valid")) != VELO_OK) return st;
   if ((st = ensure(c, c->d_hit_base, 8ull * n, "hit_base")) != VELO_OK) return st;
   if ((st = ensure(c, c->d_tracklets, 16ull * rows, "tracklets")) != VELO_OK) return st;
-  if ((st = ensure(c, c->d_rings, 32ull * rows, "rings")) != VELO_OK) return st;
+  if ((st = ensure(c, c->d_rings, 64ull * rows, "rings")) != VELO_OK) return st;
   if ((st = ensure(c, c->d_weak, 4ull * rows, "weak")) != VELO_OK) return st;
   if ((st = ensure(c, c->d_tracks, sizeof(velo_track) * rows, "tracks")) != VELO_OK) return st;
   if ((st = ensure(c, c->d_out_tracks, sizeof(velo_track) * rows, "out_tracks")) != VELO_OK) return st;
@@ -1054,12 +1054,12 @@ velo_status search_pipelined(velo_ctx* c, const uint8_t* buf, const uint64_t* of
 namespace {
 
 // Upper bound of the device bytes one event takes in a staged batch, from its
-// blob size alone (H <= (size - 8) / 16): per hit row 152 B of scratch
+// blob size alone (H <= (size - 8) / 16): per hit row 184 B of scratch
 // (tracklet, rings, weak, working track), 100 B of output and 21 B of arena,
 // plus the blob itself and its metadata.
 uint64_t event_device_bytes(uint64_t size) {
   const uint64_t rows = std::max<uint64_t>(size >= 8 ? (size - 8) / 16 : 0, 1);
-  return rows * (152 + 100 + 21) + size + 64;
+  return rows * (184 + 100 + 21) + size + 64;
 }
 
 // Events per part when the batch would not fit the device budget, else 0.

@@ -112,9 +112,8 @@ struct SearchParams {
   // global scratch
   uint8_t* global_arena;
   uint32_t* tracklets;            // 4 words per tracklet {h0, h1, h2, 0}, row hit_base[e]
-  uint32_t* rings;                // 8 words per row: the two tracks-to-follow rings of event e
-                                  // (max(H, 1) entries each) from row hit_base[e], entries
-                                  // {entry word, first hit, previous hit, last hit}
+  uint32_t* rings;                // 16 words per row: the two tracks-to-follow rings of event e
+                                  // (max(H, 1) entries of 32 bytes each) from row hit_base[e]
   uint32_t* weak;                 // weak-track list, row hit_base[e]
   velo_track* tracks;             // working tracks, row hit_base[e]
   // outputs

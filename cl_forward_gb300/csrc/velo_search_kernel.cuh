@@ -52,6 +52,8 @@
 #include <float.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "velo_internal.h"
 #include "velo_mlp_warp.cuh"
 #include "velo_partition.cuh"
@@ -65,19 +67,40 @@ __device__ __forceinline__ float fdiv(float a, float b) { return __fdiv_rn(a, b)
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr uint32_t kNone16 = 0xffffu;
+// Per-hit flag byte.  kUsed: the reference's hit_used.  kDead (set once per
+// event, only where the pair seeding runs): the hit as an h1 has no h2 window.
+constexpr uint8_t kUsed = 1, kDead = 2;
+// Per-module flags: its hits are x-sorted; its dead h1s are its last hits.
+constexpr uint8_t kSorted = 1, kDeadTail = 2;
+
+// Pair seeding (seed_pairs), per CTA: the h0s being seeded, 32 at a time, and
+// the occupancy map of the h2 module.
+constexpr int kMapRows = 64;          // 64 rows x 32 columns of cells
+constexpr int kQueue = 32;            // pairs a warp holds for the exact fits
+template <int kWarps>
+struct SeedShared {
+  float4 h0[32];                      // x, y, z, first h1 - first pair (int bits)
+  float2 reach[32];                   // the h0's y cut, and (z2 - z0) / (z1 - z0) where the map is valid
+  unsigned long long best[32];        // the h0's best (fit, Y-lane, h1, h2) so far
+  uint32_t map[2][kMapRows];          // by parity of the module being seeded
+  // owner << 14 | h1 in its module; of 32 h0s, 16 warps have at most 2 each
+  std::conditional_t<(kWarps > 8), uint16_t, uint32_t> queue[kWarps][kQueue];
+  uint16_t active[32];                // unused h0s of the block, by rank
+  uint16_t first[32];                 // the h0's first h1 in its module
+};
 
 // Per-CTA shared state for events of up to kMods modules.  Launches whose
 // events all have at most kCompactModules - 1 modules (every VELO geometry)
 // use the compact form: 4 KB less static shared memory per CTA, which goes
 // to L1 and to more resident CTAs.
-template <int kMods>
+template <int kMods, int kWarps>
 struct SharedT {
   int32_t start[kMods];
   int32_t num[kMods];
   int32_t sz[kMods];
   float zmin[kMods];
   float zmax[kMods];
-  uint8_t sorted[kMods];
+  uint8_t flags[kMods];   // kSorted, kDeadTail
   uint32_t ring_lo[2];   // forwarding entries, from the front of ring[i]
   uint32_t ring_hi[2];   // seeding entries, from the back of ring[i]
   uint32_t ntracks, ntracklets, nweak, status;
@@ -85,6 +108,7 @@ struct SharedT {
   unsigned long long out_first;
   int32_t next_event;
   int32_t seed_next[2];  // G < 32: next unclaimed h0 of the module being seeded, by ring parity
+  SeedShared<kWarps> seed;
 };
 
 struct EventView {
@@ -100,12 +124,12 @@ struct EventView {
   __device__ __forceinline__ float* zs() const { return reinterpret_cast<float*>(arena + 2u * P); }
   __device__ __forceinline__ uint2* wins() const { return reinterpret_cast<uint2*>(arena + 3u * P); }
   __device__ __forceinline__ uint8_t* useds() const { return arena + 5u * P; }
-  uint4* ring0;             // tracks-to-follow buffers, selected by parity:
-  uint4* ring1;             //   {entry word, first hit, previous hit, last hit}
+  uint4* rings;             // tracks-to-follow buffers: entry words of buffer 0 and 1, then their lines
   uint4* tracklets;         // {h0, h1, h2, 0} per tracklet
   uint32_t* weak;
   velo_track* tracks;
   bool narrow;
+  bool tame;                // every module x-sorted and every coordinate within kMaxCoordinate
   int event;
   const MlpFrag* mlp;       // learned seeding: weights in shared memory
   float keep_threshold, window_margin;
@@ -178,7 +202,7 @@ __device__ void compute_windows(const EventView& ev, const Shared& s, int h, int
   const float x0 = ev.xs()[h], z0 = ev.zs()[h];
   const float* x2 = ev.xs() + st2;
   const float* z2 = ev.zs() + st2;
-  const bool sorted = ev.narrow && s.sorted[s2];
+  const bool sorted = ev.narrow && (s.flags[s2] & kSorted);
   uint32_t r1f = kNone16, r1l = kNone16, r2f = kNone16, r2l = kNone16;
 
   // h1 window: first hit with |x1-x0| < 0.7|z1-z0|, then the first later hit
@@ -285,27 +309,59 @@ __device__ __forceinline__ uint32_t warp_reserve(uint32_t* counter, bool take) {
   return base + (uint32_t)__popc(m & lanemask_lt());
 }
 
-// (a select, not an indexed array, so the view stays in registers)
-__device__ __forceinline__ uint4* ring_buf(const EventView& ev, int b) { return b ? ev.ring1 : ev.ring0; }
+// Entry i of buffer b is a pair of 16-byte halves in two arrays: {entry word,
+// last hit, z of the previous hit, z of the last hit} and the line through
+// the last two hits {x and y of the previous hit, x and y slopes}.  The line
+// is computed when the hit is found, so an entry that finds nothing is passed
+// on as it is, and forwarding reads no hit, track or tracklet before its fit.
+__device__ __forceinline__ uint4* ring_words(const EventView& ev, int b) { return ev.rings + (size_t)b * ev.ring_cap; }
+__device__ __forceinline__ float4* ring_lines(const EventView& ev, int b) {
+  return reinterpret_cast<float4*>(ev.rings + (size_t)(2 + b) * ev.ring_cap);
+}
 
-// A ring entry carries the track's last two hits (and a tracklet's first), so
-// forwarding extrapolates without reading the track or tracklet row first.
+// The line through hit a and then hit b (z differing), as the reference
+// takes it from a track's last two hits (Kernel.cl:253-257).  td = 1 / (zb - za).
+__device__ __forceinline__ float4 line_through(float xa, float ya, float xb, float yb, float td) {
+  return make_float4(xa, ya, fmul(fsub(xb, xa), td), fmul(fsub(yb, ya), td));
+}
+
+// Writes a new tracklet's entry {h0, h1, h2} to slot i of buffer b.
+__device__ __forceinline__ void write_tracklet_entry(const EventView& ev, int b, uint32_t i, uint32_t tp, uint32_t h1,
+                                                     uint32_t h2) {
+  const float z1 = ev.zs()[h1], z2 = ev.zs()[h2];
+  const float td = fdiv(1.0f, fsub(z2, z1));
+  ring_words(ev, b)[i] = make_uint4(kTrackletFlag | tp, h2, __float_as_uint(z1), __float_as_uint(z2));
+  ring_lines(ev, b)[i] = line_through(ev.xs()[h1], ev.ys()[h1], ev.xs()[h2], ev.ys()[h2], td);
+}
+
+// A seeding warp's new tracklet goes to the back of buffer b.
 template <class Shared>
-__device__ __forceinline__ void push_back(Shared& s, const EventView& ev, int b, uint4 v) {
+__device__ __forceinline__ void push_back(Shared& s, const EventView& ev, int b, uint32_t tp, uint32_t h1,
+                                          uint32_t h2) {
   const uint32_t i = atomicAdd(&s.ring_hi[b], 1u);
-  if (i < ev.ring_cap) ring_buf(ev, b)[ev.ring_cap - 1u - i] = v;
+  if (i < ev.ring_cap) write_tracklet_entry(ev, b, ev.ring_cap - 1u - i, tp, h1, h2);
 }
 
-// i-th entry of ring[b]: the front segment, then the back segment.
-__device__ __forceinline__ uint4 ring_entry(const EventView& ev, int b, uint32_t lo, uint32_t i) {
-  const uint4* r = ring_buf(ev, b);
-  return i < lo ? r[i] : r[ev.ring_cap - 1u - (i - lo)];
+// Index of the i-th entry of a buffer: the front segment, then the back segment.
+__device__ __forceinline__ uint32_t ring_index(const EventView& ev, uint32_t lo, uint32_t i) {
+  return i < lo ? i : ev.ring_cap - 1u - (i - lo);
 }
+
+// The scatter cut (dx^2 + dy^2) / dz^2 < kMaxScatter bounds |dx| and |dy| by
+// sqrt(kMaxScatter) |dz| = 0.004 |dz|; 1 % more covers the rounding of the
+// reference's products.  At the usual 25 mm between modules that is 0.1 mm,
+// a sixth of kTolerance, so far fewer hits are tried.
+constexpr float kScatterReach = 0.00404f;
+// With |dz| at least this, 1 / dz squared stays far from overflow, so a fit
+// outside the cuts is finite and need not be evaluated.
+constexpr float kMinDz = 1e-3f;
+// Events within this of the origin (mm) take the pair seeding.
+constexpr float kMaxCoordinate = 1e4f;
 
 // Track forwarding onto module m4 (Kernel.cl:210-367), one warp at a time:
-// lane j forwards entry i0 + j of ring[b].  Track numbers, ring slots and
+// lane j forwards entry i0 + j of buffer b.  Track numbers, ring slots and
 // weak slots are reserved with one atomic per warp; new entries go to the
-// front of ring[nb].
+// front of buffer nb.
 template <class Shared>
 __device__ void forward_warp(const EventView& ev, Shared& s, int b, uint32_t lo_n, uint32_t i0, uint32_t ncur,
                              int m4, int nb) {
@@ -314,37 +370,54 @@ __device__ void forward_warp(const EventView& ev, Shared& s, int b, uint32_t lo_
   int action = kNone;
   uint32_t push_value = 0, trackno = 0, best_h2 = 0;
   uint4 en = make_uint4(0, 0, 0, 0);
+  float4 line = make_float4(0.f, 0.f, 0.f, 0.f);
+  float best_z = 0.f, best_den = 0.f;
   // the ends of module m4 for the narrowing, loaded alongside the entry
   // (same addresses in every lane)
   const int st4 = s.start[m4], n4 = s.num[m4];
+  const float zmin4 = s.zmin[m4], zmax4 = s.zmax[m4];
+  const bool single4 = zmin4 == zmax4;   // one z on the module
+  const bool narrow4 = ev.narrow && (s.flags[m4] & kSorted) && n4 > 0;
   const float* x4 = ev.xs() + st4;
+  const float* y4 = ev.ys() + st4;
+  const float* z4 = ev.zs() + st4;
   float x4_first = 0.f, x4_last = 0.f;
   if (n4 > 0) {
     x4_first = x4[0];
     x4_last = x4[n4 - 1];
   }
   if (i < ncur) {
-    en = ring_entry(ev, b, lo_n, i);
+    const uint32_t at = ring_index(ev, lo_n, i);
+    en = ring_words(ev, b)[at];
+    line = ring_lines(ev, b)[at];
     const uint32_t full = en.x;
     const bool is_tracklet = (full & kTrackletFlag) != 0;
     const uint32_t skipped = (full & kSkipMask) >> 28;
     trackno = full & kEntryNumber;
     const uint32_t n = is_tracklet ? 3u : (full >> kEntryCountShift) & 31u;
-    const uint32_t h0 = en.z, h1 = en.w;   // the last two hits
-    const float h0x = ev.xs()[h0], h0y = ev.ys()[h0], h0z = ev.zs()[h0];
-    const float h1x = ev.xs()[h1], h1y = ev.ys()[h1], h1z = ev.zs()[h1];
-    const float td = fdiv(1.0f, fsub(h1z, h0z));
-    const float tx = fmul(fsub(h1x, h0x), td);
-    const float ty = fmul(fsub(h1y, h0y), td);
-
-    const float* y4 = ev.ys() + st4;
-    const float* z4 = ev.zs() + st4;
-    int lo = 0, hi = n4;
-    if (ev.narrow && s.sorted[m4] && n4 > 0) {
-      const float xa = fadd(h0x, fmul(tx, fsub(s.zmin[m4], h0z)));
-      const float xb = fadd(h0x, fmul(tx, fsub(s.zmax[m4], h0z)));
-      if (isfinite(xa) && isfinite(xb))
-        narrow_range_ends(x4, 0, n4, x4_first, x4_last, fminf(xa, xb), fmaxf(xa, xb), kTolerance, &lo, &hi);
+    const float h0z = __uint_as_float(en.z), h1z = __uint_as_float(en.w);
+    int k = 0;
+    float ht = __int_as_float(0x7f800000);   // +inf: every hit from k on is tried
+    bool all_fits = true;                    // every fit is evaluated, for its finiteness
+    if (narrow4) {
+      const float dza = fsub(zmin4, h0z), dzb = fsub(zmax4, h0z);
+      const float xa = fadd(line.x, fmul(line.z, dza));
+      const float xb = single4 ? xa : fadd(line.x, fmul(line.z, dzb));
+      const float d_lo = fsub(zmin4, h1z), d_hi = fsub(zmax4, h1z);
+      const float reach = fmul(kScatterReach, fmaxf(fabsf(d_lo), fabsf(d_hi)));
+      const float ymax = fadd(fabsf(line.y), fmul(fabsf(line.w), fmaxf(fabsf(dza), fabsf(dzb))));
+      // the fits outside the cuts are known to be finite
+      const bool tame = ev.tame && (d_lo > kMinDz || d_hi < -kMinDz) && ymax < 1e15f;
+      const float tol = tame ? fminf(kTolerance, reach) : kTolerance;
+      const float xl = fminf(xa, xb), xh = fmaxf(xa, xb);
+      const float margin = fadd(0.01f, fmul(1e-5f, fadd(fabsf(xl), fabsf(xh))));
+      const float lt = fsub(fsub(xl, tol), margin);
+      const float h = fadd(fadd(xh, tol), margin);
+      if (isfinite(xa) && isfinite(xb) && isfinite(lt) && isfinite(h)) {
+        ht = h;
+        all_fits = !tame;
+        k = x4_last <= lt || x4_first > ht ? n4 : first_gt(x4, 0, n4, lt);
+      }
     }
     // fitHitToTrack (Kernel.cl:15-35) over the candidates, first minimum wins.
     // The scatter's 1/(z2 - z1) depends only on z2 here: it is recomputed only
@@ -354,20 +427,25 @@ __device__ void forward_warp(const EventView& ev, Shared& s, int b, uint32_t lo_
     bool degenerate = false;
     uint32_t zc = 0x7fc00001u;   // bit pattern of the z2 the cached factor belongs to (none yet)
     float den = 0.f;
-    for (int k = lo; k < hi; ++k) {
-      const float h2z = z4[k];
-      if (__float_as_uint(h2z) != zc) {
-        zc = __float_as_uint(h2z);
-        den = fdiv(1.f, fsub(h2z, h1z));
-      }
+    for (; k < n4; ++k) {
+      const float h2x = x4[k];
+      if (h2x > ht) break;
+      const float h2z = single4 ? zmin4 : z4[k];
       const float dz = fsub(h2z, h0z);
-      const float dx = fabsf(fsub(fadd(h0x, fmul(tx, dz)), x4[k]));
-      const float dy = fabsf(fsub(fadd(h0y, fmul(ty, dz)), y4[k]));
-      const float scatter = fmul(fmul(fadd(fmul(dx, dx), fmul(dy, dy)), den), den);
-      if (dx < kTolerance && dy < kTolerance && scatter < kMaxScatter) {
-        if (scatter < best) { best = scatter; best_k = k; }
-      } else if (!isfinite(scatter)) {
-        degenerate = true;   // the reference's `condition*scatter + !condition*MAX` is NaN here
+      const float dx = fabsf(fsub(fadd(line.x, fmul(line.z, dz)), h2x));
+      const float dy = fabsf(fsub(fadd(line.y, fmul(line.w, dz)), y4[k]));
+      const bool near = dx < kTolerance && dy < kTolerance;
+      if (near || all_fits) {
+        if (__float_as_uint(h2z) != zc) {
+          zc = __float_as_uint(h2z);
+          den = fdiv(1.f, fsub(h2z, h1z));
+        }
+        const float scatter = fmul(fmul(fadd(fmul(dx, dx), fmul(dy, dy)), den), den);
+        if (near && scatter < kMaxScatter) {
+          if (scatter < best) { best = scatter; best_k = k; best_z = h2z; best_den = den; }
+        } else if (!isfinite(scatter)) {
+          degenerate = true;   // the reference's `condition*scatter + !condition*MAX` is NaN here
+        }
       }
     }
     if (degenerate) atomicOr(&s.status, VELO_EVENT_DEGENERATE);
@@ -378,10 +456,11 @@ __device__ void forward_warp(const EventView& ev, Shared& s, int b, uint32_t lo_
         atomicOr(&s.status, VELO_EVENT_TRACK_OVERFLOW);
       } else {
         ev.useds()[best_h2] = 1;
+        // the entry's next line: through its last hit and the one found, whose
+        // 1 / (z2 - z1) is the fit's own
+        const float h1x = ev.xs()[en.y], h1y = ev.ys()[en.y];
+        line = line_through(h1x, h1y, x4[best_k], y4[best_k], best_den);
         if (is_tracklet) {   // third -> fourth hit: a track is allocated below; hits 0-2 marked
-          ev.useds()[en.y] = 1;
-          ev.useds()[en.z] = 1;
-          ev.useds()[en.w] = 1;
           action = kNewTrack;
         } else {
           velo_track& t = ev.tracks[trackno];
@@ -398,14 +477,17 @@ __device__ void forward_warp(const EventView& ev, Shared& s, int b, uint32_t lo_
       action = kWeak;
     }
   }
-  // new tracks (Kernel.cl:324-337)
+  // new tracks (Kernel.cl:324-337); the words past the last hit are cleared
+  // when the track is written out
   const uint32_t tn = warp_reserve(&s.ntracks, action == kNewTrack);
   if (action == kNewTrack) {
+    const uint4 tl = ev.tracklets[trackno];
+    ev.useds()[tl.x] = 1;
+    ev.useds()[tl.y] = 1;
+    ev.useds()[tl.z] = 1;
     if (tn < ev.cap) {
       uint32_t* w = reinterpret_cast<uint32_t*>(&ev.tracks[tn]);
-      w[0] = 4; w[1] = en.y; w[2] = en.z; w[3] = en.w; w[4] = best_h2;
-#pragma unroll
-      for (int k = 5; k < 25; ++k) w[k] = 0;
+      w[0] = 4; w[1] = tl.x; w[2] = tl.y; w[3] = tl.z; w[4] = best_h2;
       push_value = tn | (4u << kEntryCountShift);
     } else {
       action = kNone;
@@ -414,9 +496,11 @@ __device__ void forward_warp(const EventView& ev, Shared& s, int b, uint32_t lo_
   // tracks to follow in the next iteration (Kernel.cl:344-355)
   const bool push = action == kPushTrack || action == kNewTrack || action == kPushSkip;
   const uint32_t slot = warp_reserve(&s.ring_lo[nb], push);
-  if (push && slot < ev.ring_cap)   // a skip keeps the hits; a new hit shifts them
-    ring_buf(ev, nb)[slot] = action == kPushSkip ? make_uint4(push_value, en.y, en.z, en.w)
-                                                 : make_uint4(push_value, 0u, en.w, best_h2);
+  if (push && slot < ev.ring_cap) {   // a skip keeps the hits; a new hit shifts them
+    ring_words(ev, nb)[slot] = action == kPushSkip ? make_uint4(push_value, en.y, en.z, en.w)
+                                                   : make_uint4(push_value, best_h2, en.w, __float_as_uint(best_z));
+    ring_lines(ev, nb)[slot] = line;
+  }
   // three-hit tracklets that ran out of skips (Kernel.cl:359-363)
   const uint32_t wi = warp_reserve(&s.nweak, action == kWeak);
   if (action == kWeak && wi < ev.cap) ev.weak[wi] = trackno;
@@ -523,7 +607,7 @@ __device__ void seed_module(const EventView& ev, Shared& s, int f, int nb, const
   const uint32_t Y = (uint32_t)ev.Y;
   const uint32_t chunk_step = G == 32 ? 32u % Y : 0u;   // how far the Y-lanes turn per chunk
   const float s1_z = s.num[s1] > 0 ? ev.zs()[st1] : 0.f;   // Kernel.cl:420
-  const bool narrow4 = ev.narrow && s.sorted[m4] && n4 > 0;
+  const bool narrow4 = ev.narrow && (s.flags[m4] & kSorted) && n4 > 0;
   const float zmin4 = s.zmin[m4], zmax4 = s.zmax[m4];
   const float* x4 = ev.xs() + st4;
   const float* y4 = ev.ys() + st4;
@@ -548,7 +632,7 @@ __device__ void seed_module(const EventView& ev, Shared& s, int f, int nb, const
     uint32_t f1;
     if constexpr (G == 32) {
       h0 = st0 + ib;
-      if (ev.useds()[h0]) break;                        // warp-uniform
+      if (ev.useds()[h0] & kUsed) break;                // warp-uniform
       const uint32_t w0 = ev.wins()[h0].x;
       f1 = w0 & 0xffffu;
       if (f1 == kNone16) break;
@@ -558,7 +642,7 @@ __device__ void seed_module(const EventView& ev, Shared& s, int f, int nb, const
       h0 = st0 + ib + (lane >> kShift);
       n1 = 0;
       f1 = 0;
-      if (h0 < st0 + n0 && !ev.useds()[h0]) {
+      if (h0 < st0 + n0 && !(ev.useds()[h0] & kUsed)) {
         const uint32_t w0 = ev.wins()[h0].x;
         f1 = w0 & 0xffffu;
         if (f1 != kNone16) n1 = (int)(w0 >> 16) - (int)f1;
@@ -592,7 +676,7 @@ __device__ void seed_module(const EventView& ev, Shared& s, int f, int nb, const
       float h1x = 0.f, h1y = 0.f, h1z = 0.f;
       if (in) {
         w1 = ev.wins()[h1].y;
-        u1 = ev.useds()[h1];
+        u1 = ev.useds()[h1] & kUsed;
         h1x = ev.xs()[h1];
         h1y = ev.ys()[h1];
         h1z = ev.zs()[h1];
@@ -728,7 +812,7 @@ __device__ void seed_module(const EventView& ev, Shared& s, int f, int nb, const
         const uint32_t tp = atomicAdd(&s.ntracklets, 1u);
         if (tp < ev.cap) {
           ev.tracklets[tp] = make_uint4((uint32_t)h0, h1, h2, 0u);
-          push_back(s, ev, nb, make_uint4(kTrackletFlag | tp, (uint32_t)h0, h1, h2));
+          push_back(s, ev, nb, tp, h1, h2);
         }
       }
     } else {   // one shared-memory atomic per warp for the tracklet rows, one for the ring
@@ -741,8 +825,7 @@ __device__ void seed_module(const EventView& ev, Shared& s, int f, int nb, const
         const uint32_t h1 = (uint32_t)(st1 + (int)f1) + e;
         const uint32_t h2 = (uint32_t)st4 + (uint32_t)(best & 0x3fffu);
         ev.tracklets[tp] = make_uint4((uint32_t)h0, h1, h2, 0u);
-        if (ri < ev.ring_cap)
-          ring_buf(ev, nb)[ev.ring_cap - 1u - ri] = make_uint4(kTrackletFlag | tp, (uint32_t)h0, h1, h2);
+        if (ri < ev.ring_cap) write_tracklet_entry(ev, nb, ev.ring_cap - 1u - ri, tp, h1, h2);
       }
     }
     } while (0);
@@ -754,6 +837,339 @@ __device__ void seed_module(const EventView& ev, Shared& s, int f, int nb, const
     }
   }
   if (degenerate) atomicOr(&s.status, VELO_EVENT_DEGENERATE);
+}
+
+// seed_module for the events that the pair seeding does not take, out of
+// line, so that the module loop keeps its registers.
+template <int kMode, int G, class Shared>
+__device__ __noinline__ void seed_windows(const EventView ev, Shared& s, int f, int nb) {
+  seed_module<kMode, G>(ev, s, f, nb, seed_lanes_of(G, (uint32_t)ev.Y));
+}
+
+// The candidate windows of every hit (all threads of the CTA).
+template <class Shared>
+__device__ __noinline__ void fill_windows(const EventView ev, const Shared& s) {
+  // windows of modules 0..3 stay empty (Kernel.cl:104 gates the body on f >= 4)
+  const int hbeg = ev.S >= 5 ? s.start[4] : ev.H;
+  for (int i = threadIdx.x; i < hbeg; i += blockDim.x) ev.wins()[i] = make_uint2(0xffffffffu, 0xffffffffu);
+  for (int h = hbeg + threadIdx.x; h < ev.H; h += blockDim.x) {
+    int lo = 4, hi = ev.S - 1;   // last module whose start is <= h
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (s.start[mid] <= h) lo = mid; else hi = mid - 1;
+    }
+    compute_windows(ev, s, h, lo);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Pair seeding: the seeding of module f (h0 on f, h1 on f-2, h2 on f-4;
+// Kernel.cl:392-568 with the gather of :720-764) for events whose modules are
+// all x-sorted and whose coordinates are tame, with the results of
+// seed_module.
+//
+// Of a module's hits few are still unused when it is seeded (4 of 24 at the
+// ordinary pile-up), each with some 35 h1 candidates, of which one pair in 20
+// meets a hit of f-4.  So the unused h0s are gathered first, a warp lays the
+// (h0, h1) pairs of its h0s end to end over its lanes, whatever the h0s'
+// window lengths, and each pair only looks up the cell of its predicted
+// (x, y) in a map of the cells that f-4's hits could be met from.  The pairs
+// that pass are queued in shared memory and fitted 32 at a time.
+//
+// Measured against a group of 8 lanes per h0 walking its chunk of h1s and
+// searching h2 for every pair (seed_module): 10,000 events of 1,160 hits 3.27
+// -> 2.50 ms, 4,000 events of 4,550 hits 24.1 -> 7.4 ms.
+//
+// The windows need no table.  An h0's h1 window is bisected when the h0 is
+// seeded (most hits never are); whether an h1 has an h2 window is the flag
+// kDead; the h2 window itself is only tested on an h2 that passed the cuts.
+constexpr float kCellInv = 1.f / 1.3125f;   // cells of 1.3 mm: 32 columns span half a module's width, 64 rows its height
+
+__device__ __forceinline__ int map_cell(float v) { return __float2int_rd(fmul(v, kCellInv)); }
+
+// The map of module m4 answers for pairs whose h1 is on module s1: all hits
+// of either module at one z, so that the predicted point is the fit's own,
+// and the two z far enough apart for every fit to be finite.
+template <class Shared>
+__device__ __forceinline__ bool map_valid(const Shared& s, int s1, int m4) {
+  return s.zmin[m4] == s.zmax[m4] && s.zmin[s1] == s.zmax[s1] && fabsf(fsub(s.zmin[m4], s.zmin[s1])) > kMinDz;
+}
+
+// Marks the cells from which hit i of module m4 could be met: a pair whose
+// fit passes lies within 0.004 |z2 - z1| of it, and within kTolerance.  A
+// cell index is non-decreasing in the coordinate, so the cells of both ends
+// of the reach bracket the pair's; 0.01 mm covers the rounding.  Indices wrap
+// around, which can only let a pair through.
+template <class Shared>
+__device__ __forceinline__ void mark_map(const EventView& ev, const Shared& s, uint32_t* map, int s1, int m4, int i) {
+  const float dz = fabsf(fsub(s.zmin[m4], s.zmin[s1]));
+  const float reach = fadd(fminf(kTolerance, fmul(kScatterReach, dz)), 0.01f);
+  const float x = ev.xs()[s.start[m4] + i], y = ev.ys()[s.start[m4] + i];
+  uint32_t bits = 0;
+  for (int c = map_cell(fsub(x, reach)); c <= map_cell(fadd(x, reach)); ++c) bits |= 1u << (c & 31);
+  for (int r = map_cell(fsub(y, reach)); r <= map_cell(fadd(y, reach)); ++r) atomicOr(&map[r & (kMapRows - 1)], bits);
+}
+
+// The bounds of an h1's h2 window (Kernel.cl:85-102) for h1 at (x, z) on
+// module s1: the window is the first hit of f-4 above *lo, up to the first
+// later one above *hi.
+__device__ __forceinline__ void h2_bounds(float x, float z, int sz0, int sz2, float* lo, float* hi) {
+  const float fz0 = __int2float_rn(sz0), fz2 = __int2float_rn(sz2);
+  const float dxmax = fmul(kMaxXSlopeCandidates, fabsf(fsub(z, fz0)));
+  const float x_min = fsub(x, dxmax), x_max = fadd(x, dxmax);
+  const float z2_tz = fdiv(fsub(fz2, fz0), fsub(z, fz0));
+  *lo = fsub(fadd(x_max, fmul(fsub(x, x_max), z2_tz)), kToleranceCandidates);
+  *hi = fadd(fadd(x_min, fmul(fsub(x, x_min), z2_tz)), kToleranceCandidates);
+}
+
+// An h1 of module m has no h2 window: no hit of module m-2 lies above its
+// lower bound (modules 0-3 and the last two have no windows at all,
+// Kernel.cl:104,137).
+template <class Shared>
+__device__ __forceinline__ bool h1_dead(const EventView& ev, const Shared& s, int m, int h) {
+  if (m < 4 || m > ev.S - 3 || s.num[m - 2] == 0) return true;
+  float lo, hi;
+  h2_bounds(ev.xs()[h], ev.zs()[h], s.sz[m + 2], s.sz[m - 2], &lo, &hi);
+  return !(ev.xs()[s.start[m - 2] + s.num[m - 2] - 1] > lo);
+}
+
+// The h1 window of an h0 at (x0, z0) on x-sorted module s1: the first hit
+// with |x1 - x0| < 0.7 |z1 - z0| and the first later one that fails it
+// (Kernel.cl:115-135,161-165).  With one z on the module the passing hits
+// are a contiguous range, bisected at both ends at once.
+template <class Shared>
+__device__ __forceinline__ void h1_window(const EventView& ev, const Shared& s, int s1, float x0, float z0,
+                                          int* first, int* last) {
+  const int st = s.start[s1], n = s.num[s1];
+  const float* x = ev.xs() + st;
+  if (s.zmin[s1] == s.zmax[s1]) {
+    const float dxmax = fmul(kMaxXSlopeCandidates, fabsf(fsub(s.zmin[s1], z0)));
+    int a = 0, b = 0, len = n;   // a: first with x - x0 > -dxmax; b: first with x - x0 >= dxmax
+    while (len > 0) {            // a and b keep ranges of one length, so both loads go out together
+      const int half = len >> 1;
+      const float da = fsub(x[a + half], x0), db = fsub(x[b + half], x0);
+      if (!(da > -dxmax)) a += len - half;
+      if (db < dxmax) b += len - half;
+      len = half;
+    }
+    *first = a;
+    *last = b;
+  } else {
+    int lo = 0, hi = n;
+    const float D = fmul(kMaxXSlopeCandidates,
+                         fmaxf(fabsf(fsub(s.zmin[s1], z0)), fabsf(fsub(s.zmax[s1], z0))));   // >= every hit's dxmax
+    narrow_range(x, 0, n, x0, x0, D, &lo, &hi);
+    const float* z = ev.zs() + st;
+    auto passes = [&](int e) {
+      return fabsf(fsub(x[e], x0)) < fmul(kMaxXSlopeCandidates, fabsf(fsub(z[e], z0)));
+    };
+    while (lo < hi && !passes(lo)) ++lo;
+    int end = lo;
+    while (end < hi && passes(end)) ++end;
+    *first = lo;
+    *last = end;
+  }
+}
+
+template <class Shared, class Seed>
+__device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Seed& sd, int f, int nb) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int s1 = f - 2, m4 = f - 4;
+  const int st0 = s.start[f], n0 = s.num[f], st1 = s.start[s1], st4 = s.start[m4], n4 = s.num[m4];
+  const float zmin1 = s.zmin[s1], zmin4 = s.zmin[m4], zmax4 = s.zmax[m4];
+  const bool single1 = zmin1 == s.zmax[s1], single4 = zmin4 == zmax4;
+  const bool use_map = map_valid(s, s1, m4);
+  const uint32_t* map = sd.map[f & 1];
+  const float* x4 = ev.xs() + st4;
+  const float* y4 = ev.ys() + st4;
+  const float* z4 = ev.zs() + st4;
+  const uint32_t Y = (uint32_t)ev.Y;
+  if (n0 == 0 || n4 == 0 || s.num[s1] == 0) return;
+  const float s1_z = ev.zs()[st1];   // Kernel.cl:420
+  bool degenerate = false;
+
+  for (int block = 0; block < n0; block += 32) {   // warp-uniform
+    __syncwarp();   // the previous block's reads of the lists are done
+    // the block's unused h0s, dealt to the warps by rank
+    const int i0 = block + lane;
+    const bool unused = i0 < n0 && !(ev.useds()[st0 + i0] & kUsed);
+    const unsigned um = __ballot_sync(kFull, unused);
+    const int rank = __popc(um & lanemask_lt());
+    if (unused && (rank & (nwarps - 1)) == warp) sd.active[rank] = (uint16_t)i0;
+    __syncwarp();
+    const int mine = warp + lane * nwarps;
+    int h0 = 0, first = 0, count = 0;
+    float h0x = 0.f, h0y = 0.f, h0z = 0.f;
+    if (mine < __popc(um)) {
+      h0 = st0 + sd.active[mine];
+      h0x = ev.xs()[h0];
+      h0y = ev.ys()[h0];
+      h0z = ev.zs()[h0];
+      int last;
+      h1_window(ev, s, s1, h0x, h0z, &first, &last);
+      count = max(last - first, 0);
+    }
+    // the pairs of the warp's h0s, end to end
+    int end = count;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(kFull, end, o);
+      if (lane >= o) end += v;
+    }
+    const int total = __shfl_sync(kFull, end, 31);
+    if (total == 0) continue;
+    const int begin = end - count;
+    const unsigned om = __ballot_sync(kFull, count > 0);
+    const int slot = warp + __popc(om & lanemask_lt()) * nwarps;   // below 32: the warp's ranks leave it that many
+    if (count > 0) {
+      sd.h0[slot] = make_float4(h0x, h0y, h0z, __int_as_float(st1 + first - begin));
+      sd.reach[slot] = make_float2(fmul(kMaxYSlope, fabsf(fsub(s1_z, h0z))),
+                                   fmul(fsub(zmin4, h0z), fdiv(1.f, fsub(zmin1, h0z))));
+      sd.best[slot] = ~0ull;
+      sd.first[slot] = (uint16_t)first;
+    }
+    __syncwarp();
+
+    int owners = 0, queued = 0;
+    for (int base = 0;; base += 32) {
+      const bool more = base < total;   // warp-uniform
+      bool pass = false;
+      int h1 = 0, o = 0;
+      if (more) {
+        // the h0 of each lane's pair: count the h0s that begin up to it
+        const uint32_t starts =
+            __reduce_or_sync(kFull, count > 0 && begin >= base && begin < base + 32 ? 1u << (begin - base) : 0u);
+        o = owners + __popc(starts & (2u * (1u << lane) - 1u)) - 1;
+        owners += __popc(starts);
+        if (base + lane < total) {
+          const float4 q = sd.h0[warp + o * nwarps];
+          const float2 r = sd.reach[warp + o * nwarps];
+          h1 = __float_as_int(q.w) + base + lane;
+          const uint8_t u1 = ev.useds()[h1];
+          const float h1x = ev.xs()[h1], h1y = ev.ys()[h1];
+          pass = u1 == 0 && fabsf(fsub(h1y, q.y)) < r.x;
+          if (pass && use_map) {   // the fit's own predicted point
+            const float px = fadd(q.x, fmul(fsub(h1x, q.x), r.y));
+            const float py = fadd(q.y, fmul(fsub(h1y, q.y), r.y));
+            pass = (map[map_cell(py) & (kMapRows - 1)] >> (map_cell(px) & 31)) & 1u;
+          }
+        }
+      }
+      const unsigned pm = __ballot_sync(kFull, pass);
+      if (queued + __popc(pm) > kQueue || !more) {   // warp-uniform
+        __syncwarp();
+        const uint32_t entry = sd.queue[warp][lane];
+        const int own = warp + (int)(entry >> 14) * nwarps;
+        const int local1 = (int)(entry & 0x3fffu), hit1 = st1 + local1;
+        // a Y-lane stops at its first dead h1: where the dead h1s are not the
+        // module's last ones, look for one before this pair's
+        bool reached = lane < queued;
+        if (!(s.flags[s1] & kDeadTail) && reached)
+          for (int e = local1 - (int)Y; e >= (int)sd.first[own]; e -= (int)Y) reached &= !h1_dead(ev, s, s1, st1 + e);
+        if (reached) {
+          // Kernel.cl:468-529 for one (h0, h1): the fits of the h2s in reach
+          const float4 q = sd.h0[own];
+          const float h1x = ev.xs()[hit1], h1y = ev.ys()[hit1], h1z = single1 ? zmin1 : ev.zs()[hit1];
+          const float dz_inverted = fdiv(1.f, fsub(h1z, q.z));
+          const float ddx = fsub(h1x, q.x), ddy = fsub(h1y, q.y);
+          const float xa = fadd(q.x, fmul(ddx, fmul(fsub(zmin4, q.z), dz_inverted)));
+          const float xb = single4 ? xa : fadd(q.x, fmul(ddx, fmul(fsub(zmax4, q.z), dz_inverted)));
+          const float d_lo = fsub(zmin4, h1z), d_hi = fsub(zmax4, h1z);
+          const float reach = fmul(kScatterReach, fmaxf(fabsf(d_lo), fabsf(d_hi)));
+          const float tol = d_lo > kMinDz || d_hi < -kMinDz ? fminf(kTolerance, reach) : kTolerance;
+          const float xl = fminf(xa, xb), xh = fmaxf(xa, xb);
+          const float margin = fadd(0.01f, fmul(1e-5f, fadd(fabsf(xl), fabsf(xh))));
+          const float lt = fsub(fsub(xl, tol), margin);
+          float ht = fadd(fadd(xh, tol), margin);
+          int k = 0;
+          if (isfinite(xa) && isfinite(xb) && isfinite(lt) && isfinite(ht))
+            k = first_gt(x4, 0, n4, lt);
+          else
+            ht = __int_as_float(0x7f800000);   // +inf: every hit is tried
+          float best = FLT_MAX;
+          int best_k = -1;
+          uint32_t zc = 0x7fc00001u;
+          float z2_tz = 0.f, den = 0.f;
+          for (; k < n4; ++k) {
+            const float h2x = x4[k];
+            if (h2x > ht) break;
+            const float h2z = single4 ? zmin4 : z4[k];
+            if (__float_as_uint(h2z) != zc) {   // both factors depend on h2z only (per h0, h1)
+              zc = __float_as_uint(h2z);
+              z2_tz = fmul(fsub(h2z, q.z), dz_inverted);
+              den = fdiv(1.f, fsub(h2z, h1z));
+            }
+            const float dx = fsub(fadd(q.x, fmul(ddx, z2_tz)), h2x);
+            const float dy = fsub(fadd(q.y, fmul(ddy, z2_tz)), y4[k]);
+            if (fabsf(dx) < kTolerance && fabsf(dy) < kTolerance) {
+              const float scatter = fmul(fmul(fadd(fmul(dx, dx), fmul(dy, dy)), den), den);
+              if (scatter < kMaxScatter ? scatter < best : !isfinite(scatter)) {
+                // the h2 must lie in the h1's window: from the first hit above
+                // the lower bound (that one even if it is above the upper
+                // bound) up to the first later one above the upper bound
+                float lo, hi;
+                h2_bounds(h1x, h1z, s.sz[f], s.sz[m4], &lo, &hi);
+                if (h2x > lo && (!(h2x > hi) || k == 0 || !(x4[k - 1] > lo))) {
+                  if (scatter < kMaxScatter) {
+                    best = scatter;
+                    best_k = k;
+                  } else {
+                    degenerate = true;
+                  }
+                }
+              }
+            }
+          }
+          if (best_k >= 0) {   // smallest fit, then Y-lane, h1, h2
+            const uint32_t e = (uint32_t)local1 - sd.first[own];
+            atomicMin(&sd.best[own], ((unsigned long long)__float_as_uint(best) << 32) |
+                                         ((unsigned long long)(e % Y) << 28) | ((unsigned long long)e << 14) |
+                                         (unsigned long long)best_k);
+          }
+        }
+        queued = 0;
+        __syncwarp();
+      }
+      if (!more) break;
+      if (pass) sd.queue[warp][queued + __popc(pm & lanemask_lt())] = ((uint32_t)o << 14) | (uint32_t)(h1 - st1);
+      queued += __popc(pm);
+    }
+    // Kernel.cl:550-567: one shared-memory atomic per warp for the tracklet rows, one for the ring
+    const unsigned long long best = count > 0 ? sd.best[slot] : ~0ull;
+    const bool win = best != ~0ull;
+    const uint32_t tp = warp_reserve(&s.ntracklets, win);
+    const bool push = win && tp < ev.cap;
+    const uint32_t ri = warp_reserve(&s.ring_hi[nb], push);
+    if (push) {
+      const uint32_t h1 = (uint32_t)(st1 + first) + ((uint32_t)(best >> 14) & 0x3fffu);
+      const uint32_t h2 = (uint32_t)st4 + (uint32_t)(best & 0x3fffu);
+      ev.tracklets[tp] = make_uint4((uint32_t)h0, h1, h2, 0u);
+      if (ri < ev.ring_cap) write_tracklet_entry(ev, nb, ev.ring_cap - 1u - ri, tp, h1, h2);
+    }
+  }
+  if (degenerate) atomicOr(&s.status, VELO_EVENT_DEGENERATE);
+}
+
+// The flags of module m's hits before the search (one warp): unused, and
+// kDead where the hit as an h1 has no h2 window; whether the dead hits are
+// the module's last ones.
+template <class Shared>
+__device__ __forceinline__ bool clear_flags(const EventView& ev, const Shared& s, int m) {
+  const int lane = threadIdx.x & 31;
+  const int st = s.start[m], n = s.num[m];
+  bool tail = true;
+  unsigned before = 0;   // dead hits so far
+  for (int i0 = 0; i0 < n; i0 += 32) {
+    const int i = i0 + lane;
+    const bool in = i < n;
+    const bool dead = in && h1_dead(ev, s, m, st + i);
+    if (in) ev.useds()[st + i] = dead ? kDead : 0;
+    const unsigned dm = __ballot_sync(kFull, dead), im = __ballot_sync(kFull, in);
+    const unsigned live = im & ~dm, from_dead = 0u - (dm & (0u - dm));   // lanes from the first dead hit on
+    if ((before && live) || (live & from_dead)) tail = false;
+    before |= dm;
+  }
+  return tail;
 }
 
 // Per-phase cycle counters, compiled in only with -DVELO_PHASE_CLOCKS
@@ -927,8 +1343,7 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
   ev.arena = arena;
   ev.P = L.y;
   const uint64_t hb = p.hit_base[e];
-  ev.ring0 = reinterpret_cast<uint4*>(p.rings + 8 * hb);
-  ev.ring1 = ev.ring0 + ev.cap;
+  ev.rings = reinterpret_cast<uint4*>(p.rings + 16 * hb);
   ev.tracklets = reinterpret_cast<uint4*>(p.tracklets + 4 * hb);
   ev.weak = p.weak + hb;
   ev.tracks = p.tracks + hb;
@@ -946,6 +1361,7 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
   // stage the event; the module table must tile [0, H) in order (the host
   // checked only the header and the blob's length)
   bool bad = tid == 0 && S == 0 && H != 0;
+  bool wild = !ev.narrow;   // the event does not take the pair seeding
   for (int m = tid; m < S; m += nt) {
     const int32_t st = gstart[m], nm = gnum[m];
     const int64_t expect = m == 0 ? 0 : (int64_t)gstart[m - 1] + (int64_t)gnum[m - 1];
@@ -965,7 +1381,7 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
     ev.xs()[i] = xv;
     ev.ys()[i] = yv;
     ev.zs()[i] = zv;
-    ev.useds()[i] = 0;
+    wild |= fmaxf(fabsf(xv), fmaxf(fabsf(yv), fabsf(zv))) > kMaxCoordinate;
     if (p.sort_events) ids[i] = gid[i];
   }
   if (tid == 0) {
@@ -974,6 +1390,7 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
     s.considered = 0; s.kept = 0;
     s.seed_next[0] = 0; s.seed_next[1] = 0;
   }
+  for (int i = tid; i < 2 * kMapRows; i += nt) s.seed.map[i / kMapRows][i % kMapRows] = 0;
   if (__syncthreads_or(bad)) {   // a bad module table, or a non-finite coordinate
     if (tid == 0) {
       p.out_counts[e] = 0;
@@ -1001,7 +1418,7 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
   }
   VELO_PHASE(0);
 
-  // per-module z range and x-sortedness (one warp per module)
+  // per-module z range, x-sortedness and hit flags (one warp per module)
   for (int m = warp; m < S; m += nwarps) {
     const int st = s.start[m], n = s.num[m];
     float zmn = FLT_MAX, zmx = -FLT_MAX;
@@ -1018,42 +1435,35 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
       zmx = fmaxf(zmx, __shfl_xor_sync(kFull, zmx, o));
     }
     sorted = __all_sync(kFull, sorted);
+    wild |= !sorted;
+    const bool tail = clear_flags(ev, s, m);
     if (lane == 0) {
       s.zmin[m] = zmn;
       s.zmax[m] = zmx;
-      s.sorted[m] = sorted ? 1 : 0;
+      s.flags[m] = (sorted ? kSorted : 0) | (tail ? kDeadTail : 0);
     }
   }
-  // windows of modules 0..3 stay empty (Kernel.cl:104 gates the body on f >= 4)
-  const int hbeg = S >= 5 ? s.start[4] : H;
-  for (int i = tid; i < hbeg; i += nt) ev.wins()[i] = make_uint2(0xffffffffu, 0xffffffffu);
-  __syncthreads();
+  ev.tame = !__syncthreads_or(wild);
   VELO_PHASE(1);
 
-  // candidate windows for every hit of modules >= 4
-  for (int h = hbeg + tid; h < H; h += nt) {
-    int lo = 4, hi = S - 1;   // last module whose start is <= h
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (s.start[mid] <= h) lo = mid; else hi = mid - 1;
-    }
-    compute_windows(ev, s, h, lo);
+  bool learned = kMode == kLearned && (p.learned_max_hits == 0 || (uint32_t)H <= p.learned_max_hits);
+  // per-lane constants of the learned seeding's ballots
+  SeedLanes sl{};
+  if constexpr (kMode == kLearned) sl = seed_lanes_of(kLanes, (uint32_t)ev.Y);
+  // candidate windows for the seedings that read them
+  if (kMode != kPlain || !ev.tame) {
+    fill_windows(ev, s);
+    __syncthreads();
   }
-
-  // per-lane constants of the seeding ballots (the host checked that
-  // seed_lanes is 8, 16 or 32, and a multiple of Y below 32)
-  const SeedLanes sl = seed_lanes_of(kLanes, (uint32_t)ev.Y);
-  __syncthreads();
   VELO_PHASE(2);
 
   // The learned seeding runs first when enabled; if it kept too small a
   // fraction of the doublets it scored, the event is searched again by the
-  // plain method (used flags and lists reset; windows kept).
-  bool learned = kMode == kLearned && (p.learned_max_hits == 0 || (uint32_t)H <= p.learned_max_hits);
+  // plain method (flags and lists reset; windows kept).
   uint32_t fallback = (kMode == kLearned && !learned) ? VELO_EVENT_LEARNED_FALLBACK : 0u;
   for (int attempt = 0; attempt < 2; ++attempt) {
     if (attempt > 0) {
-      for (int i = tid; i < H; i += nt) ev.useds()[i] = 0;
+      for (int m = warp; m < S; m += nwarps) clear_flags(ev, s, m);
       if (tid == 0) {
         s.ring_lo[0] = 0; s.ring_lo[1] = 0; s.ring_hi[0] = 0; s.ring_hi[1] = 0;
         s.ntracks = 0; s.ntracklets = 0; s.nweak = 0; s.status = 0;
@@ -1061,9 +1471,14 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
       }
       __syncthreads();
     }
+    const bool pairs = kMode == kPlain && ev.tame;
     // module loop, Kernel.cl:671-767
     int b = 0;   // ring[b] holds the entries to follow in this iteration
     for (int f = S - 1; f >= 4; --f) {
+      // the map of the h2 module, by the last warps (the first ones have the
+      // most entries to forward)
+      if (pairs && map_valid(s, f - 2, f - 4))
+        for (int i = nt - 1 - tid; i < s.num[f - 4]; i += nt) mark_map(ev, s, s.seed.map[f & 1], f - 2, f - 4, i);
       const uint32_t lo_n = min(s.ring_lo[b], ev.ring_cap);
       const uint32_t ncur = min(lo_n + s.ring_hi[b], ev.ring_cap);
       if (tid == 0 && s.ring_lo[b] + s.ring_hi[b] > VELO_TTF_MODULO) s.status |= VELO_EVENT_RING_OVERFLOW;
@@ -1080,11 +1495,14 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
         s.ring_lo[b] = 0;   // ring[b] is refilled two iterations on
         s.ring_hi[b] = 0;
       }
-      if (s.num[f] > 0) {
-        if (learned)
+      if (pairs) {
+        for (int i = tid; i < kMapRows; i += nt) s.seed.map[(f & 1) ^ 1][i] = 0;   // for the next module
+        seed_pairs(ev, s, s.seed, f, b ^ 1);
+      } else if (s.num[f] > 0) {
+        if (kMode == kLearned && learned)
           seed_module<kLearned, kLanes>(ev, s, f, b ^ 1, sl);
         else
-          seed_module<kMode == kDump ? kDump : kPlain, kLanes>(ev, s, f, b ^ 1, sl);
+          seed_windows<kMode == kDump ? kDump : kPlain, kLanes>(ev, s, f, b ^ 1);
       }
       __syncthreads();
       VELO_PHASE(4);
@@ -1097,7 +1515,7 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
       const uint32_t lo_n = min(s.ring_lo[b], ev.ring_cap);
       const uint32_t ncur = min(lo_n + s.ring_hi[b], ev.ring_cap);
       for (uint32_t i = tid; i < ncur; i += nt) {
-        const uint32_t v = ring_entry(ev, b, lo_n, i).x;
+        const uint32_t v = ring_words(ev, b)[ring_index(ev, lo_n, i)].x;
         if (v & kTrackletFlag) {
           const uint32_t wi = atomicAdd(&s.nweak, 1u);
           if (wi < ev.cap) ev.weak[wi] = v & kEntryNumber;
@@ -1111,13 +1529,11 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
       for (uint32_t i = tid; i < nweak; i += nt) {
         const uint4 t = ev.tracklets[ev.weak[i]];
         const uint32_t a = t.x, bb = t.y, c = t.z;
-        if (!ev.useds()[a] && !ev.useds()[bb] && !ev.useds()[c]) {
+        if (((ev.useds()[a] | ev.useds()[bb] | ev.useds()[c]) & kUsed) == 0) {
           const uint32_t tn = atomicAdd(&s.ntracks, 1u);
           if (tn >= ev.cap) continue;
           uint32_t* wr = reinterpret_cast<uint32_t*>(&ev.tracks[tn]);
           wr[0] = 3; wr[1] = a; wr[2] = bb; wr[3] = c;
-  #pragma unroll
-          for (int k = 4; k < 25; ++k) wr[k] = 0;
         }
       }
     }
@@ -1148,7 +1564,10 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
     const uint32_t words = (uint32_t)min((unsigned long long)min(s.ntracks, ev.cap), room) * 25u;
     const uint32_t* src = reinterpret_cast<const uint32_t*>(ev.tracks);
     uint32_t* dst = reinterpret_cast<uint32_t*>(p.out_tracks + s.out_first);
-    for (uint32_t w = tid; w < words; w += nt) dst[w] = src[w];
+    for (uint32_t w = tid; w < words; w += nt) {   // words past a track's last hit are zero
+      const uint32_t t = w / 25u;
+      dst[w] = w - 25u * t <= src[25u * t] ? src[w] : 0u;
+    }
   }
   if (p.results) {   // streaming: the tracks first, then the record
     __threadfence_system();
@@ -1170,7 +1589,7 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
 template <int kMaxThreads, int kMinCtas, int kMode, int kMods, int kLanes>
 __global__ void __launch_bounds__(kMaxThreads, kMinCtas) search_kernel(const SearchParams p) {
   extern __shared__ __align__(16) uint8_t dyn_smem_raw[];
-  __shared__ SharedT<kMods> s;
+  __shared__ SharedT<kMods, kMaxThreads / 32> s;
   // learned seeding: the MLP weights lead the dynamic shared memory
   const MlpFrag* mlp_smem = nullptr;
   uint8_t* dyn_smem = dyn_smem_raw;

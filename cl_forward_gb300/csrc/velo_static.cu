@@ -35,7 +35,7 @@
 namespace velo {
 namespace {
 
-constexpr uint64_t kRowBytes = 16u + 32u + 4u + sizeof(velo_track);   // tracklet + rings + weak + track per hit row
+constexpr uint64_t kRowBytes = 16u + 64u + 4u + sizeof(velo_track);   // tracklet + rings + weak + track per hit row
 constexpr uint64_t kEventBytes = 4u + 4u + 4u + 8u + 8u;         // hits, maxmod, valid, hit_base, arena_off
 constexpr uint64_t kCounterBytes = 256;
 constexpr uint64_t kOffEvents = kCounterBytes;
@@ -53,7 +53,7 @@ struct StaticView {
   uint64_t* hit_base;
   uint64_t* arena_off;
   uint32_t* tracklets;          // 4 words per row
-  uint32_t* rings;              // 8 words per row
+  uint32_t* rings;              // 16 words per row
   uint32_t* weak;               // 1 per row
   velo_track* tracks;           // 1 per row
 };
