@@ -112,8 +112,8 @@ struct SearchParams {
   // global scratch
   uint8_t* global_arena;
   uint32_t* tracklets;            // 4 words per tracklet {h0, h1, h2, 0}, row hit_base[e]
-  uint32_t* rings;                // 16 words per row: the two tracks-to-follow rings of event e
-                                  // (max(H, 1) entries of 32 bytes each) from row hit_base[e]
+  uint32_t* entry_words;          // tracks-to-follow entries, row hit_base[e]: 4 words and
+  uint32_t* entry_lines;          //   4 floats per row (velo_search_kernel.cuh: Worker)
   uint32_t* weak;                 // weak-track list, row hit_base[e]
   velo_track* tracks;             // working tracks, row hit_base[e]
   // outputs

@@ -12,7 +12,7 @@
 // fits the launch's tile, else in global scratch with the same layout, which
 // L1 caches.  On GB300 the fastest launch keeps the tile tiny: shared memory
 // and L1 share each SM's storage, and resident CTAs are register-bound, so L1
-// serves the arenas better than staging does.  The tracks-to-follow rings,
+// serves the arenas better than staging does.  The tracks-to-follow entries,
 // tracklets and working tracks are per-hit-row global scratch.
 //
 // Decisions are the reference's, bit for bit:
@@ -32,15 +32,9 @@
 // unsorted module the full sequential scan runs.  Narrowing changes work, not
 // results.
 //
-// Per module iteration the CTA meets at two barriers: after forwarding (its
-// used-hit marks feed seeding) and after seeding (its tracklets feed the next
-// forwarding).  Seeding gives each h0 to a group of G lanes of a warp (G =
-// 8, 16 or 32, the kernel build's seeding width), whose lanes take the h0's
-// h1 candidates; lane cut-offs come from a ballot and the winner from a
-// group min-reduction, so seeding itself needs no block barrier.  Each
-// tracks-to-follow buffer is filled from both ends (forwarding from the
-// front, seeding from the back), which keeps the two counts separate without
-// another barrier.
+// The two parities of modules are seeded by different warps, each with its own
+// tracks-to-follow entries, so a CTA meets at one barrier per two module
+// iterations (Worker).
 //
 // Optional per launch: the x-sort of each event while it is staged, with the
 // sorted hit arrays written back into the input (sort_events), and a
@@ -73,20 +67,19 @@ constexpr uint8_t kUsed = 1, kDead = 2;
 // Per-module flags: its hits are x-sorted; its dead h1s are its last hits.
 constexpr uint8_t kSorted = 1, kDeadTail = 2;
 
-// Pair seeding (seed_pairs), per CTA: the h0s being seeded, 32 at a time, and
-// the occupancy map of the h2 module.
+// Seeding state per CTA: each warp's lists, and per module parity the
+// occupancy map of the h2 module.  kOwn: the h0s a warp seeds at once.
 constexpr int kMapRows = 64;          // 64 rows x 32 columns of cells
 constexpr int kQueue = 32;            // pairs a warp holds for the exact fits
-template <int kWarps>
+template <int kWarps, int kOwn>
 struct SeedShared {
-  float4 h0[32];                      // x, y, z, first h1 - first pair (int bits)
-  float2 reach[32];                   // the h0's y cut, and (z2 - z0) / (z1 - z0) where the map is valid
-  unsigned long long best[32];        // the h0's best (fit, Y-lane, h1, h2) so far
-  uint32_t map[2][kMapRows];          // by parity of the module being seeded
-  // owner << 14 | h1 in its module; of 32 h0s, 16 warps have at most 2 each
-  std::conditional_t<(kWarps > 8), uint16_t, uint32_t> queue[kWarps][kQueue];
-  uint16_t active[32];                // unused h0s of the block, by rank
-  uint16_t first[32];                 // the h0's first h1 in its module
+  float4 h0[kWarps][kOwn];            // x, y, z, first h1 - first pair (int bits)
+  float2 reach[kWarps][kOwn];         // the h0's y cut, and (z2 - z0) / (z1 - z0) where the map is valid
+  unsigned long long best[kWarps][kOwn];   // the h0's best (fit, Y-lane, h1, h2) so far
+  uint32_t map[2][kMapRows];
+  std::conditional_t<(kOwn > 4), uint32_t, uint16_t> queue[kWarps][kQueue];   // h0 << 14 | h1 in its module
+  uint16_t first[kWarps][kOwn];       // the h0's first h1 in its module
+  uint8_t active[kWarps][32];         // the warp's unused h0s of a block of 32 hits
 };
 
 // Per-CTA shared state for events of up to kMods modules.  Launches whose
@@ -95,50 +88,46 @@ struct SeedShared {
 // to L1 and to more resident CTAs.
 template <int kMods, int kWarps>
 struct SharedT {
-  int32_t start[kMods];
-  int32_t num[kMods];
+  // h0s per warp and round: with two warps a block of 32 hits rarely leaves
+  // more than 16 unused; the others keep the static state below 8 KB
+  static constexpr int kOwn = kWarps <= 2 ? 16 : kMods <= kCompactModules ? 64 / kWarps : 16 / kWarps + (kWarps <= 8) * 2;
+  static constexpr int kMaxWarps = kWarps;
+  SeedShared<kWarps, kOwn> seed;
+  int32_t start[kMods];       // [S] = H
   int32_t sz[kMods];
   float zmin[kMods];
   float zmax[kMods];
-  uint8_t flags[kMods];   // kSorted, kDeadTail
-  uint32_t ring_lo[2];   // forwarding entries, from the front of ring[i]
-  uint32_t ring_hi[2];   // seeding entries, from the back of ring[i]
-  uint32_t ntracks, ntracklets, nweak, status;
-  uint32_t considered, kept;   // learned seeding: doublets scored / kept
+  uint32_t inflight[kMods];   // forwarding f: entries at its start | entries at its start and pushed << 16
+  uint8_t flags[kMods];       // kSorted, kDeadTail
+  uint32_t tracks[kWarps];    // tracks of each warp
+  uint32_t status;
+  uint32_t considered, kept;  // learned seeding: doublets scored / kept
   unsigned long long out_first;
   int32_t next_event;
-  int32_t seed_next[2];  // G < 32: next unclaimed h0 of the module being seeded, by ring parity
-  SeedShared<kWarps> seed;
+  __device__ __forceinline__ int num(int m) const { return start[m + 1] - start[m]; }
 };
 
 struct EventView {
-  int S, H, Y;
-  uint32_t cap;             // tracklet / track / weak rows (max(H, 1))
-  uint32_t ring_cap;        // entries of each tracks-to-follow buffer (max(H, 1): one per seeded h0 at most)
+  const SearchParams* p;    // the kernel's parameters (constant memory)
+  int S, H;
+  int event;
   // the arena: x, y, z, windows (per hit {h1 first | h1 last << 16, h2 first
-  // | h2 last << 16}) and used flags at multiples of one stride P
+  // | h2 last << 16}) and flags at multiples of one stride P
   uint8_t* arena;
   uint32_t P;
+  bool tame;                // every module x-sorted and every coordinate within kMaxCoordinate
+  const MlpFrag* mlp;       // learned seeding: weights in shared memory
   __device__ __forceinline__ float* xs() const { return reinterpret_cast<float*>(arena); }
   __device__ __forceinline__ float* ys() const { return reinterpret_cast<float*>(arena + P); }
   __device__ __forceinline__ float* zs() const { return reinterpret_cast<float*>(arena + 2u * P); }
   __device__ __forceinline__ uint2* wins() const { return reinterpret_cast<uint2*>(arena + 3u * P); }
   __device__ __forceinline__ uint8_t* useds() const { return arena + 5u * P; }
-  uint4* rings;             // tracks-to-follow buffers: entry words of buffer 0 and 1, then their lines
-  uint4* tracklets;         // {h0, h1, h2, 0} per tracklet
-  uint32_t* weak;
-  velo_track* tracks;
-  bool narrow;
-  bool tame;                // every module x-sorted and every coordinate within kMaxCoordinate
-  int event;
-  const MlpFrag* mlp;       // learned seeding: weights in shared memory
-  float keep_threshold, window_margin;
-  int learned_min_window;   // doublets with narrower h2 windows are searched exactly, unscored
-  float* dump_features;     // training-data dump
-  uint32_t* dump_ids;
-  unsigned long long* dump_count;
-  uint64_t dump_capacity;
-  uint32_t dump_keep;
+  // scratch by row: tracklets {h0, h1, h2, 0}, tracks, weak list, entries
+  __device__ __forceinline__ uint4* tracklets() const { return reinterpret_cast<uint4*>(p->tracklets); }
+  __device__ __forceinline__ velo_track* tracks() const { return p->tracks; }
+  __device__ __forceinline__ uint32_t* weak() const { return p->weak; }
+  __device__ __forceinline__ uint4* entry_words() const { return reinterpret_cast<uint4*>(p->entry_words); }
+  __device__ __forceinline__ float4* entry_lines() const { return reinterpret_cast<float4*>(p->entry_lines); }
 };
 
 // First index i in [lo, hi) with x[i] > c, for non-decreasing x.
@@ -198,11 +187,11 @@ template <class Shared>
 __device__ void compute_windows(const EventView& ev, const Shared& s, int h, int f) {
   const int s2 = f - 2;
   const bool proc_h2 = f <= ev.S - 3;
-  const int st2 = s.start[s2], n2 = s.num[s2];
+  const int st2 = s.start[s2], n2 = s.num(s2);
   const float x0 = ev.xs()[h], z0 = ev.zs()[h];
   const float* x2 = ev.xs() + st2;
   const float* z2 = ev.zs() + st2;
-  const bool sorted = ev.narrow && (s.flags[s2] & kSorted);
+  const bool sorted = ev.p->narrow && (s.flags[s2] & kSorted);
   uint32_t r1f = kNone16, r1l = kNone16, r2f = kNone16, r2l = kNone16;
 
   // h1 window: first hit with |x1-x0| < 0.7|z1-z0|, then the first later hit
@@ -287,37 +276,54 @@ __device__ void compute_windows(const EventView& ev, const Shared& s, int h, int
 }
 
 // ---------------------------------------------------------------------------
-// Tracks-to-follow entries.  Bit 31 marks a tracklet (3 hits, number = its
-// row in the tracklet list) and bits 28-30 count skipped modules, as in the
-// reference (Kernel.cl:222-225,351,566).  This kernel also keeps a track's
-// hit count in bits 23-27 (the reference re-reads it from the track), so
-// numbers use bits 0-22.
+// Work split.  Seeding module f touches modules f, f-2 and f-4 only, so the
+// two parities of modules are seeded by different warps: half of the CTA's
+// warps seed the modules f = S-1, S-3, ..., the other half S-2, S-4, ...
+// Each warp owns the tracks-to-follow entries of its own seeds, forwards them
+// in every iteration (onto modules of either parity), and keeps its
+// tracklets, tracks and weak list in its own rows, so none of them needs an
+// atomic or a barrier.  What the warps share is the hits' used flags:
+//  * an extension in the forwarding of iteration f marks a hit of f-4, first
+//    read by the seeding of f-2;
+//  * a tracklet's promotion marks hits of its own parity; a seeding of that
+//    parity must see the promotions before it and none after it: both are
+//    the warp's own (or, with more than two warps, its group's), in order.
+// So the warps meet once per two iterations: when iterations f and f-1 begin,
+// every forwarding down to f+1 has been done by all of them.
+//
+// Before, all warps forwarded and seeded each module together: two barriers
+// per iteration, shared-memory counters, and each module's 4 unused h0s spread
+// over the warps.  With 64 threads the split runs one warp per parity: 173 k ->
+// 142 k warp instructions per event, 10,000 events of 1,160 hits 2.50 -> 1.97
+// ms, one event 0.42 -> 0.29 ms.
+struct Worker {
+  uint32_t row;        // first of its scratch rows
+  uint32_t n, tracklets, tracks, weak;
+  // warp in the CTA; the parity it seeds, (S-1-f) & 1 (one warp: every f); its
+  // place among the `of` warps of that parity
+  __device__ __forceinline__ static int warp() { return threadIdx.x >> 5; }
+  __device__ __forceinline__ static bool alone() { return blockDim.x == 32; }
+  __device__ __forceinline__ static int parity() { return warp() & 1; }
+  __device__ __forceinline__ static int idx() { return warp() >> 1; }
+  __device__ __forceinline__ static int of() { return alone() ? 1 : (int)blockDim.x >> 6; }
+};
+
+// An entry is {word, last hit | iteration it was found in << 24, z of the
+// previous hit, z of the last hit} and the line through the last two hits {x
+// and y of the previous hit, x and y slopes}.  Bit 31 of the word marks a
+// tracklet (3 hits, number = its row among the warp's tracklets), as in the
+// reference (Kernel.cl:222-225,566); otherwise bits 23-27 are the track's hit
+// count and bits 0-22 its row among the warp's tracks.  The iteration says
+// how many modules were skipped (the reference counts them in bits 28-30), so
+// an entry that finds nothing stays as it is, where it is.  The line is
+// computed when the hit is found: forwarding reads no hit, track or tracklet
+// before its fit.
 constexpr uint32_t kEntryNumber = 0x007FFFFFu;
 constexpr uint32_t kEntryCountShift = 23;
+constexpr uint32_t kEntryHit = 0x00FFFFFFu;   // 255 modules of 16,383 hits: 22 bits
+constexpr uint32_t kEntryIterationShift = 24;
 
 __device__ __forceinline__ unsigned lanemask_lt() { return (1u << (threadIdx.x & 31)) - 1u; }
-
-// One shared-memory atomic per warp: lanes with `take` get consecutive slots
-// from *counter; returns this lane's slot.
-__device__ __forceinline__ uint32_t warp_reserve(uint32_t* counter, bool take) {
-  const unsigned m = __ballot_sync(kFull, take);
-  if (m == 0) return 0;
-  const int leader = __ffs(m) - 1;
-  uint32_t base = 0;
-  if ((int)(threadIdx.x & 31) == leader) base = atomicAdd(counter, (uint32_t)__popc(m));
-  base = __shfl_sync(kFull, base, leader);
-  return base + (uint32_t)__popc(m & lanemask_lt());
-}
-
-// Entry i of buffer b is a pair of 16-byte halves in two arrays: {entry word,
-// last hit, z of the previous hit, z of the last hit} and the line through
-// the last two hits {x and y of the previous hit, x and y slopes}.  The line
-// is computed when the hit is found, so an entry that finds nothing is passed
-// on as it is, and forwarding reads no hit, track or tracklet before its fit.
-__device__ __forceinline__ uint4* ring_words(const EventView& ev, int b) { return ev.rings + (size_t)b * ev.ring_cap; }
-__device__ __forceinline__ float4* ring_lines(const EventView& ev, int b) {
-  return reinterpret_cast<float4*>(ev.rings + (size_t)(2 + b) * ev.ring_cap);
-}
 
 // The line through hit a and then hit b (z differing), as the reference
 // takes it from a track's last two hits (Kernel.cl:253-257).  td = 1 / (zb - za).
@@ -325,26 +331,52 @@ __device__ __forceinline__ float4 line_through(float xa, float ya, float xb, flo
   return make_float4(xa, ya, fmul(fsub(xb, xa), td), fmul(fsub(yb, ya), td));
 }
 
-// Writes a new tracklet's entry {h0, h1, h2} to slot i of buffer b.
-__device__ __forceinline__ void write_tracklet_entry(const EventView& ev, int b, uint32_t i, uint32_t tp, uint32_t h1,
-                                                     uint32_t h2) {
-  const float z1 = ev.zs()[h1], z2 = ev.zs()[h2];
-  const float td = fdiv(1.0f, fsub(z2, z1));
-  ring_words(ev, b)[i] = make_uint4(kTrackletFlag | tp, h2, __float_as_uint(z1), __float_as_uint(z2));
-  ring_lines(ev, b)[i] = line_through(ev.xs()[h1], ev.ys()[h1], ev.xs()[h2], ev.ys()[h2], td);
+// Appends the tracklets {h0, h1, h2} of the lanes with `win`, seeded in
+// iteration f, to the warp's rows and entries (Kernel.cl:550-567).
+__device__ __forceinline__ void append_tracklets(const EventView& ev, Worker& w, bool win, uint32_t h0, uint32_t h1,
+                                                 uint32_t h2, int f) {
+  const unsigned m = __ballot_sync(kFull, win);
+  if (m == 0) return;
+  if (win) {
+    const uint32_t r = (uint32_t)__popc(m & lanemask_lt());
+    const uint32_t tp = w.tracklets + r, i = w.row + w.n + r;
+    ev.tracklets()[w.row + tp] = make_uint4(h0, h1, h2, 0u);
+    const float z1 = ev.zs()[h1], z2 = ev.zs()[h2];
+    ev.entry_words()[i] = make_uint4(kTrackletFlag | tp, h2 | ((uint32_t)f << kEntryIterationShift),
+                                    __float_as_uint(z1), __float_as_uint(z2));
+    ev.entry_lines()[i] =
+        line_through(ev.xs()[h1], ev.ys()[h1], ev.xs()[h2], ev.ys()[h2], fdiv(1.0f, fsub(z2, z1)));
+  }
+  w.tracklets += __popc(m);
+  w.n += __popc(m);
 }
 
-// A seeding warp's new tracklet goes to the back of buffer b.
+// Barrier of the warps of one parity.
+template <int kWarps>
+__device__ __forceinline__ void group_sync(const Worker& w) {
+  if (kWarps <= 2 || w.of() == 1)
+    __syncwarp();
+  else if (w.parity() == 0)   // constant names: a variable one reserves all 16 of the CTA, and 4 CTAs fill an SM
+    asm volatile("bar.sync 1, %0;" ::"r"(32 * w.of()) : "memory");
+  else
+    asm volatile("bar.sync 2, %0;" ::"r"(32 * w.of()) : "memory");
+}
+
+// The rows of a warp: as many as it can seed h0s.  A module's hits are dealt
+// by rank within blocks of 32 to the warps of its parity (see active_h0s).
 template <class Shared>
-__device__ __forceinline__ void push_back(Shared& s, const EventView& ev, int b, uint32_t tp, uint32_t h1,
-                                          uint32_t h2) {
-  const uint32_t i = atomicAdd(&s.ring_hi[b], 1u);
-  if (i < ev.ring_cap) write_tracklet_entry(ev, b, ev.ring_cap - 1u - i, tp, h1, h2);
-}
-
-// Index of the i-th entry of a buffer: the front segment, then the back segment.
-__device__ __forceinline__ uint32_t ring_index(const EventView& ev, uint32_t lo, uint32_t i) {
-  return i < lo ? i : ev.ring_cap - 1u - (i - lo);
+__device__ __forceinline__ uint32_t first_row(const Shared& s, const Worker& w, int S) {
+  if (w.alone()) return 0u;
+  int rows = 0;
+  const int per = 32 / w.of();
+  for (int m = threadIdx.x & 31; m < S; m += 32) {
+    const int n = s.num(m), rem = n & 31, parity = (S - 1 - m) & 1;
+    if (parity == w.parity())
+      rows += (n >> 5) * per * w.idx() + rem / w.of() * w.idx() + min(rem % w.of(), w.idx());
+    else if (w.parity() == 1)
+      rows += n;
+  }
+  return (uint32_t)__reduce_add_sync(kFull, rows);
 }
 
 // The scatter cut (dx^2 + dy^2) / dz^2 < kMaxScatter bounds |dx| and |dy| by
@@ -358,26 +390,36 @@ constexpr float kMinDz = 1e-3f;
 // Events within this of the origin (mm) take the pair seeding.
 constexpr float kMaxCoordinate = 1e4f;
 
-// Track forwarding onto module m4 (Kernel.cl:210-367), one warp at a time:
-// lane j forwards entry i0 + j of buffer b.  Track numbers, ring slots and
-// weak slots are reserved with one atomic per warp; new entries go to the
-// front of buffer nb.
+// Per-warp counts of entries are summed in 16 bits: each is cut off well
+// above VELO_TTF_MODULO, where the event is flagged in any case.
+constexpr uint32_t kInflightMax = 2 * VELO_TTF_MODULO;
+
+// The unused h0s of hits [block, block + 32) of module f (Kernel.cl:720-764)
+// are dealt by rank to the warps of the module's parity; their number for
+// this warp, the hits (relative to block) in `active`.
+__device__ __forceinline__ int active_h0s(const EventView& ev, const Worker& w, int st0, int n0, int block,
+                                          uint8_t* active) {
+  __syncwarp();   // the previous block's list has been read
+  const int lane = threadIdx.x & 31;
+  const bool unused = block + lane < n0 && !(ev.useds()[st0 + block + lane] & kUsed);
+  const unsigned m = __ballot_sync(kFull, unused);
+  const int rank = __popc(m & lanemask_lt()), total = __popc(m);
+  if (unused && (rank & (w.of() - 1)) == w.idx()) active[rank / w.of()] = (uint8_t)lane;
+  __syncwarp();
+  return (total + w.of() - 1 - w.idx()) / w.of();
+}
+
+// Track forwarding of iteration f, onto module f-4 (Kernel.cl:210-367): the
+// warp's entries, 32 at a time, kept in place or moved down over dropped ones.
 template <class Shared>
-__device__ void forward_warp(const EventView& ev, Shared& s, int b, uint32_t lo_n, uint32_t i0, uint32_t ncur,
-                             int m4, int nb) {
-  enum { kNone = 0, kPushTrack, kNewTrack, kPushSkip, kWeak };
-  const uint32_t i = i0 + (threadIdx.x & 31);
-  int action = kNone;
-  uint32_t push_value = 0, trackno = 0, best_h2 = 0;
-  uint4 en = make_uint4(0, 0, 0, 0);
-  float4 line = make_float4(0.f, 0.f, 0.f, 0.f);
-  float best_z = 0.f, best_den = 0.f;
-  // the ends of module m4 for the narrowing, loaded alongside the entry
-  // (same addresses in every lane)
-  const int st4 = s.start[m4], n4 = s.num[m4];
+__device__ __forceinline__ void forward(const EventView& ev, Shared& s, Worker& w, int f) {
+  if (w.n == 0) return;   // warp-uniform
+  const int lane = threadIdx.x & 31, m4 = f - 4;
+  // the ends of module m4 for the narrowing (same addresses in every lane)
+  const int st4 = s.start[m4], n4 = s.num(m4);
   const float zmin4 = s.zmin[m4], zmax4 = s.zmax[m4];
   const bool single4 = zmin4 == zmax4;   // one z on the module
-  const bool narrow4 = ev.narrow && (s.flags[m4] & kSorted) && n4 > 0;
+  const bool narrow4 = ev.p->narrow && (s.flags[m4] & kSorted) && n4 > 0;
   const float* x4 = ev.xs() + st4;
   const float* y4 = ev.ys() + st4;
   const float* z4 = ev.zs() + st4;
@@ -386,124 +428,134 @@ __device__ void forward_warp(const EventView& ev, Shared& s, int b, uint32_t lo_
     x4_first = x4[0];
     x4_last = x4[n4 - 1];
   }
-  if (i < ncur) {
-    const uint32_t at = ring_index(ev, lo_n, i);
-    en = ring_words(ev, b)[at];
-    line = ring_lines(ev, b)[at];
-    const uint32_t full = en.x;
-    const bool is_tracklet = (full & kTrackletFlag) != 0;
-    const uint32_t skipped = (full & kSkipMask) >> 28;
-    trackno = full & kEntryNumber;
-    const uint32_t n = is_tracklet ? 3u : (full >> kEntryCountShift) & 31u;
-    const float h0z = __uint_as_float(en.z), h1z = __uint_as_float(en.w);
-    int k = 0;
-    float ht = __int_as_float(0x7f800000);   // +inf: every hit from k on is tried
-    bool all_fits = true;                    // every fit is evaluated, for its finiteness
-    if (narrow4) {
-      const float dza = fsub(zmin4, h0z), dzb = fsub(zmax4, h0z);
-      const float xa = fadd(line.x, fmul(line.z, dza));
-      const float xb = single4 ? xa : fadd(line.x, fmul(line.z, dzb));
-      const float d_lo = fsub(zmin4, h1z), d_hi = fsub(zmax4, h1z);
-      const float reach = fmul(kScatterReach, fmaxf(fabsf(d_lo), fabsf(d_hi)));
-      const float ymax = fadd(fabsf(line.y), fmul(fabsf(line.w), fmaxf(fabsf(dza), fabsf(dzb))));
-      // the fits outside the cuts are known to be finite
-      const bool tame = ev.tame && (d_lo > kMinDz || d_hi < -kMinDz) && ymax < 1e15f;
-      const float tol = tame ? fminf(kTolerance, reach) : kTolerance;
-      const float xl = fminf(xa, xb), xh = fmaxf(xa, xb);
-      const float margin = fadd(0.01f, fmul(1e-5f, fadd(fabsf(xl), fabsf(xh))));
-      const float lt = fsub(fsub(xl, tol), margin);
-      const float h = fadd(fadd(xh, tol), margin);
-      if (isfinite(xa) && isfinite(xb) && isfinite(lt) && isfinite(h)) {
-        ht = h;
-        all_fits = !tame;
-        k = x4_last <= lt || x4_first > ht ? n4 : first_gt(x4, 0, n4, lt);
-      }
-    }
-    // fitHitToTrack (Kernel.cl:15-35) over the candidates, first minimum wins.
-    // The scatter's 1/(z2 - z1) depends only on z2 here: it is recomputed only
-    // when z2's bit pattern changes (same operands, same rounded value).
-    float best = FLT_MAX;
-    int best_k = -1;
-    bool degenerate = false;
-    uint32_t zc = 0x7fc00001u;   // bit pattern of the z2 the cached factor belongs to (none yet)
-    float den = 0.f;
-    for (; k < n4; ++k) {
-      const float h2x = x4[k];
-      if (h2x > ht) break;
-      const float h2z = single4 ? zmin4 : z4[k];
-      const float dz = fsub(h2z, h0z);
-      const float dx = fabsf(fsub(fadd(line.x, fmul(line.z, dz)), h2x));
-      const float dy = fabsf(fsub(fadd(line.y, fmul(line.w, dz)), y4[k]));
-      const bool near = dx < kTolerance && dy < kTolerance;
-      if (near || all_fits) {
-        if (__float_as_uint(h2z) != zc) {
-          zc = __float_as_uint(h2z);
-          den = fdiv(1.f, fsub(h2z, h1z));
-        }
-        const float scatter = fmul(fmul(fadd(fmul(dx, dx), fmul(dy, dy)), den), den);
-        if (near && scatter < kMaxScatter) {
-          if (scatter < best) { best = scatter; best_k = k; best_z = h2z; best_den = den; }
-        } else if (!isfinite(scatter)) {
-          degenerate = true;   // the reference's `condition*scatter + !condition*MAX` is NaN here
+  const uint32_t n = w.n;
+  uint32_t kept = 0;
+  for (uint32_t i0 = 0; i0 < n; i0 += 32) {   // warp-uniform
+    const uint32_t i = i0 + lane;
+    bool keep = false, changed = false, promote = false, weak = false;
+    uint4 en = make_uint4(0, 0, 0, 0);
+    float4 line = make_float4(0.f, 0.f, 0.f, 0.f);
+    uint32_t found = 0;
+    if (i < n) {
+      en = ev.entry_words()[w.row + i];
+      line = ev.entry_lines()[w.row + i];
+      const bool is_tracklet = (en.x & kTrackletFlag) != 0;
+      const float h0z = __uint_as_float(en.z), h1z = __uint_as_float(en.w);
+      int k = 0;
+      float ht = __int_as_float(0x7f800000);   // +inf: every hit from k on is tried
+      bool all_fits = true;                    // every fit is evaluated, for its finiteness
+      if (narrow4) {
+        const float dza = fsub(zmin4, h0z), dzb = fsub(zmax4, h0z);
+        const float xa = fadd(line.x, fmul(line.z, dza));
+        const float xb = single4 ? xa : fadd(line.x, fmul(line.z, dzb));
+        const float d_lo = fsub(zmin4, h1z), d_hi = fsub(zmax4, h1z);
+        const float reach = fmul(kScatterReach, fmaxf(fabsf(d_lo), fabsf(d_hi)));
+        const float ymax = fadd(fabsf(line.y), fmul(fabsf(line.w), fmaxf(fabsf(dza), fabsf(dzb))));
+        // the fits outside the cuts are known to be finite
+        const bool tame = ev.tame && (d_lo > kMinDz || d_hi < -kMinDz) && ymax < 1e15f;
+        const float tol = tame ? fminf(kTolerance, reach) : kTolerance;
+        const float xl = fminf(xa, xb), xh = fmaxf(xa, xb);
+        const float margin = fadd(0.01f, fmul(1e-5f, fadd(fabsf(xl), fabsf(xh))));
+        const float lt = fsub(fsub(xl, tol), margin);
+        const float h = fadd(fadd(xh, tol), margin);
+        if (isfinite(xa) && isfinite(xb) && isfinite(lt) && isfinite(h)) {
+          ht = h;
+          all_fits = !tame;
+          k = x4_last <= lt || x4_first > ht ? n4 : first_gt(x4, 0, n4, lt);
         }
       }
-    }
-    if (degenerate) atomicOr(&s.status, VELO_EVENT_DEGENERATE);
+      // fitHitToTrack (Kernel.cl:15-35) over the candidates, first minimum wins.
+      // The scatter's 1/(z2 - z1) depends only on z2 here: it is recomputed only
+      // when z2's bit pattern changes (same operands, same rounded value).
+      float best = FLT_MAX, best_z = 0.f, best_den = 0.f;
+      int best_k = -1;
+      bool degenerate = false;
+      uint32_t zc = 0x7fc00001u;   // bit pattern of the z2 the cached factor belongs to (none yet)
+      float den = 0.f;
+      for (; k < n4; ++k) {
+        const float h2x = x4[k];
+        if (h2x > ht) break;
+        const float h2z = single4 ? zmin4 : z4[k];
+        const float dz = fsub(h2z, h0z);
+        const float dx = fabsf(fsub(fadd(line.x, fmul(line.z, dz)), h2x));
+        const float dy = fabsf(fsub(fadd(line.y, fmul(line.w, dz)), y4[k]));
+        const bool near = dx < kTolerance && dy < kTolerance;
+        if (near || all_fits) {
+          if (__float_as_uint(h2z) != zc) {
+            zc = __float_as_uint(h2z);
+            den = fdiv(1.f, fsub(h2z, h1z));
+          }
+          const float scatter = fmul(fmul(fadd(fmul(dx, dx), fmul(dy, dy)), den), den);
+          if (near && scatter < kMaxScatter) {
+            if (scatter < best) { best = scatter; best_k = k; best_z = h2z; best_den = den; }
+          } else if (!isfinite(scatter)) {
+            degenerate = true;   // the reference's `condition*scatter + !condition*MAX` is NaN here
+          }
+        }
+      }
+      if (degenerate) atomicOr(&s.status, VELO_EVENT_DEGENERATE);
 
-    if (best_k >= 0) {
-      best_h2 = (uint32_t)(st4 + best_k);
-      if (n >= VELO_MAX_TRACK_SIZE) {   // the reference writes past hits[24] here
-        atomicOr(&s.status, VELO_EVENT_TRACK_OVERFLOW);
-      } else {
-        ev.useds()[best_h2] = 1;
-        // the entry's next line: through its last hit and the one found, whose
-        // 1 / (z2 - z1) is the fit's own
-        const float h1x = ev.xs()[en.y], h1y = ev.ys()[en.y];
-        line = line_through(h1x, h1y, x4[best_k], y4[best_k], best_den);
-        if (is_tracklet) {   // third -> fourth hit: a track is allocated below; hits 0-2 marked
-          action = kNewTrack;
+      if (best_k >= 0) {
+        const uint32_t hits = is_tracklet ? 3u : (en.x >> kEntryCountShift) & 31u;
+        if (hits >= VELO_MAX_TRACK_SIZE) {   // the reference writes past hits[24] here
+          atomicOr(&s.status, VELO_EVENT_TRACK_OVERFLOW);
         } else {
-          velo_track& t = ev.tracks[trackno];
-          t.hits[n] = best_h2;
-          t.hitsNum = n + 1;
-          action = kPushTrack;
-          push_value = trackno | ((n + 1u) << kEntryCountShift);
+          found = (uint32_t)(st4 + best_k);
+          ev.useds()[found] = kUsed;
+          // the entry's next line: through its last hit and the one found, whose
+          // 1 / (z2 - z1) is the fit's own
+          const uint32_t h1 = en.y & kEntryHit;
+          line = line_through(ev.xs()[h1], ev.ys()[h1], x4[best_k], y4[best_k], best_den);
+          keep = changed = true;
+          promote = is_tracklet;   // third -> fourth hit: a track is made below
+          if (!is_tracklet) {
+            velo_track& t = ev.tracks()[w.row + (en.x & kEntryNumber)];
+            t.hits[hits] = found;
+            t.hitsNum = hits + 1;
+            en.x += 1u << kEntryCountShift;
+          }
+          en.y = found | ((uint32_t)f << kEntryIterationShift);
+          en.z = en.w;
+          en.w = __float_as_uint(best_z);
         }
+      } else {
+        // dropped when it has skipped more than kMaxSkippedModules before this one
+        keep = (en.y >> kEntryIterationShift) - 1u - (uint32_t)f <= kMaxSkippedModules;
+        weak = !keep && is_tracklet;
       }
-    } else if (skipped <= kMaxSkippedModules) {
-      action = kPushSkip;
-      push_value = ((skipped + 1u) << 28) | (full & 0x8FFFFFFFu);
-    } else if (is_tracklet) {
-      action = kWeak;
     }
-  }
-  // new tracks (Kernel.cl:324-337); the words past the last hit are cleared
-  // when the track is written out
-  const uint32_t tn = warp_reserve(&s.ntracks, action == kNewTrack);
-  if (action == kNewTrack) {
-    const uint4 tl = ev.tracklets[trackno];
-    ev.useds()[tl.x] = 1;
-    ev.useds()[tl.y] = 1;
-    ev.useds()[tl.z] = 1;
-    if (tn < ev.cap) {
-      uint32_t* w = reinterpret_cast<uint32_t*>(&ev.tracks[tn]);
-      w[0] = 4; w[1] = tl.x; w[2] = tl.y; w[3] = tl.z; w[4] = best_h2;
-      push_value = tn | (4u << kEntryCountShift);
-    } else {
-      action = kNone;
+    // new tracks (Kernel.cl:324-337); the words past the last hit are cleared
+    // when the track is written out
+    const unsigned pm = __ballot_sync(kFull, promote);
+    if (promote) {
+      const uint4 tl = ev.tracklets()[w.row + (en.x & kEntryNumber)];
+      ev.useds()[tl.x] = kUsed;
+      ev.useds()[tl.y] = kUsed;
+      ev.useds()[tl.z] = kUsed;
+      const uint32_t tn = w.tracks + (uint32_t)__popc(pm & lanemask_lt());
+      uint32_t* t = reinterpret_cast<uint32_t*>(&ev.tracks()[w.row + tn]);
+      t[0] = 4; t[1] = tl.x; t[2] = tl.y; t[3] = tl.z; t[4] = found;
+      en.x = tn | (4u << kEntryCountShift);
     }
+    w.tracks += __popc(pm);
+    // three-hit tracklets that ran out of skips (Kernel.cl:359-363)
+    const unsigned wm = __ballot_sync(kFull, weak);
+    if (weak) ev.weak()[w.row + w.weak + (uint32_t)__popc(wm & lanemask_lt())] = en.x & kEntryNumber;
+    w.weak += __popc(wm);
+    // entries to follow in the next iteration (Kernel.cl:344-355): every lane
+    // has read its own, and slots below i0 are done with
+    const unsigned km = __ballot_sync(kFull, keep);
+    const uint32_t to = kept + (uint32_t)__popc(km & lanemask_lt());
+    if (keep && (changed || to != i)) {
+      ev.entry_words()[w.row + to] = en;
+      ev.entry_lines()[w.row + to] = line;
+    }
+    kept += __popc(km);
+    __syncwarp();
   }
-  // tracks to follow in the next iteration (Kernel.cl:344-355)
-  const bool push = action == kPushTrack || action == kNewTrack || action == kPushSkip;
-  const uint32_t slot = warp_reserve(&s.ring_lo[nb], push);
-  if (push && slot < ev.ring_cap) {   // a skip keeps the hits; a new hit shifts them
-    ring_words(ev, nb)[slot] = action == kPushSkip ? make_uint4(push_value, en.y, en.z, en.w)
-                                                   : make_uint4(push_value, best_h2, en.w, __float_as_uint(best_z));
-    ring_lines(ev, nb)[slot] = line;
-  }
-  // three-hit tracklets that ran out of skips (Kernel.cl:359-363)
-  const uint32_t wi = warp_reserve(&s.nweak, action == kWeak);
-  if (action == kWeak && wi < ev.cap) ev.weak[wi] = trackno;
+  w.n = kept;
+  if (ev.H > VELO_TTF_MODULO / 2 && lane == 0)   // smaller events cannot overrun the reference's buffer
+    atomicAdd(&s.inflight[f], min(n, kInflightMax) | (min(n + kept, kInflightMax) << 16));
 }
 
 // Features of an (h0, h1) doublet seen by the learned seeding (and recorded
@@ -595,19 +647,19 @@ static __device__ __noinline__ float2 score_doublets(const MlpFrag* mlp, bool sc
 // host allows G < 32 only where Y divides G, so that a lane's Y-lane is the
 // same in every chunk.  New tracklets go to the back of ring[nb].
 template <int kMode, int G, class Shared>
-__device__ void seed_module(const EventView& ev, Shared& s, int f, int nb, const SeedLanes& sl) {
+__device__ void seed_module(const EventView& ev, Shared& s, Worker& w, int f, const SeedLanes& sl) {
   constexpr int kShift = G == 8 ? 3 : G == 16 ? 4 : 5;
   constexpr int kGroups = 32 / G;
   static_assert(G == 8 || G == 16 || G == 32, "8, 16 or 32 lanes per h0");
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31;
   const int jl = lane & (G - 1);
-  const int st0 = s.start[f], n0 = s.num[f];
+  const int st0 = s.start[f], n0 = s.num(f);
   const int s1 = f - 2, m4 = f - 4;
-  const int st1 = s.start[s1], st4 = s.start[m4], n4 = s.num[m4];
-  const uint32_t Y = (uint32_t)ev.Y;
+  const int st1 = s.start[s1], st4 = s.start[m4], n4 = s.num(m4);
+  const uint32_t Y = (uint32_t)ev.p->y_lanes;
   const uint32_t chunk_step = G == 32 ? 32u % Y : 0u;   // how far the Y-lanes turn per chunk
-  const float s1_z = s.num[s1] > 0 ? ev.zs()[st1] : 0.f;   // Kernel.cl:420
-  const bool narrow4 = ev.narrow && (s.flags[m4] & kSorted) && n4 > 0;
+  const float s1_z = s.num(s1) > 0 ? ev.zs()[st1] : 0.f;   // Kernel.cl:420
+  const bool narrow4 = ev.p->narrow && (s.flags[m4] & kSorted) && n4 > 0;
   const float zmin4 = s.zmin[m4], zmax4 = s.zmax[m4];
   const float* x4 = ev.xs() + st4;
   const float* y4 = ev.ys() + st4;
@@ -618,41 +670,21 @@ __device__ void seed_module(const EventView& ev, Shared& s, int f, int nb, const
   uint32_t zk0 = 0x7fc00001u, zk1 = 0x7fc00001u;
   float dz_inv_cached = 0.f;
 
-  // G = 32: h0s dealt to the warps in turn; G < 32: each warp claims its
-  // next 32 / G h0s from a shared counter (one atomic per warp and claim),
-  // which evens out the warps' work before the barrier that ends seeding
-  int ib = G == 32 ? warp : 0;
-  if constexpr (G < 32) {
-    if (lane == 0) ib = atomicAdd(&s.seed_next[nb ^ 1], kGroups);   // seed_next[b] of the module loop
-    ib = __shfl_sync(kFull, ib, 0);
-  }
-  for (; ib < n0;) {   // warp-uniform
-    do {   // one claim of h0s; `break` moves on to the next claim
-    int h0, n1, c_end;
-    uint32_t f1;
-    if constexpr (G == 32) {
-      h0 = st0 + ib;
-      if (ev.useds()[h0] & kUsed) break;                // warp-uniform
+  uint8_t* active = s.seed.active[w.warp()];
+  for (int block = 0; block < n0; block += 32)                    // warp-uniform
+  for (int c0 = 0, mine = active_h0s(ev, w, st0, n0, block, active); c0 < mine; c0 += kGroups) {
+    int h0 = 0, n1 = 0;
+    uint32_t f1 = 0;
+    if (c0 + lane / G < mine) {
+      h0 = st0 + block + active[c0 + lane / G];
       const uint32_t w0 = ev.wins()[h0].x;
       f1 = w0 & 0xffffu;
-      if (f1 == kNone16) break;
-      n1 = (int)(w0 >> 16) - (int)f1;                   // > 0 when a first hit was found
-      c_end = n1;
-    } else {
-      h0 = st0 + ib + (lane >> kShift);
-      n1 = 0;
-      f1 = 0;
-      if (h0 < st0 + n0 && !(ev.useds()[h0] & kUsed)) {
-        const uint32_t w0 = ev.wins()[h0].x;
-        f1 = w0 & 0xffffu;
-        if (f1 != kNone16) n1 = (int)(w0 >> 16) - (int)f1;
-      }
-      const int chunks = (int)__reduce_max_sync(kFull, (uint32_t)((n1 + G - 1) >> kShift));
-      if (chunks == 0) break;                           // warp-uniform
-      c_end = chunks << kShift;
+      if (f1 != kNone16) n1 = (int)(w0 >> 16) - (int)f1;
     }
+    const int c_end = G * (int)__reduce_max_sync(kFull, (uint32_t)((n1 + G - 1) >> kShift));
+    if (c_end == 0) continue;                           // warp-uniform
     float h0x = 0.f, h0y = 0.f, h0z = 0.f;
-    if (G == 32 || n1 > 0) {
+    if (n1 > 0) {
       h0x = ev.xs()[h0];
       h0y = ev.ys()[h0];
       h0z = ev.zs()[h0];
@@ -714,28 +746,28 @@ __device__ void seed_module(const EventView& ev, Shared& s, int f, int nb, const
           hs ^= hs >> 15;
           hs *= 0x2C1B3C6Du;
           hs ^= hs >> 12;
-          if (hs % ev.dump_keep == 0u) {
-            const unsigned long long k = atomicAdd(ev.dump_count, 1ull);
-            if (k < ev.dump_capacity) {
+          if (hs % max(ev.p->dump_keep, 1u) == 0u) {
+            const unsigned long long k = atomicAdd(ev.p->dump_count, 1ull);
+            if (k < ev.p->dump_capacity) {
 #pragma unroll
-              for (int q = 0; q < kMlpIn; ++q) ev.dump_features[k * kMlpIn + q] = feat[q];
-              ev.dump_ids[3 * k + 0] = (uint32_t)ev.event;
-              ev.dump_ids[3 * k + 1] = (uint32_t)h0;
-              ev.dump_ids[3 * k + 2] = (uint32_t)h1;
+              for (int q = 0; q < kMlpIn; ++q) ev.p->dump_features[k * kMlpIn + q] = feat[q];
+              ev.p->dump_ids[3 * k + 0] = (uint32_t)ev.event;
+              ev.p->dump_ids[3 * k + 1] = (uint32_t)h0;
+              ev.p->dump_ids[3 * k + 2] = (uint32_t)h1;
             }
           }
         }
       }
       if constexpr (kMode == kLearned) {
         // only doublets with a wide exact h2 window are worth scoring
-        const bool score = cand && b - a >= ev.learned_min_window;
+        const bool score = cand && b - a >= ev.p->learned_min_window;
         bool keep = true;
         if (__any_sync(kFull, score)) {             // the warp scores its doublets together
           const float2 r = score_doublets(ev.mlp, score, h0x, h0y, h0z, h1x, h1y, h1z, dz_inverted,
                                           0.5f * (zmin4 + zmax4), b - a, f, ev.S, dymax);
           if (score) {
-            keep = r.x >= ev.keep_threshold;
-            tol = fminf(kTolerance, fmaxf(r.y, 0.f) + ev.window_margin);
+            keep = r.x >= ev.p->keep_threshold;
+            tol = fminf(kTolerance, fmaxf(r.y, 0.f) + ev.p->window_margin);
           }
         }
         // keep-rate bookkeeping for the guard: the scored doublets
@@ -803,38 +835,10 @@ __device__ void seed_module(const EventView& ev, Shared& s, int f, int nb, const
       for (int o = G >> 1; o > 0; o >>= 1) lmin = min(lmin, __shfl_xor_sync(kFull, lmin, o));
     }
     best = ((unsigned long long)hmin << 32) | lmin;
-    // Kernel.cl:550-567: each group's first lane appends its tracklet
-    if constexpr (G == 32) {
-      if (lane == 0 && best != ~0ull) {
-        const uint32_t e = (uint32_t)(best >> 14) & 0x3fffu;
-        const uint32_t h1 = (uint32_t)(st1 + (int)f1) + e;
-        const uint32_t h2 = (uint32_t)st4 + (uint32_t)(best & 0x3fffu);
-        const uint32_t tp = atomicAdd(&s.ntracklets, 1u);
-        if (tp < ev.cap) {
-          ev.tracklets[tp] = make_uint4((uint32_t)h0, h1, h2, 0u);
-          push_back(s, ev, nb, tp, h1, h2);
-        }
-      }
-    } else {   // one shared-memory atomic per warp for the tracklet rows, one for the ring
-      const bool win = jl == 0 && best != ~0ull;
-      const uint32_t tp = warp_reserve(&s.ntracklets, win);
-      const bool push = win && tp < ev.cap;
-      const uint32_t ri = warp_reserve(&s.ring_hi[nb], push);
-      if (push) {
-        const uint32_t e = (uint32_t)(best >> 14) & 0x3fffu;
-        const uint32_t h1 = (uint32_t)(st1 + (int)f1) + e;
-        const uint32_t h2 = (uint32_t)st4 + (uint32_t)(best & 0x3fffu);
-        ev.tracklets[tp] = make_uint4((uint32_t)h0, h1, h2, 0u);
-        if (ri < ev.ring_cap) write_tracklet_entry(ev, nb, ev.ring_cap - 1u - ri, tp, h1, h2);
-      }
-    }
-    } while (0);
-    if constexpr (G == 32) {
-      ib += nwarps;
-    } else {
-      if (lane == 0) ib = atomicAdd(&s.seed_next[nb ^ 1], kGroups);
-      ib = __shfl_sync(kFull, ib, 0);
-    }
+    // each group's first lane appends its tracklet
+    const uint32_t h1 = (uint32_t)(st1 + (int)f1) + ((uint32_t)(best >> 14) & 0x3fffu);
+    append_tracklets(ev, w, jl == 0 && best != ~0ull, (uint32_t)h0, h1,
+                     (uint32_t)st4 + (uint32_t)(best & 0x3fffu), f);
   }
   if (degenerate) atomicOr(&s.status, VELO_EVENT_DEGENERATE);
 }
@@ -842,8 +846,9 @@ __device__ void seed_module(const EventView& ev, Shared& s, int f, int nb, const
 // seed_module for the events that the pair seeding does not take, out of
 // line, so that the module loop keeps its registers.
 template <int kMode, int G, class Shared>
-__device__ __noinline__ void seed_windows(const EventView ev, Shared& s, int f, int nb) {
-  seed_module<kMode, G>(ev, s, f, nb, seed_lanes_of(G, (uint32_t)ev.Y));
+__device__ __noinline__ Worker seed_windows(const EventView ev, Shared& s, Worker w, int f) {
+  seed_module<kMode, G>(ev, s, w, f, seed_lanes_of(G, (uint32_t)ev.p->y_lanes));
+  return w;
 }
 
 // The candidate windows of every hit (all threads of the CTA).
@@ -927,10 +932,10 @@ __device__ __forceinline__ void h2_bounds(float x, float z, int sz0, int sz2, fl
 // Kernel.cl:104,137).
 template <class Shared>
 __device__ __forceinline__ bool h1_dead(const EventView& ev, const Shared& s, int m, int h) {
-  if (m < 4 || m > ev.S - 3 || s.num[m - 2] == 0) return true;
+  if (m < 4 || m > ev.S - 3 || s.num(m - 2) == 0) return true;
   float lo, hi;
   h2_bounds(ev.xs()[h], ev.zs()[h], s.sz[m + 2], s.sz[m - 2], &lo, &hi);
-  return !(ev.xs()[s.start[m - 2] + s.num[m - 2] - 1] > lo);
+  return !(ev.xs()[s.start[m - 2] + s.num(m - 2) - 1] > lo);
 }
 
 // The h1 window of an h0 at (x0, z0) on x-sorted module s1: the first hit
@@ -940,7 +945,7 @@ __device__ __forceinline__ bool h1_dead(const EventView& ev, const Shared& s, in
 template <class Shared>
 __device__ __forceinline__ void h1_window(const EventView& ev, const Shared& s, int s1, float x0, float z0,
                                           int* first, int* last) {
-  const int st = s.start[s1], n = s.num[s1];
+  const int st = s.start[s1], n = s.num(s1);
   const float* x = ev.xs() + st;
   if (s.zmin[s1] == s.zmax[s1]) {
     const float dxmax = fmul(kMaxXSlopeCandidates, fabsf(fsub(s.zmin[s1], z0)));
@@ -971,37 +976,35 @@ __device__ __forceinline__ void h1_window(const EventView& ev, const Shared& s, 
   }
 }
 
-template <class Shared, class Seed>
-__device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Seed& sd, int f, int nb) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+template <class Shared>
+__device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Worker& w, int f) {
+  constexpr int kOwn = Shared::kOwn;
+  auto& sd = s.seed;
+  const int lane = threadIdx.x & 31;
   const int s1 = f - 2, m4 = f - 4;
-  const int st0 = s.start[f], n0 = s.num[f], st1 = s.start[s1], st4 = s.start[m4], n4 = s.num[m4];
+  const int st0 = s.start[f], n0 = s.num(f), st1 = s.start[s1], st4 = s.start[m4], n4 = s.num(m4);
   const float zmin1 = s.zmin[s1], zmin4 = s.zmin[m4], zmax4 = s.zmax[m4];
   const bool single1 = zmin1 == s.zmax[s1], single4 = zmin4 == zmax4;
   const bool use_map = map_valid(s, s1, m4);
-  const uint32_t* map = sd.map[f & 1];
+  const uint32_t* map = sd.map[w.parity()];
+  float4* own_h0 = sd.h0[w.warp()];
+  float2* own_reach = sd.reach[w.warp()];
+  unsigned long long* own_best = sd.best[w.warp()];
+  uint16_t* own_first = sd.first[w.warp()];
   const float* x4 = ev.xs() + st4;
   const float* y4 = ev.ys() + st4;
   const float* z4 = ev.zs() + st4;
-  const uint32_t Y = (uint32_t)ev.Y;
-  if (n0 == 0 || n4 == 0 || s.num[s1] == 0) return;
+  const uint32_t Y = (uint32_t)ev.p->y_lanes;
+  if (n0 == 0 || n4 == 0 || s.num(s1) == 0) return;
   const float s1_z = ev.zs()[st1];   // Kernel.cl:420
   bool degenerate = false;
 
-  for (int block = 0; block < n0; block += 32) {   // warp-uniform
-    __syncwarp();   // the previous block's reads of the lists are done
-    // the block's unused h0s, dealt to the warps by rank
-    const int i0 = block + lane;
-    const bool unused = i0 < n0 && !(ev.useds()[st0 + i0] & kUsed);
-    const unsigned um = __ballot_sync(kFull, unused);
-    const int rank = __popc(um & lanemask_lt());
-    if (unused && (rank & (nwarps - 1)) == warp) sd.active[rank] = (uint16_t)i0;
-    __syncwarp();
-    const int mine = warp + lane * nwarps;
+  for (int block = 0; block < n0; block += 32)   // warp-uniform
+  for (int c0 = 0, mine = active_h0s(ev, w, st0, n0, block, sd.active[w.warp()]); c0 < mine; c0 += kOwn) {
     int h0 = 0, first = 0, count = 0;
     float h0x = 0.f, h0y = 0.f, h0z = 0.f;
-    if (mine < __popc(um)) {
-      h0 = st0 + sd.active[mine];
+    if (lane < kOwn && c0 + lane < mine) {
+      h0 = st0 + block + sd.active[w.warp()][c0 + lane];
       h0x = ev.xs()[h0];
       h0y = ev.ys()[h0];
       h0z = ev.zs()[h0];
@@ -1020,13 +1023,14 @@ __device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Seed&
     if (total == 0) continue;
     const int begin = end - count;
     const unsigned om = __ballot_sync(kFull, count > 0);
-    const int slot = warp + __popc(om & lanemask_lt()) * nwarps;   // below 32: the warp's ranks leave it that many
+    const int slot = __popc(om & lanemask_lt());
+    __syncwarp();   // the previous round's lists have been read
     if (count > 0) {
-      sd.h0[slot] = make_float4(h0x, h0y, h0z, __int_as_float(st1 + first - begin));
-      sd.reach[slot] = make_float2(fmul(kMaxYSlope, fabsf(fsub(s1_z, h0z))),
+      own_h0[slot] = make_float4(h0x, h0y, h0z, __int_as_float(st1 + first - begin));
+      own_reach[slot] = make_float2(fmul(kMaxYSlope, fabsf(fsub(s1_z, h0z))),
                                    fmul(fsub(zmin4, h0z), fdiv(1.f, fsub(zmin1, h0z))));
-      sd.best[slot] = ~0ull;
-      sd.first[slot] = (uint16_t)first;
+      own_best[slot] = ~0ull;
+      own_first[slot] = (uint16_t)first;
     }
     __syncwarp();
 
@@ -1042,8 +1046,8 @@ __device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Seed&
         o = owners + __popc(starts & (2u * (1u << lane) - 1u)) - 1;
         owners += __popc(starts);
         if (base + lane < total) {
-          const float4 q = sd.h0[warp + o * nwarps];
-          const float2 r = sd.reach[warp + o * nwarps];
+          const float4 q = own_h0[o];
+          const float2 r = own_reach[o];
           h1 = __float_as_int(q.w) + base + lane;
           const uint8_t u1 = ev.useds()[h1];
           const float h1x = ev.xs()[h1], h1y = ev.ys()[h1];
@@ -1058,17 +1062,17 @@ __device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Seed&
       const unsigned pm = __ballot_sync(kFull, pass);
       if (queued + __popc(pm) > kQueue || !more) {   // warp-uniform
         __syncwarp();
-        const uint32_t entry = sd.queue[warp][lane];
-        const int own = warp + (int)(entry >> 14) * nwarps;
+        const uint32_t entry = sd.queue[w.warp()][lane];
+        const int own = (int)(entry >> 14);
         const int local1 = (int)(entry & 0x3fffu), hit1 = st1 + local1;
         // a Y-lane stops at its first dead h1: where the dead h1s are not the
         // module's last ones, look for one before this pair's
         bool reached = lane < queued;
         if (!(s.flags[s1] & kDeadTail) && reached)
-          for (int e = local1 - (int)Y; e >= (int)sd.first[own]; e -= (int)Y) reached &= !h1_dead(ev, s, s1, st1 + e);
+          for (int e = local1 - (int)Y; e >= (int)own_first[own]; e -= (int)Y) reached &= !h1_dead(ev, s, s1, st1 + e);
         if (reached) {
           // Kernel.cl:468-529 for one (h0, h1): the fits of the h2s in reach
-          const float4 q = sd.h0[own];
+          const float4 q = own_h0[own];
           const float h1x = ev.xs()[hit1], h1y = ev.ys()[hit1], h1z = single1 ? zmin1 : ev.zs()[hit1];
           const float dz_inverted = fdiv(1.f, fsub(h1z, q.z));
           const float ddx = fsub(h1x, q.x), ddy = fsub(h1y, q.y);
@@ -1121,8 +1125,8 @@ __device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Seed&
             }
           }
           if (best_k >= 0) {   // smallest fit, then Y-lane, h1, h2
-            const uint32_t e = (uint32_t)local1 - sd.first[own];
-            atomicMin(&sd.best[own], ((unsigned long long)__float_as_uint(best) << 32) |
+            const uint32_t e = (uint32_t)local1 - own_first[own];
+            atomicMin(&own_best[own], ((unsigned long long)__float_as_uint(best) << 32) |
                                          ((unsigned long long)(e % Y) << 28) | ((unsigned long long)e << 14) |
                                          (unsigned long long)best_k);
           }
@@ -1131,21 +1135,12 @@ __device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Seed&
         __syncwarp();
       }
       if (!more) break;
-      if (pass) sd.queue[warp][queued + __popc(pm & lanemask_lt())] = ((uint32_t)o << 14) | (uint32_t)(h1 - st1);
+      if (pass) sd.queue[w.warp()][queued + __popc(pm & lanemask_lt())] = ((uint32_t)o << 14) | (uint32_t)(h1 - st1);
       queued += __popc(pm);
     }
-    // Kernel.cl:550-567: one shared-memory atomic per warp for the tracklet rows, one for the ring
-    const unsigned long long best = count > 0 ? sd.best[slot] : ~0ull;
-    const bool win = best != ~0ull;
-    const uint32_t tp = warp_reserve(&s.ntracklets, win);
-    const bool push = win && tp < ev.cap;
-    const uint32_t ri = warp_reserve(&s.ring_hi[nb], push);
-    if (push) {
-      const uint32_t h1 = (uint32_t)(st1 + first) + ((uint32_t)(best >> 14) & 0x3fffu);
-      const uint32_t h2 = (uint32_t)st4 + (uint32_t)(best & 0x3fffu);
-      ev.tracklets[tp] = make_uint4((uint32_t)h0, h1, h2, 0u);
-      if (ri < ev.ring_cap) write_tracklet_entry(ev, nb, ev.ring_cap - 1u - ri, tp, h1, h2);
-    }
+    const unsigned long long best = count > 0 ? own_best[slot] : ~0ull;
+    append_tracklets(ev, w, best != ~0ull, (uint32_t)h0, (uint32_t)(st1 + first) + ((uint32_t)(best >> 14) & 0x3fffu),
+                     (uint32_t)st4 + (uint32_t)(best & 0x3fffu), f);
   }
   if (degenerate) atomicOr(&s.status, VELO_EVENT_DEGENERATE);
 }
@@ -1156,7 +1151,7 @@ __device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Seed&
 template <class Shared>
 __device__ __forceinline__ bool clear_flags(const EventView& ev, const Shared& s, int m) {
   const int lane = threadIdx.x & 31;
-  const int st = s.start[m], n = s.num[m];
+  const int st = s.start[m], n = s.num(m);
   bool tail = true;
   unsigned before = 0;   // dead hits so far
   for (int i0 = 0; i0 < n; i0 += 32) {
@@ -1216,7 +1211,7 @@ __device__ bool sort_arena(const EventView& ev, const Shared& s, int S, uint32_t
   float* z = ev.zs();
   bool moved = false;
   for (int m = warp; m < S; m += nwarps) {   // warp-uniform
-    const int s0 = s.start[m], n = s.num[m];
+    const int s0 = s.start[m], n = s.num(m);
     if (n < 2) continue;
     if (n > kArenaRankMax) {
       bool changed = false;
@@ -1324,13 +1319,10 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
   }
   const int32_t* hdr = reinterpret_cast<const int32_t*>(p.input + p.ev_offset[e]);
   EventView ev;
+  ev.p = &p;
   ev.S = hdr[0];
   ev.H = hdr[1];
-  ev.Y = p.y_lanes;
-  ev.narrow = p.narrow != 0;
   const int S = ev.S, H = ev.H;
-  ev.cap = H > 0 ? (uint32_t)H : 1u;
-  ev.ring_cap = ev.cap;
   const int32_t* gZ = hdr + 2;
   const int32_t* gstart = gZ + S;
   const int32_t* gnum = gstart + S;
@@ -1338,39 +1330,25 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
   const float* gy = gx + H;
   const float* gz = gy + H;
 
-  const ArenaLayout L = arena_layout((uint32_t)H, p.ev_maxmod[e], (uint32_t)ev.Y);
-  uint8_t* arena = p.arena_off[e] == kNoArena ? dyn : p.global_arena + p.arena_off[e];
-  ev.arena = arena;
+  const ArenaLayout L = arena_layout((uint32_t)H, p.ev_maxmod[e], (uint32_t)p.y_lanes);
+  ev.arena = p.arena_off[e] == kNoArena ? dyn : p.global_arena + p.arena_off[e];
   ev.P = L.y;
-  const uint64_t hb = p.hit_base[e];
-  ev.rings = reinterpret_cast<uint4*>(p.rings + 16 * hb);
-  ev.tracklets = reinterpret_cast<uint4*>(p.tracklets + 4 * hb);
-  ev.weak = p.weak + hb;
-  ev.tracks = p.tracks + hb;
   ev.event = e;
   ev.mlp = mlp_smem;
-  ev.keep_threshold = p.keep_threshold;
-  ev.learned_min_window = p.learned_min_window;
-  ev.window_margin = p.window_margin;
-  ev.dump_features = p.dump_features;
-  ev.dump_ids = p.dump_ids;
-  ev.dump_count = p.dump_count;
-  ev.dump_capacity = p.dump_capacity;
-  ev.dump_keep = p.dump_keep > 0 ? p.dump_keep : 1u;
 
   // stage the event; the module table must tile [0, H) in order (the host
   // checked only the header and the blob's length)
   bool bad = tid == 0 && S == 0 && H != 0;
-  bool wild = !ev.narrow;   // the event does not take the pair seeding
+  bool wild = !ev.p->narrow;   // the event does not take the pair seeding
   for (int m = tid; m < S; m += nt) {
     const int32_t st = gstart[m], nm = gnum[m];
     const int64_t expect = m == 0 ? 0 : (int64_t)gstart[m - 1] + (int64_t)gnum[m - 1];
     bad |= nm < 0 || nm > VELO_MAX_MODULE_HITS || (int64_t)st != expect ||
            (m == S - 1 && (int64_t)st + (int64_t)nm != (int64_t)H);
     s.start[m] = st;
-    s.num[m] = nm;
     s.sz[m] = gZ[m];
   }
+  for (int m = tid; m <= S; m += nt) s.inflight[m] = 0;
   // with sort_events the IDs are staged too, in the window area (written
   // only after the sort)
   const uint32_t* gid = reinterpret_cast<const uint32_t*>(gnum + S);
@@ -1385,12 +1363,10 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
     if (p.sort_events) ids[i] = gid[i];
   }
   if (tid == 0) {
-    s.ring_lo[0] = 0; s.ring_lo[1] = 0; s.ring_hi[0] = 0; s.ring_hi[1] = 0;
-    s.ntracks = 0; s.ntracklets = 0; s.nweak = 0; s.status = 0;
+    s.start[S] = H;
+    s.status = 0;
     s.considered = 0; s.kept = 0;
-    s.seed_next[0] = 0; s.seed_next[1] = 0;
   }
-  for (int i = tid; i < 2 * kMapRows; i += nt) s.seed.map[i / kMapRows][i % kMapRows] = 0;
   if (__syncthreads_or(bad)) {   // a bad module table, or a non-finite coordinate
     if (tid == 0) {
       p.out_counts[e] = 0;
@@ -1420,7 +1396,7 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
 
   // per-module z range, x-sortedness and hit flags (one warp per module)
   for (int m = warp; m < S; m += nwarps) {
-    const int st = s.start[m], n = s.num[m];
+    const int st = s.start[m], n = s.num(m);
     float zmn = FLT_MAX, zmx = -FLT_MAX;
     bool sorted = true;
     for (int i = lane; i < n; i += 32) {
@@ -1449,7 +1425,7 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
   bool learned = kMode == kLearned && (p.learned_max_hits == 0 || (uint32_t)H <= p.learned_max_hits);
   // per-lane constants of the learned seeding's ballots
   SeedLanes sl{};
-  if constexpr (kMode == kLearned) sl = seed_lanes_of(kLanes, (uint32_t)ev.Y);
+  if constexpr (kMode == kLearned) sl = seed_lanes_of(kLanes, (uint32_t)ev.p->y_lanes);
   // candidate windows for the seedings that read them
   if (kMode != kPlain || !ev.tame) {
     fill_windows(ev, s);
@@ -1461,82 +1437,71 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
   // fraction of the doublets it scored, the event is searched again by the
   // plain method (flags and lists reset; windows kept).
   uint32_t fallback = (kMode == kLearned && !learned) ? VELO_EVENT_LEARNED_FALLBACK : 0u;
+  Worker w{};
+  w.row = (uint32_t)p.hit_base[e] + first_row(s, w, S);
   for (int attempt = 0; attempt < 2; ++attempt) {
     if (attempt > 0) {
       for (int m = warp; m < S; m += nwarps) clear_flags(ev, s, m);
-      if (tid == 0) {
-        s.ring_lo[0] = 0; s.ring_lo[1] = 0; s.ring_hi[0] = 0; s.ring_hi[1] = 0;
-        s.ntracks = 0; s.ntracklets = 0; s.nweak = 0; s.status = 0;
-        s.seed_next[0] = 0; s.seed_next[1] = 0;
-      }
+      for (int m = tid; m <= S; m += nt) s.inflight[m] = 0;
+      if (tid == 0) s.status = 0;
+      w.n = w.tracklets = w.tracks = w.weak = 0;
       __syncthreads();
     }
     const bool pairs = kMode == kPlain && ev.tame;
-    // module loop, Kernel.cl:671-767
-    int b = 0;   // ring[b] holds the entries to follow in this iteration
+    // module loop, Kernel.cl:671-767 (see Worker for the order of the warps)
     for (int f = S - 1; f >= 4; --f) {
-      // the map of the h2 module, by the last warps (the first ones have the
-      // most entries to forward)
-      if (pairs && map_valid(s, f - 2, f - 4))
-        for (int i = nt - 1 - tid; i < s.num[f - 4]; i += nt) mark_map(ev, s, s.seed.map[f & 1], f - 2, f - 4, i);
-      const uint32_t lo_n = min(s.ring_lo[b], ev.ring_cap);
-      const uint32_t ncur = min(lo_n + s.ring_hi[b], ev.ring_cap);
-      if (tid == 0 && s.ring_lo[b] + s.ring_hi[b] > VELO_TTF_MODULO) s.status |= VELO_EVENT_RING_OVERFLOW;
-      for (uint32_t i0 = (uint32_t)warp * 32u; i0 < ncur; i0 += (uint32_t)nt)   // warp-uniform
-        forward_warp(ev, s, b, lo_n, i0, ncur, f - 4, b ^ 1);
-      __syncthreads();
+      forward(ev, s, w, f);
       VELO_PHASE(3);
-      if (tid == 0) {
-        if (ncur + s.ring_lo[b ^ 1] > VELO_TTF_MODULO) s.status |= VELO_EVENT_RING_OVERFLOW;
-        // this iteration's seeding claims h0s from seed_next[b]; the next
-        // one (parity b ^ 1) from seed_next[b ^ 1], last used before the
-        // barrier that closed the previous iteration
-        s.seed_next[b ^ 1] = 0;
-        s.ring_lo[b] = 0;   // ring[b] is refilled two iterations on
-        s.ring_hi[b] = 0;
+      const int step = (S - 1 - f) & 1;
+      if (w.alone() || step == w.parity()) {
+        if (pairs) {
+          uint32_t* map = s.seed.map[w.parity()];
+          const int gt = w.idx() * 32 + lane, gn = w.of() * 32;
+          for (int i = gt; i < kMapRows; i += gn) map[i] = 0;
+          group_sync<Shared::kMaxWarps>(w);
+          if (map_valid(s, f - 2, f - 4))
+            for (int i = gt; i < s.num(f - 4); i += gn) mark_map(ev, s, map, f - 2, f - 4, i);
+          group_sync<Shared::kMaxWarps>(w);
+          seed_pairs(ev, s, w, f);
+        } else {
+          group_sync<Shared::kMaxWarps>(w);
+          if (kMode == kLearned && learned)
+            seed_module<kLearned, kLanes>(ev, s, w, f, sl);
+          else
+            w = seed_windows<kMode == kDump ? kDump : kPlain, kLanes>(ev, s, w, f);
+        }
+        group_sync<Shared::kMaxWarps>(w);
       }
-      if (pairs) {
-        for (int i = tid; i < kMapRows; i += nt) s.seed.map[(f & 1) ^ 1][i] = 0;   // for the next module
-        seed_pairs(ev, s, s.seed, f, b ^ 1);
-      } else if (s.num[f] > 0) {
-        if (kMode == kLearned && learned)
-          seed_module<kLearned, kLanes>(ev, s, f, b ^ 1, sl);
-        else
-          seed_windows<kMode == kDump ? kDump : kPlain, kLanes>(ev, s, f, b ^ 1);
-      }
-      __syncthreads();
+      if (step == 1 || f == 4) __syncthreads();
       VELO_PHASE(4);
-      b ^= 1;
     }
 
     // leftover tracklets become weak (Kernel.cl:771-792)
-    {
-      if (tid == 0 && s.ring_lo[b] + s.ring_hi[b] > VELO_TTF_MODULO) s.status |= VELO_EVENT_RING_OVERFLOW;
-      const uint32_t lo_n = min(s.ring_lo[b], ev.ring_cap);
-      const uint32_t ncur = min(lo_n + s.ring_hi[b], ev.ring_cap);
-      for (uint32_t i = tid; i < ncur; i += nt) {
-        const uint32_t v = ring_words(ev, b)[ring_index(ev, lo_n, i)].x;
-        if (v & kTrackletFlag) {
-          const uint32_t wi = atomicAdd(&s.nweak, 1u);
-          if (wi < ev.cap) ev.weak[wi] = v & kEntryNumber;
-        }
-      }
+    if (ev.H > VELO_TTF_MODULO / 2 && lane == 0) atomicAdd(&s.inflight[3], min(w.n, kInflightMax));
+    for (uint32_t i0 = 0; i0 < w.n; i0 += 32) {   // warp-uniform
+      const uint32_t v = i0 + lane < w.n ? ev.entry_words()[w.row + i0 + lane].x : 0u;
+      const unsigned m = __ballot_sync(kFull, (v & kTrackletFlag) != 0);
+      if (v & kTrackletFlag) ev.weak()[w.row + w.weak + (uint32_t)__popc(m & lanemask_lt())] = v & kEntryNumber;
+      w.weak += __popc(m);
     }
-    __syncthreads();
+    __syncwarp();
     // weak tracks made of three unused hits (Kernel.cl:796-815)
-    {
-      const uint32_t nweak = min(s.nweak, ev.cap);
-      for (uint32_t i = tid; i < nweak; i += nt) {
-        const uint4 t = ev.tracklets[ev.weak[i]];
-        const uint32_t a = t.x, bb = t.y, c = t.z;
-        if (((ev.useds()[a] | ev.useds()[bb] | ev.useds()[c]) & kUsed) == 0) {
-          const uint32_t tn = atomicAdd(&s.ntracks, 1u);
-          if (tn >= ev.cap) continue;
-          uint32_t* wr = reinterpret_cast<uint32_t*>(&ev.tracks[tn]);
-          wr[0] = 3; wr[1] = a; wr[2] = bb; wr[3] = c;
-        }
+    for (uint32_t i0 = 0; i0 < w.weak; i0 += 32) {
+      uint4 t = make_uint4(0, 0, 0, 0);
+      bool take = false;
+      if (i0 + lane < w.weak) {
+        t = ev.tracklets()[w.row + ev.weak()[w.row + i0 + lane]];
+        take = ((ev.useds()[t.x] | ev.useds()[t.y] | ev.useds()[t.z]) & kUsed) == 0;
       }
+      const unsigned m = __ballot_sync(kFull, take);
+      if (take) {
+        uint32_t* wr =
+            reinterpret_cast<uint32_t*>(&ev.tracks()[w.row + w.tracks + (uint32_t)__popc(m & lanemask_lt())]);
+        wr[0] = 3; wr[1] = t.x; wr[2] = t.y; wr[3] = t.z;
+      }
+      w.tracks += __popc(m);
     }
+    if (lane == 0) s.tracks[warp] = w.tracks;
     __syncthreads();
     VELO_PHASE(5);
     if (!learned) break;
@@ -1547,32 +1512,44 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
     __syncthreads();   // everyone has read the counters before the reset
   }
 
-  // compacted output: one atomic per event reserves its range
+  // compacted output: one atomic per event reserves its range, the warps'
+  // tracks one after another
+  uint32_t count = 0, before = 0;
+  for (int k = 0; k < nwarps; ++k) {
+    const uint32_t c = s.tracks[k];
+    if (k < warp) before += c;
+    count += c;
+  }
+  if (H > VELO_TTF_MODULO / 2)   // Kernel.cl:344,354,565
+    for (int f = 3 + tid; f < S; f += nt)
+      if ((s.inflight[f] & 0xffffu) > VELO_TTF_MODULO || (s.inflight[f] >> 16) > VELO_TTF_MODULO)
+        atomicOr(&s.status, VELO_EVENT_RING_OVERFLOW);
   if (tid == 0) {
-    const uint32_t cnt = min(s.ntracks, ev.cap);
-    if (s.ntracks > VELO_MAX_TRACKS) s.status |= VELO_EVENT_MAX_TRACKS;
-    const unsigned long long first = atomicAdd(p.out_cursor, (unsigned long long)cnt);
-    s.out_first = first;
-    p.out_counts[e] = cnt;
-    p.out_first[e] = first;
-    p.out_status[e] = s.status | fallback;
+    if (count > VELO_MAX_TRACKS) atomicOr(&s.status, VELO_EVENT_MAX_TRACKS);
+    s.out_first = atomicAdd(p.out_cursor, (unsigned long long)count);
   }
   __syncthreads();
+  if (tid == 0) {
+    p.out_counts[e] = count;
+    p.out_first[e] = s.out_first;
+    p.out_status[e] = s.status | fallback;
+  }
   {
     // rows past out_capacity stay unwritten (the host reports the shortfall)
-    const unsigned long long room = s.out_first < p.out_capacity ? p.out_capacity - s.out_first : 0ull;
-    const uint32_t words = (uint32_t)min((unsigned long long)min(s.ntracks, ev.cap), room) * 25u;
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(ev.tracks);
-    uint32_t* dst = reinterpret_cast<uint32_t*>(p.out_tracks + s.out_first);
-    for (uint32_t w = tid; w < words; w += nt) {   // words past a track's last hit are zero
-      const uint32_t t = w / 25u;
-      dst[w] = w - 25u * t <= src[25u * t] ? src[w] : 0u;
+    const unsigned long long first = s.out_first + before;
+    const unsigned long long room = first < p.out_capacity ? p.out_capacity - first : 0ull;
+    const uint32_t words = (uint32_t)min((unsigned long long)w.tracks, room) * 25u;
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(ev.tracks() + w.row);
+    uint32_t* dst = reinterpret_cast<uint32_t*>(p.out_tracks + first);
+    for (uint32_t i = lane; i < words; i += 32) {   // words past a track's last hit are zero
+      const uint32_t t = i / 25u;
+      dst[i] = i - 25u * t <= src[25u * t] ? src[i] : 0u;
     }
   }
   if (p.results) {   // streaming: the tracks first, then the record
     __threadfence_system();
     __syncthreads();
-    if (tid == 0) publish_result(p, e, s.out_first, min(s.ntracks, ev.cap), s.status | fallback);
+    if (tid == 0) publish_result(p, e, s.out_first, count, s.status | fallback);
   }
   VELO_PHASE(6);
   VELO_PHASE_END();
@@ -1587,7 +1564,7 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
 // one seeding width kLanes (lanes per h0), so that a kernel holds one copy of
 // the seeding loop.
 template <int kMaxThreads, int kMinCtas, int kMode, int kMods, int kLanes>
-__global__ void __launch_bounds__(kMaxThreads, kMinCtas) search_kernel(const SearchParams p) {
+__global__ void __launch_bounds__(kMaxThreads, kMinCtas) search_kernel(const __grid_constant__ SearchParams p) {
   extern __shared__ __align__(16) uint8_t dyn_smem_raw[];
   __shared__ SharedT<kMods, kMaxThreads / 32> s;
   // learned seeding: the MLP weights lead the dynamic shared memory

@@ -35,7 +35,7 @@
 namespace velo {
 namespace {
 
-constexpr uint64_t kRowBytes = 16u + 64u + 4u + sizeof(velo_track);   // tracklet + rings + weak + track per hit row
+constexpr uint64_t kRowBytes = 16u + 32u + 4u + sizeof(velo_track);   // tracklet + entry + weak + track per hit row
 constexpr uint64_t kEventBytes = 4u + 4u + 4u + 8u + 8u;         // hits, maxmod, valid, hit_base, arena_off
 constexpr uint64_t kCounterBytes = 256;
 constexpr uint64_t kOffEvents = kCounterBytes;
@@ -53,7 +53,7 @@ struct StaticView {
   uint64_t* hit_base;
   uint64_t* arena_off;
   uint32_t* tracklets;          // 4 words per row
-  uint32_t* rings;              // 16 words per row
+  uint32_t* entries;            // 4 words, then 4 floats, per row
   uint32_t* weak;               // 1 per row
   velo_track* tracks;           // 1 per row
 };
@@ -72,7 +72,7 @@ __host__ __device__ StaticView view_of(uint8_t* base) {
   v.tracks = reinterpret_cast<velo_track*>(rows);
   v.tracklets = reinterpret_cast<uint32_t*>(rows + sizeof(velo_track) * VELO_STATIC_MAX_HIT_ROWS);
   v.weak = reinterpret_cast<uint32_t*>(rows + (sizeof(velo_track) + 16u) * VELO_STATIC_MAX_HIT_ROWS);
-  v.rings = reinterpret_cast<uint32_t*>(rows + (sizeof(velo_track) + 20u) * VELO_STATIC_MAX_HIT_ROWS);
+  v.entries = reinterpret_cast<uint32_t*>(rows + (sizeof(velo_track) + 20u) * VELO_STATIC_MAX_HIT_ROWS);
   return v;
 }
 
@@ -213,7 +213,8 @@ extern "C" velo_status velo_search_device_static(const uint8_t* d_input, const u
   p.smem_arena_bytes = smem;
   p.global_arena = nullptr;
   p.tracklets = v.tracklets;
-  p.rings = v.rings;
+  p.entry_words = v.entries;
+  p.entry_lines = v.entries + 4ull * VELO_STATIC_MAX_HIT_ROWS;
   p.weak = v.weak;
   p.tracks = v.tracks;
   p.out_tracks = d_tracks_out;

@@ -111,7 +111,7 @@ typedef struct velo_options {
                                  Results are identical; the context holds no staged batch
                                  afterwards.  0 = off */
   int32_t device_budget_mb;   /* velo_search / velo_search_packed: device memory one call may
-                                 use; a batch that needs more (about 305 B per hit) is cut into
+                                 use; a batch that needs more (about 275 B per hit) is cut into
                                  pipelined parts that fit.  0 = half the free device memory */
   int32_t seed_lanes;         /* seeding: lanes given to one h0's h1 candidates, 8, 16 or 32 (a
                                  warp then seeds 32 / seed_lanes h0s at once); below 32 it must
@@ -348,7 +348,7 @@ int32_t velo_device_sm_count(const velo_ctx* ctx);
  * NULL = the legacy default stream) and the results are valid once it is
  * synchronised.  Y-lanes as in velo_options; narrowing is on.
  *
- * All other memory is one file-scope device array of about 24 MB per GPU,
+ * All other memory is one file-scope device array of about 20 MB per GPU,
  * held from library load to process exit.  Limits per call, rejected with
  * VELO_ERR_CAPACITY: n_events <= VELO_STATIC_MAX_EVENTS;
  * total_hits + n_events <= VELO_STATIC_MAX_HIT_ROWS (total_hits = the sum of
