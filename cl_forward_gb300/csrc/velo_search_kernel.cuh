@@ -74,7 +74,7 @@ constexpr int kQueue = 32;            // pairs a warp holds for the exact fits
 template <int kWarps, int kOwn>
 struct SeedShared {
   float4 h0[kWarps][kOwn];            // x, y, z, first h1 - first pair (int bits)
-  float2 reach[kWarps][kOwn];         // the h0's y cut, and (z2 - z0) / (z1 - z0) where the map is valid
+  float2 reach[kWarps][kOwn];         // the h0's y cut, and in plain geometry (z2 - z0) / (z1 - z0)
   unsigned long long best[kWarps][kOwn];   // the h0's best (fit, Y-lane, h1, h2) so far
   uint32_t map[2][kMapRows];
   std::conditional_t<(kOwn > 4), uint32_t, uint16_t> queue[kWarps][kQueue];   // h0 << 14 | h1 in its module
@@ -116,6 +116,7 @@ struct EventView {
   uint8_t* arena;
   uint32_t P;
   bool tame;                // every module x-sorted and every coordinate within kMaxCoordinate
+  bool plain;               // plain geometry: tame, one z per module, ascending
   const MlpFrag* mlp;       // learned seeding: weights in shared memory
   __device__ __forceinline__ float* xs() const { return reinterpret_cast<float*>(arena); }
   __device__ __forceinline__ float* ys() const { return reinterpret_cast<float*>(arena + P); }
@@ -123,11 +124,12 @@ struct EventView {
   __device__ __forceinline__ uint2* wins() const { return reinterpret_cast<uint2*>(arena + 3u * P); }
   __device__ __forceinline__ uint8_t* useds() const { return arena + 5u * P; }
   // scratch by row: tracklets {h0, h1, h2, 0}, tracks, weak list, entries
-  __device__ __forceinline__ uint4* tracklets() const { return reinterpret_cast<uint4*>(p->tracklets); }
-  __device__ __forceinline__ velo_track* tracks() const { return p->tracks; }
-  __device__ __forceinline__ uint32_t* weak() const { return p->weak; }
-  __device__ __forceinline__ uint4* entry_words() const { return reinterpret_cast<uint4*>(p->entry_words); }
-  __device__ __forceinline__ float4* entry_lines() const { return reinterpret_cast<float4*>(p->entry_lines); }
+  uint4* tracklets;
+  velo_track* tracks;
+  uint32_t* weak;
+  uint4* entry_words;
+  float4* entry_lines;
+  int y_lanes, narrow;
 };
 
 // First index i in [lo, hi) with x[i] > c, for non-decreasing x.
@@ -191,7 +193,7 @@ __device__ void compute_windows(const EventView& ev, const Shared& s, int h, int
   const float x0 = ev.xs()[h], z0 = ev.zs()[h];
   const float* x2 = ev.xs() + st2;
   const float* z2 = ev.zs() + st2;
-  const bool sorted = ev.p->narrow && (s.flags[s2] & kSorted);
+  const bool sorted = ev.narrow && (s.flags[s2] & kSorted);
   uint32_t r1f = kNone16, r1l = kNone16, r2f = kNone16, r2l = kNone16;
 
   // h1 window: first hit with |x1-x0| < 0.7|z1-z0|, then the first later hit
@@ -313,7 +315,7 @@ struct Worker {
 // and y of the previous hit, x and y slopes}.  Bit 31 of the word marks a
 // tracklet (3 hits, number = its row among the warp's tracklets), as in the
 // reference (Kernel.cl:222-225,566); otherwise bits 23-27 are the track's hit
-// count and bits 0-22 its row among the warp's tracks.  The iteration says
+// count and bits 0-22 its row among the warp's tracks.   The iteration says
 // how many modules were skipped (the reference counts them in bits 28-30), so
 // an entry that finds nothing stays as it is, where it is.  The line is
 // computed when the hit is found: forwarding reads no hit, track or tracklet
@@ -331,6 +333,24 @@ __device__ __forceinline__ float4 line_through(float xa, float ya, float xb, flo
   return make_float4(xa, ya, fmul(fsub(xb, xa), td), fmul(fsub(yb, ya), td));
 }
 
+// The scatter cut (dx^2 + dy^2) / dz^2 < kMaxScatter bounds |dx| and |dy| by
+// sqrt(kMaxScatter) |dz| = 0.004 |dz|; 1 % more covers the rounding of the
+// reference's products.  At the usual 25 mm between modules that is 0.1 mm,
+// a sixth of kTolerance, so far fewer hits are tried.
+constexpr float kScatterReach = 0.00404f;
+// With |dz| at least this, 1 / dz squared stays far from overflow, so a fit
+// outside the cuts is finite and need not be evaluated.
+constexpr float kMinDz = 1e-3f;
+// Plain-geometry events (EventView::plain): every module x-sorted and of one
+// z, the modules' z ascending by more than kMinGap, every coordinate within
+// kMaxCoordinate of the origin (mm).  A line through hits of two modules then
+// predicts one point on a module, below 4e9, its fits with the module's hits
+// are finite, and where the point is near a hit its sum with a reach is
+// rounded by less than kRounding.
+constexpr float kMaxCoordinate = 1e4f;
+constexpr float kMinGap = 0.1f;
+constexpr float kRounding = 0.01f;
+
 // Appends the tracklets {h0, h1, h2} of the lanes with `win`, seeded in
 // iteration f, to the warp's rows and entries (Kernel.cl:550-567).
 __device__ __forceinline__ void append_tracklets(const EventView& ev, Worker& w, bool win, uint32_t h0, uint32_t h1,
@@ -340,12 +360,13 @@ __device__ __forceinline__ void append_tracklets(const EventView& ev, Worker& w,
   if (win) {
     const uint32_t r = (uint32_t)__popc(m & lanemask_lt());
     const uint32_t tp = w.tracklets + r, i = w.row + w.n + r;
-    ev.tracklets()[w.row + tp] = make_uint4(h0, h1, h2, 0u);
+    ev.tracklets[w.row + tp] = make_uint4(h0, h1, h2, 0u);
     const float z1 = ev.zs()[h1], z2 = ev.zs()[h2];
-    ev.entry_words()[i] = make_uint4(kTrackletFlag | tp, h2 | ((uint32_t)f << kEntryIterationShift),
-                                    __float_as_uint(z1), __float_as_uint(z2));
-    ev.entry_lines()[i] =
+    const float4 line =
         line_through(ev.xs()[h1], ev.ys()[h1], ev.xs()[h2], ev.ys()[h2], fdiv(1.0f, fsub(z2, z1)));
+    ev.entry_words[i] = make_uint4(kTrackletFlag | tp, h2 | ((uint32_t)f << kEntryIterationShift),
+                                     __float_as_uint(z1), __float_as_uint(z2));
+    ev.entry_lines[i] = line;
   }
   w.tracklets += __popc(m);
   w.n += __popc(m);
@@ -379,17 +400,6 @@ __device__ __forceinline__ uint32_t first_row(const Shared& s, const Worker& w, 
   return (uint32_t)__reduce_add_sync(kFull, rows);
 }
 
-// The scatter cut (dx^2 + dy^2) / dz^2 < kMaxScatter bounds |dx| and |dy| by
-// sqrt(kMaxScatter) |dz| = 0.004 |dz|; 1 % more covers the rounding of the
-// reference's products.  At the usual 25 mm between modules that is 0.1 mm,
-// a sixth of kTolerance, so far fewer hits are tried.
-constexpr float kScatterReach = 0.00404f;
-// With |dz| at least this, 1 / dz squared stays far from overflow, so a fit
-// outside the cuts is finite and need not be evaluated.
-constexpr float kMinDz = 1e-3f;
-// Events within this of the origin (mm) take the pair seeding.
-constexpr float kMaxCoordinate = 1e4f;
-
 // Per-warp counts of entries are summed in 16 bits: each is cut off well
 // above VELO_TTF_MODULO, where the event is flagged in any case.
 constexpr uint32_t kInflightMax = 2 * VELO_TTF_MODULO;
@@ -409,22 +419,95 @@ __device__ __forceinline__ int active_h0s(const EventView& ev, const Worker& w, 
   return (total + w.of() - 1 - w.idx()) / w.of();
 }
 
-// Track forwarding of iteration f, onto module f-4 (Kernel.cl:210-367): the
-// warp's entries, 32 at a time, kept in place or moved down over dropped ones.
+// The best hit of module m4 for an entry (fitHitToTrack, Kernel.cl:15-35, first
+// minimum over the module's hits), any module and any line: its place in the
+// module or -1, its z, and the fit's 1 / (z2 - z1).
+struct Fit {
+  int k;
+  float z, den;
+  bool degenerate;
+};
+
 template <class Shared>
-__device__ __forceinline__ void forward(const EventView& ev, Shared& s, Worker& w, int f) {
-  if (w.n == 0) return;   // warp-uniform
-  const int lane = threadIdx.x & 31, m4 = f - 4;
-  // the ends of module m4 for the narrowing (same addresses in every lane)
+__device__ __forceinline__ Fit fit_any(const EventView& ev, const Shared& s, int m4, float4 line, float h0z,
+                                       float h1z) {
   const int st4 = s.start[m4], n4 = s.num(m4);
   const float zmin4 = s.zmin[m4], zmax4 = s.zmax[m4];
-  const bool single4 = zmin4 == zmax4;   // one z on the module
-  const bool narrow4 = ev.p->narrow && (s.flags[m4] & kSorted) && n4 > 0;
   const float* x4 = ev.xs() + st4;
   const float* y4 = ev.ys() + st4;
   const float* z4 = ev.zs() + st4;
+  int k = 0;
+  float ht = __int_as_float(0x7f800000);   // +inf: every hit from k on is tried
+  bool all_fits = true;                    // every fit is evaluated, for its finiteness
+  if (ev.narrow && (s.flags[m4] & kSorted) && n4 > 0) {
+    const float dza = fsub(zmin4, h0z), dzb = fsub(zmax4, h0z);
+    const float xa = fadd(line.x, fmul(line.z, dza)), xb = fadd(line.x, fmul(line.z, dzb));
+    const float d_lo = fsub(zmin4, h1z), d_hi = fsub(zmax4, h1z);
+    const float reach = fmul(kScatterReach, fmaxf(fabsf(d_lo), fabsf(d_hi)));
+    const float ymax = fadd(fabsf(line.y), fmul(fabsf(line.w), fmaxf(fabsf(dza), fabsf(dzb))));
+    // the fits outside the cuts are known to be finite
+    const bool tame = ev.tame && (d_lo > kMinDz || d_hi < -kMinDz) && ymax < 1e15f;
+    const float tol = tame ? fminf(kTolerance, reach) : kTolerance;
+    const float xl = fminf(xa, xb), xh = fmaxf(xa, xb);
+    const float margin = fadd(0.01f, fmul(1e-5f, fadd(fabsf(xl), fabsf(xh))));
+    const float lt = fsub(fsub(xl, tol), margin);
+    const float h = fadd(fadd(xh, tol), margin);
+    if (isfinite(xa) && isfinite(xb) && isfinite(lt) && isfinite(h)) {
+      ht = h;
+      all_fits = !tame;
+      k = x4[n4 - 1] <= lt || x4[0] > ht ? n4 : first_gt(x4, 0, n4, lt);
+    }
+  }
+  // The scatter's 1/(z2 - z1) depends only on z2 here: it is recomputed only
+  // when z2's bit pattern changes (same operands, same rounded value).
+  Fit fit{-1, 0.f, 0.f, false};
+  float best = FLT_MAX;
+  uint32_t zc = 0x7fc00001u;   // bit pattern of the z2 the cached factor belongs to (none yet)
+  float den = 0.f;
+  for (; k < n4; ++k) {
+    const float h2x = x4[k];
+    if (h2x > ht) break;
+    const float h2z = z4[k];
+    const float dz = fsub(h2z, h0z);
+    const float dx = fabsf(fsub(fadd(line.x, fmul(line.z, dz)), h2x));
+    const float dy = fabsf(fsub(fadd(line.y, fmul(line.w, dz)), y4[k]));
+    const bool near = dx < kTolerance && dy < kTolerance;
+    if (near || all_fits) {
+      if (__float_as_uint(h2z) != zc) {
+        zc = __float_as_uint(h2z);
+        den = fdiv(1.f, fsub(h2z, h1z));
+      }
+      const float scatter = fmul(fmul(fadd(fmul(dx, dx), fmul(dy, dy)), den), den);
+      if (near && scatter < kMaxScatter) {
+        if (scatter < best) {
+          best = scatter;
+          fit.k = k;
+          fit.z = h2z;
+          fit.den = den;
+        }
+      } else if (!isfinite(scatter)) {
+        fit.degenerate = true;   // the reference's `condition*scatter + !condition*MAX` is NaN here
+      }
+    }
+  }
+  return fit;
+}
+
+// Track forwarding of iteration f, onto module f-4 (Kernel.cl:210-367): the
+// warp's entries, 32 at a time, kept in place or moved down over dropped ones.
+// In plain geometry one factor 1 / (z2 - z1) serves all hits of the module,
+// and only the hits within reach of the predicted x are fitted.
+template <bool kPlainGeometry, class Shared>
+__device__ __forceinline__ void forward(const EventView& ev, Shared& s, Worker& w, int f) {
+  if (w.n == 0) return;   // warp-uniform
+  const int lane = threadIdx.x & 31, m4 = f - 4;
+  const int st4 = s.start[m4], n4 = s.num(m4);
+  const float z4 = s.zmin[m4];
+  const float* x4 = ev.xs() + st4;
+  const float* y4 = ev.ys() + st4;
+  // the ends of module m4 (same addresses in every lane)
   float x4_first = 0.f, x4_last = 0.f;
-  if (n4 > 0) {
+  if (kPlainGeometry && n4 > 0) {
     x4_first = x4[0];
     x4_last = x4[n4 - 1];
   }
@@ -437,63 +520,38 @@ __device__ __forceinline__ void forward(const EventView& ev, Shared& s, Worker& 
     float4 line = make_float4(0.f, 0.f, 0.f, 0.f);
     uint32_t found = 0;
     if (i < n) {
-      en = ev.entry_words()[w.row + i];
-      line = ev.entry_lines()[w.row + i];
+      en = ev.entry_words[w.row + i];
+      line = ev.entry_lines[w.row + i];
       const bool is_tracklet = (en.x & kTrackletFlag) != 0;
       const float h0z = __uint_as_float(en.z), h1z = __uint_as_float(en.w);
-      int k = 0;
-      float ht = __int_as_float(0x7f800000);   // +inf: every hit from k on is tried
-      bool all_fits = true;                    // every fit is evaluated, for its finiteness
-      if (narrow4) {
-        const float dza = fsub(zmin4, h0z), dzb = fsub(zmax4, h0z);
-        const float xa = fadd(line.x, fmul(line.z, dza));
-        const float xb = single4 ? xa : fadd(line.x, fmul(line.z, dzb));
-        const float d_lo = fsub(zmin4, h1z), d_hi = fsub(zmax4, h1z);
-        const float reach = fmul(kScatterReach, fmaxf(fabsf(d_lo), fabsf(d_hi)));
-        const float ymax = fadd(fabsf(line.y), fmul(fabsf(line.w), fmaxf(fabsf(dza), fabsf(dzb))));
-        // the fits outside the cuts are known to be finite
-        const bool tame = ev.tame && (d_lo > kMinDz || d_hi < -kMinDz) && ymax < 1e15f;
-        const float tol = tame ? fminf(kTolerance, reach) : kTolerance;
-        const float xl = fminf(xa, xb), xh = fmaxf(xa, xb);
-        const float margin = fadd(0.01f, fmul(1e-5f, fadd(fabsf(xl), fabsf(xh))));
-        const float lt = fsub(fsub(xl, tol), margin);
-        const float h = fadd(fadd(xh, tol), margin);
-        if (isfinite(xa) && isfinite(xb) && isfinite(lt) && isfinite(h)) {
-          ht = h;
-          all_fits = !tame;
-          k = x4_last <= lt || x4_first > ht ? n4 : first_gt(x4, 0, n4, lt);
-        }
-      }
-      // fitHitToTrack (Kernel.cl:15-35) over the candidates, first minimum wins.
-      // The scatter's 1/(z2 - z1) depends only on z2 here: it is recomputed only
-      // when z2's bit pattern changes (same operands, same rounded value).
-      float best = FLT_MAX, best_z = 0.f, best_den = 0.f;
       int best_k = -1;
-      bool degenerate = false;
-      uint32_t zc = 0x7fc00001u;   // bit pattern of the z2 the cached factor belongs to (none yet)
-      float den = 0.f;
-      for (; k < n4; ++k) {
-        const float h2x = x4[k];
-        if (h2x > ht) break;
-        const float h2z = single4 ? zmin4 : z4[k];
-        const float dz = fsub(h2z, h0z);
-        const float dx = fabsf(fsub(fadd(line.x, fmul(line.z, dz)), h2x));
-        const float dy = fabsf(fsub(fadd(line.y, fmul(line.w, dz)), y4[k]));
-        const bool near = dx < kTolerance && dy < kTolerance;
-        if (near || all_fits) {
-          if (__float_as_uint(h2z) != zc) {
-            zc = __float_as_uint(h2z);
-            den = fdiv(1.f, fsub(h2z, h1z));
-          }
-          const float scatter = fmul(fmul(fadd(fmul(dx, dx), fmul(dy, dy)), den), den);
-          if (near && scatter < kMaxScatter) {
-            if (scatter < best) { best = scatter; best_k = k; best_z = h2z; best_den = den; }
-          } else if (!isfinite(scatter)) {
-            degenerate = true;   // the reference's `condition*scatter + !condition*MAX` is NaN here
+      float best_z = z4, best_den;
+      if constexpr (kPlainGeometry) {
+        const float d = fsub(z4, h1z), dz = fsub(z4, h0z);
+        const float xp = fadd(line.x, fmul(line.z, dz)), yp = fadd(line.y, fmul(line.w, dz));
+        const float tol = fadd(fminf(kTolerance, fmul(kScatterReach, fabsf(d))), kRounding);
+        const float lt = fsub(xp, tol), ht = fadd(xp, tol);
+        int k = n4;
+        if (n4 > 0 && x4_last > lt && x4_first <= ht) k = first_gt(x4, 0, n4, lt);
+        best_den = fdiv(1.f, d);
+        float best = FLT_MAX;
+        for (; k < n4; ++k) {
+          const float h2x = x4[k];
+          if (h2x > ht) break;
+          const float dx = fabsf(fsub(xp, h2x)), dy = fabsf(fsub(yp, y4[k]));
+          const float scatter = fmul(fmul(fadd(fmul(dx, dx), fmul(dy, dy)), best_den), best_den);
+          if (dx < kTolerance && dy < kTolerance && scatter < kMaxScatter && scatter < best) {
+            best = scatter;
+            best_k = k;
           }
         }
+      } else {
+        const Fit fit = fit_any(ev, s, m4, line, h0z, h1z);
+        best_k = fit.k;
+        best_z = fit.z;
+        best_den = fit.den;
+        if (fit.degenerate) atomicOr(&s.status, VELO_EVENT_DEGENERATE);
       }
-      if (degenerate) atomicOr(&s.status, VELO_EVENT_DEGENERATE);
 
       if (best_k >= 0) {
         const uint32_t hits = is_tracklet ? 3u : (en.x >> kEntryCountShift) & 31u;
@@ -509,7 +567,7 @@ __device__ __forceinline__ void forward(const EventView& ev, Shared& s, Worker& 
           keep = changed = true;
           promote = is_tracklet;   // third -> fourth hit: a track is made below
           if (!is_tracklet) {
-            velo_track& t = ev.tracks()[w.row + (en.x & kEntryNumber)];
+            velo_track& t = ev.tracks[w.row + (en.x & kEntryNumber)];
             t.hits[hits] = found;
             t.hitsNum = hits + 1;
             en.x += 1u << kEntryCountShift;
@@ -528,27 +586,27 @@ __device__ __forceinline__ void forward(const EventView& ev, Shared& s, Worker& 
     // when the track is written out
     const unsigned pm = __ballot_sync(kFull, promote);
     if (promote) {
-      const uint4 tl = ev.tracklets()[w.row + (en.x & kEntryNumber)];
+      const uint4 tl = ev.tracklets[w.row + (en.x & kEntryNumber)];
       ev.useds()[tl.x] = kUsed;
       ev.useds()[tl.y] = kUsed;
       ev.useds()[tl.z] = kUsed;
       const uint32_t tn = w.tracks + (uint32_t)__popc(pm & lanemask_lt());
-      uint32_t* t = reinterpret_cast<uint32_t*>(&ev.tracks()[w.row + tn]);
+      uint32_t* t = reinterpret_cast<uint32_t*>(&ev.tracks[w.row + tn]);
       t[0] = 4; t[1] = tl.x; t[2] = tl.y; t[3] = tl.z; t[4] = found;
       en.x = tn | (4u << kEntryCountShift);
     }
     w.tracks += __popc(pm);
     // three-hit tracklets that ran out of skips (Kernel.cl:359-363)
     const unsigned wm = __ballot_sync(kFull, weak);
-    if (weak) ev.weak()[w.row + w.weak + (uint32_t)__popc(wm & lanemask_lt())] = en.x & kEntryNumber;
+    if (weak) ev.weak[w.row + w.weak + (uint32_t)__popc(wm & lanemask_lt())] = en.x & kEntryNumber;
     w.weak += __popc(wm);
     // entries to follow in the next iteration (Kernel.cl:344-355): every lane
     // has read its own, and slots below i0 are done with
     const unsigned km = __ballot_sync(kFull, keep);
     const uint32_t to = kept + (uint32_t)__popc(km & lanemask_lt());
     if (keep && (changed || to != i)) {
-      ev.entry_words()[w.row + to] = en;
-      ev.entry_lines()[w.row + to] = line;
+      ev.entry_words[w.row + to] = en;
+      ev.entry_lines[w.row + to] = line;
     }
     kept += __popc(km);
     __syncwarp();
@@ -640,7 +698,9 @@ static __device__ __noinline__ float2 score_doublets(const MlpFrag* mlp, bool sc
 }
 
 // Seeding of module f: h0 on f, h1 on f-2, h2 on f-4 (Kernel.cl:392-568
-// with the unused-h0 gather of :720-764), G lanes per h0 (SeedLanes).
+// with the unused-h0 gather of :720-764), G lanes per h0 (SeedLanes): the
+// form that walks the candidate windows, for unsorted events, for learned
+// seeding of several z per module, and for the training-data dump.
 // G = 32: one warp per unused h0.  G = 8 or 16: a warp seeds 32 / G h0s at
 // once and walks the chunks of its groups' h1 windows together, so every
 // ballot and the groups' minimum reductions run with all lanes present; the
@@ -656,10 +716,10 @@ __device__ void seed_module(const EventView& ev, Shared& s, Worker& w, int f, co
   const int st0 = s.start[f], n0 = s.num(f);
   const int s1 = f - 2, m4 = f - 4;
   const int st1 = s.start[s1], st4 = s.start[m4], n4 = s.num(m4);
-  const uint32_t Y = (uint32_t)ev.p->y_lanes;
+  const uint32_t Y = (uint32_t)ev.y_lanes;
   const uint32_t chunk_step = G == 32 ? 32u % Y : 0u;   // how far the Y-lanes turn per chunk
   const float s1_z = s.num(s1) > 0 ? ev.zs()[st1] : 0.f;   // Kernel.cl:420
-  const bool narrow4 = ev.p->narrow && (s.flags[m4] & kSorted) && n4 > 0;
+  const bool narrow4 = ev.narrow && (s.flags[m4] & kSorted) && n4 > 0;
   const float zmin4 = s.zmin[m4], zmax4 = s.zmax[m4];
   const float* x4 = ev.xs() + st4;
   const float* y4 = ev.ys() + st4;
@@ -843,14 +903,6 @@ __device__ void seed_module(const EventView& ev, Shared& s, Worker& w, int f, co
   if (degenerate) atomicOr(&s.status, VELO_EVENT_DEGENERATE);
 }
 
-// seed_module for the events that the pair seeding does not take, out of
-// line, so that the module loop keeps its registers.
-template <int kMode, int G, class Shared>
-__device__ __noinline__ Worker seed_windows(const EventView ev, Shared& s, Worker w, int f) {
-  seed_module<kMode, G>(ev, s, w, f, seed_lanes_of(G, (uint32_t)ev.p->y_lanes));
-  return w;
-}
-
 // The candidate windows of every hit (all threads of the CTA).
 template <class Shared>
 __device__ __noinline__ void fill_windows(const EventView ev, const Shared& s) {
@@ -891,14 +943,6 @@ __device__ __noinline__ void fill_windows(const EventView ev, const Shared& s) {
 constexpr float kCellInv = 1.f / 1.3125f;   // cells of 1.3 mm: 32 columns span half a module's width, 64 rows its height
 
 __device__ __forceinline__ int map_cell(float v) { return __float2int_rd(fmul(v, kCellInv)); }
-
-// The map of module m4 answers for pairs whose h1 is on module s1: all hits
-// of either module at one z, so that the predicted point is the fit's own,
-// and the two z far enough apart for every fit to be finite.
-template <class Shared>
-__device__ __forceinline__ bool map_valid(const Shared& s, int s1, int m4) {
-  return s.zmin[m4] == s.zmax[m4] && s.zmin[s1] == s.zmax[s1] && fabsf(fsub(s.zmin[m4], s.zmin[s1])) > kMinDz;
-}
 
 // Marks the cells from which hit i of module m4 could be met: a pair whose
 // fit passes lies within 0.004 |z2 - z1| of it, and within kTolerance.  A
@@ -976,28 +1020,94 @@ __device__ __forceinline__ void h1_window(const EventView& ev, const Shared& s, 
   }
 }
 
+// h2 (hit k of module m4, at x) lies in the window of an h1 with bounds lo and
+// hi: from the first hit above lo (that one even if it is above hi) up to the
+// first later one above hi.
+__device__ __forceinline__ bool in_h2_window(const float* x4, int k, float x, float lo, float hi) {
+  return x > lo && (!(x > hi) || k == 0 || !(x4[k - 1] > lo));
+}
+
+// The best h2 of one (h0, h1) on module m4 (Kernel.cl:468-529) where the
+// modules hold several z values or the fits may not be finite; h0 = {x, y, z}.
 template <class Shared>
+__device__ __forceinline__ Fit pair_fit_any(const EventView& ev, const Shared& s, int f, float h0x, float h0y, float h0z,
+                                         int hit1, float* scatter_out) {
+  const int m4 = f - 4, st4 = s.start[m4], n4 = s.num(m4);
+  const float zmin4 = s.zmin[m4], zmax4 = s.zmax[m4];
+  const float* x4 = ev.xs() + st4;
+  const float* y4 = ev.ys() + st4;
+  const float* z4 = ev.zs() + st4;
+  const float h1x = ev.xs()[hit1], h1y = ev.ys()[hit1], h1z = ev.zs()[hit1];
+  float lo, hi;
+  h2_bounds(h1x, h1z, s.sz[f], s.sz[m4], &lo, &hi);
+  const float dz_inverted = fdiv(1.f, fsub(h1z, h0z));
+  const float ddx = fsub(h1x, h0x), ddy = fsub(h1y, h0y);
+  const float xa = fadd(h0x, fmul(ddx, fmul(fsub(zmin4, h0z), dz_inverted)));
+  const float xb = fadd(h0x, fmul(ddx, fmul(fsub(zmax4, h0z), dz_inverted)));
+  const float d_lo = fsub(zmin4, h1z), d_hi = fsub(zmax4, h1z);
+  const float reach = fmul(kScatterReach, fmaxf(fabsf(d_lo), fabsf(d_hi)));
+  const float tol = d_lo > kMinDz || d_hi < -kMinDz ? fminf(kTolerance, reach) : kTolerance;
+  const float xl = fminf(xa, xb), xh = fmaxf(xa, xb);
+  const float margin = fadd(0.01f, fmul(1e-5f, fadd(fabsf(xl), fabsf(xh))));
+  const float lt = fsub(fsub(xl, tol), margin);
+  float ht = fadd(fadd(xh, tol), margin);
+  int k = 0;
+  if (isfinite(xa) && isfinite(xb) && isfinite(lt) && isfinite(ht))
+    k = first_gt(x4, 0, n4, lt);
+  else
+    ht = __int_as_float(0x7f800000);   // +inf: every hit is tried
+  Fit fit{-1, 0.f, 0.f, false};
+  float best = FLT_MAX;
+  uint32_t zc = 0x7fc00001u;
+  float z2_tz = 0.f, den = 0.f;
+  for (; k < n4; ++k) {
+    const float h2x = x4[k];
+    if (h2x > ht) break;
+    const float h2z = z4[k];
+    if (__float_as_uint(h2z) != zc) {   // both factors depend on h2z only (per h0, h1)
+      zc = __float_as_uint(h2z);
+      z2_tz = fmul(fsub(h2z, h0z), dz_inverted);
+      den = fdiv(1.f, fsub(h2z, h1z));
+    }
+    const float dx = fsub(fadd(h0x, fmul(ddx, z2_tz)), h2x);
+    const float dy = fsub(fadd(h0y, fmul(ddy, z2_tz)), y4[k]);
+    if (fabsf(dx) < kTolerance && fabsf(dy) < kTolerance && in_h2_window(x4, k, h2x, lo, hi)) {
+      const float scatter = fmul(fmul(fadd(fmul(dx, dx), fmul(dy, dy)), den), den);
+      if (scatter < kMaxScatter) {
+        if (scatter < best) {
+          best = scatter;
+          fit.k = k;
+        }
+      } else if (!isfinite(scatter)) {
+        fit.degenerate = true;
+      }
+    }
+  }
+  *scatter_out = best;
+  return fit;
+}
+
+template <int kMode, bool kPlainGeometry, class Shared>
 __device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Worker& w, int f) {
   constexpr int kOwn = Shared::kOwn;
   auto& sd = s.seed;
   const int lane = threadIdx.x & 31;
   const int s1 = f - 2, m4 = f - 4;
   const int st0 = s.start[f], n0 = s.num(f), st1 = s.start[s1], st4 = s.start[m4], n4 = s.num(m4);
-  const float zmin1 = s.zmin[s1], zmin4 = s.zmin[m4], zmax4 = s.zmax[m4];
-  const bool single1 = zmin1 == s.zmax[s1], single4 = zmin4 == zmax4;
-  const bool use_map = map_valid(s, s1, m4);
+  const float zmin1 = s.zmin[s1], zmin4 = s.zmin[m4];
   const uint32_t* map = sd.map[w.parity()];
   float4* own_h0 = sd.h0[w.warp()];
   float2* own_reach = sd.reach[w.warp()];
   unsigned long long* own_best = sd.best[w.warp()];
   uint16_t* own_first = sd.first[w.warp()];
+  // plain geometry: one factor 1 / (z2 - z1), and the reach in x
+  const float d41 = fsub(zmin4, zmin1);
+  const float den = fdiv(1.f, d41), tol = fadd(fminf(kTolerance, fmul(kScatterReach, fabsf(d41))), kRounding);
   const float* x4 = ev.xs() + st4;
   const float* y4 = ev.ys() + st4;
-  const float* z4 = ev.zs() + st4;
-  const uint32_t Y = (uint32_t)ev.p->y_lanes;
+  const uint32_t Y = (uint32_t)ev.y_lanes;
   if (n0 == 0 || n4 == 0 || s.num(s1) == 0) return;
   const float s1_z = ev.zs()[st1];   // Kernel.cl:420
-  bool degenerate = false;
 
   for (int block = 0; block < n0; block += 32)   // warp-uniform
   for (int c0 = 0, mine = active_h0s(ev, w, st0, n0, block, sd.active[w.warp()]); c0 < mine; c0 += kOwn) {
@@ -1052,7 +1162,7 @@ __device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Worke
           const uint8_t u1 = ev.useds()[h1];
           const float h1x = ev.xs()[h1], h1y = ev.ys()[h1];
           pass = u1 == 0 && fabsf(fsub(h1y, q.y)) < r.x;
-          if (pass && use_map) {   // the fit's own predicted point
+          if (kPlainGeometry && kMode == kPlain && pass) {   // the fit's own predicted point
             const float px = fadd(q.x, fmul(fsub(h1x, q.x), r.y));
             const float py = fadd(q.y, fmul(fsub(h1y, q.y), r.y));
             pass = (map[map_cell(py) & (kMapRows - 1)] >> (map_cell(px) & 31)) & 1u;
@@ -1070,59 +1180,82 @@ __device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Worke
         bool reached = lane < queued;
         if (!(s.flags[s1] & kDeadTail) && reached)
           for (int e = local1 - (int)Y; e >= (int)own_first[own]; e -= (int)Y) reached &= !h1_dead(ev, s, s1, st1 + e);
+        // learned: the batch is scored together, and a kept doublet's h2 lies
+        // within its own tolerance, in the h1's exact window
+        float learned_tol = kTolerance;
+        int a = 0, b = n4;
+        if constexpr (kMode == kLearned) {
+          float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+          float h1x = 0.f, h1y = 0.f;
+          if (reached) {
+            q = own_h0[own];
+            h1x = ev.xs()[hit1];
+            h1y = ev.ys()[hit1];
+            const uint32_t w1 = ev.wins()[hit1].y;
+            a = (int)(w1 & 0xffffu);
+            b = (int)(w1 >> 16);
+          }
+          // only doublets with a wide exact h2 window are worth scoring
+          const bool score = reached && b - a >= ev.p->learned_min_window;
+          bool keep = true;
+          if (__any_sync(kFull, score)) {
+            const float2 r = score_doublets(ev.mlp, score, q.x, q.y, q.z, h1x, h1y, zmin1,
+                                            fdiv(1.f, fsub(zmin1, q.z)), 0.5f * (zmin4 + zmin4), b - a, f, ev.S,
+                                            reached ? own_reach[own].x : 0.f);
+            if (score) {
+              keep = r.x >= ev.p->keep_threshold;
+              learned_tol = fminf(kTolerance, fmaxf(r.y, 0.f) + ev.p->window_margin);
+            }
+          }
+          // keep-rate bookkeeping for the guard: the scored doublets
+          const unsigned mc = __ballot_sync(kFull, score), mk = __ballot_sync(kFull, score && keep);
+          if (lane == 0 && mc) {
+            atomicAdd(&s.considered, (uint32_t)__popc(mc));
+            atomicAdd(&s.kept, (uint32_t)__popc(mk));
+          }
+          reached = reached && keep;
+        }
         if (reached) {
-          // Kernel.cl:468-529 for one (h0, h1): the fits of the h2s in reach
           const float4 q = own_h0[own];
-          const float h1x = ev.xs()[hit1], h1y = ev.ys()[hit1], h1z = single1 ? zmin1 : ev.zs()[hit1];
-          const float dz_inverted = fdiv(1.f, fsub(h1z, q.z));
-          const float ddx = fsub(h1x, q.x), ddy = fsub(h1y, q.y);
-          const float xa = fadd(q.x, fmul(ddx, fmul(fsub(zmin4, q.z), dz_inverted)));
-          const float xb = single4 ? xa : fadd(q.x, fmul(ddx, fmul(fsub(zmax4, q.z), dz_inverted)));
-          const float d_lo = fsub(zmin4, h1z), d_hi = fsub(zmax4, h1z);
-          const float reach = fmul(kScatterReach, fmaxf(fabsf(d_lo), fabsf(d_hi)));
-          const float tol = d_lo > kMinDz || d_hi < -kMinDz ? fminf(kTolerance, reach) : kTolerance;
-          const float xl = fminf(xa, xb), xh = fmaxf(xa, xb);
-          const float margin = fadd(0.01f, fmul(1e-5f, fadd(fabsf(xl), fabsf(xh))));
-          const float lt = fsub(fsub(xl, tol), margin);
-          float ht = fadd(fadd(xh, tol), margin);
-          int k = 0;
-          if (isfinite(xa) && isfinite(xb) && isfinite(lt) && isfinite(ht))
-            k = first_gt(x4, 0, n4, lt);
-          else
-            ht = __int_as_float(0x7f800000);   // +inf: every hit is tried
           float best = FLT_MAX;
           int best_k = -1;
-          uint32_t zc = 0x7fc00001u;
-          float z2_tz = 0.f, den = 0.f;
-          for (; k < n4; ++k) {
-            const float h2x = x4[k];
-            if (h2x > ht) break;
-            const float h2z = single4 ? zmin4 : z4[k];
-            if (__float_as_uint(h2z) != zc) {   // both factors depend on h2z only (per h0, h1)
-              zc = __float_as_uint(h2z);
-              z2_tz = fmul(fsub(h2z, q.z), dz_inverted);
-              den = fdiv(1.f, fsub(h2z, h1z));
+          if constexpr (kPlainGeometry) {
+            // Kernel.cl:468-529 for one (h0, h1): the fits of the h2s in reach
+            const float z2_tz = own_reach[own].y;
+            const float h1x = ev.xs()[hit1], h1y = ev.ys()[hit1];
+            const float px = fadd(q.x, fmul(fsub(h1x, q.x), z2_tz)), py = fadd(q.y, fmul(fsub(h1y, q.y), z2_tz));
+            float lt = fsub(px, tol), ht = fadd(px, tol);
+            if constexpr (kMode == kLearned) {
+              const float margin = fadd(0.01f, fmul(1e-5f, fadd(fabsf(px), fabsf(px))));
+              const float l = fsub(fsub(px, learned_tol), margin), h = fadd(fadd(px, learned_tol), margin);
+              if (isfinite(l) && isfinite(h)) {   // else the whole window is tried
+                lt = fmaxf(lt, l);
+                ht = fminf(ht, h);
+              }
+              if (!((map[map_cell(py) & (kMapRows - 1)] >> (map_cell(px) & 31)) & 1u)) b = a;   // no hit in reach
             }
-            const float dx = fsub(fadd(q.x, fmul(ddx, z2_tz)), h2x);
-            const float dy = fsub(fadd(q.y, fmul(ddy, z2_tz)), y4[k]);
-            if (fabsf(dx) < kTolerance && fabsf(dy) < kTolerance) {
+            for (int k = first_gt(x4, a, b, lt); k < b; ++k) {
+              const float h2x = x4[k];
+              if (h2x > ht) break;
+              const float dx = fsub(px, h2x), dy = fsub(py, y4[k]);
               const float scatter = fmul(fmul(fadd(fmul(dx, dx), fmul(dy, dy)), den), den);
-              if (scatter < kMaxScatter ? scatter < best : !isfinite(scatter)) {
-                // the h2 must lie in the h1's window: from the first hit above
-                // the lower bound (that one even if it is above the upper
-                // bound) up to the first later one above the upper bound
-                float lo, hi;
-                h2_bounds(h1x, h1z, s.sz[f], s.sz[m4], &lo, &hi);
-                if (h2x > lo && (!(h2x > hi) || k == 0 || !(x4[k - 1] > lo))) {
-                  if (scatter < kMaxScatter) {
-                    best = scatter;
-                    best_k = k;
-                  } else {
-                    degenerate = true;
-                  }
+              if (fabsf(dx) < kTolerance && fabsf(dy) < kTolerance && scatter < kMaxScatter && scatter < best) {
+                bool in = kMode == kLearned;   // [a, b) is the window
+                if constexpr (kMode == kPlain) {
+                  float lo, hi;
+                  h2_bounds(h1x, zmin1, s.sz[f], s.sz[m4], &lo, &hi);
+                  in = in_h2_window(x4, k, h2x, lo, hi);
+                }
+                if (in) {
+                  best = scatter;
+                  best_k = k;
                 }
               }
             }
+          } else {
+            const Fit fit = pair_fit_any(ev, s, f, q.x, q.y, q.z, hit1, &best);
+            best_k = fit.k;
+            if (fit.degenerate) atomicOr(&s.status, VELO_EVENT_DEGENERATE);
           }
           if (best_k >= 0) {   // smallest fit, then Y-lane, h1, h2
             const uint32_t e = (uint32_t)local1 - own_first[own];
@@ -1142,7 +1275,6 @@ __device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Worke
     append_tracklets(ev, w, best != ~0ull, (uint32_t)h0, (uint32_t)(st1 + first) + ((uint32_t)(best >> 14) & 0x3fffu),
                      (uint32_t)st4 + (uint32_t)(best & 0x3fffu), f);
   }
-  if (degenerate) atomicOr(&s.status, VELO_EVENT_DEGENERATE);
 }
 
 // The flags of module m's hits before the search (one warp): unused, and
@@ -1167,30 +1299,10 @@ __device__ __forceinline__ bool clear_flags(const EventView& ev, const Shared& s
   return tail;
 }
 
-// Per-phase cycle counters, compiled in only with -DVELO_PHASE_CLOCKS
-// (diagnostic builds): thread 0 of every CTA adds the clock64() time between
-// the barriers that close each phase; slot 7 counts events.
-#ifdef VELO_PHASE_CLOCKS
-static __device__ unsigned long long g_phase_cycles[8];   // one per translation unit
-#define VELO_PHASE_BEGIN() long long ph_t = clock64(); unsigned long long ph[7] = {0, 0, 0, 0, 0, 0, 0}
-#define VELO_PHASE(k)                 \
-  do {                                \
-    const long long t_ = clock64();   \
-    ph[k] += (unsigned long long)(t_ - ph_t); \
-    ph_t = t_;                        \
-  } while (0)
-#define VELO_PHASE_END()                                              \
-  do {                                                                \
-    if (threadIdx.x == 0) {                                           \
-      for (int k_ = 0; k_ < 7; ++k_) atomicAdd(&g_phase_cycles[k_], ph[k_]); \
-      atomicAdd(&g_phase_cycles[7], 1ull);                            \
-    }                                                                 \
-  } while (0)
-#else
-#define VELO_PHASE_BEGIN() do {} while (0)
-#define VELO_PHASE(k) do {} while (0)
-#define VELO_PHASE_END() do {} while (0)
-#endif
+// Words a thread loads before it stores any, while an event is staged.
+constexpr int kStageWords = 6;
+// Words of tracks a lane loads before it stores any, while they are written out.
+constexpr int kCopyWords = 4;
 
 // Hits of a module that one warp sorts by rank in registers (4 per lane).
 constexpr int kArenaRankMax = 128;
@@ -1302,6 +1414,70 @@ __device__ __forceinline__ void publish_result(const SearchParams& p, int e, uns
   *reinterpret_cast<volatile uint32_t*>(&r->ready) = 1u;
 }
 
+// Per-phase cycle counters, compiled in only with -DVELO_PHASE_CLOCKS
+// (diagnostic builds): thread 0 of every CTA adds the clock64() time between
+// the barriers that close each phase; slot 7 counts events.
+#ifdef VELO_PHASE_CLOCKS
+static __device__ unsigned long long g_phase_cycles[8];   // one per translation unit
+#define VELO_PHASE_BEGIN() long long ph_t = clock64(); unsigned long long ph[7] = {0, 0, 0, 0, 0, 0, 0}
+#define VELO_PHASE(k)                 \
+  do {                                \
+    const long long t_ = clock64();   \
+    ph[k] += (unsigned long long)(t_ - ph_t); \
+    ph_t = t_;                        \
+  } while (0)
+#define VELO_PHASE_END()                                              \
+  do {                                                                \
+    if (threadIdx.x == 0) {                                           \
+      for (int k_ = 0; k_ < 7; ++k_) atomicAdd(&g_phase_cycles[k_], ph[k_]); \
+      atomicAdd(&g_phase_cycles[7], 1ull);                            \
+    }                                                                 \
+  } while (0)
+#else
+#define VELO_PHASE_BEGIN() do {} while (0)
+#define VELO_PHASE(k) do {} while (0)
+#define VELO_PHASE_END() do {} while (0)
+#endif
+
+// The module loop, Kernel.cl:671-767 (see Worker for the order of the warps).
+// kMode: the seeding; kPlainGeometry: the event is of plain geometry.
+template <int kMode, int kLanes, bool kPlainGeometry, class Shared>
+__device__ __forceinline__ Worker module_loop(const EventView& ev, Shared& s, Worker w) {
+  const int lane = threadIdx.x & 31, S = ev.S;
+  for (int f = S - 1; f >= 4; --f) {
+    forward<kPlainGeometry>(ev, s, w, f);
+    const int step = (S - 1 - f) & 1;
+    if (w.alone() || step == w.parity()) {
+      if (kMode != kDump && kPlainGeometry) {
+        uint32_t* map = s.seed.map[w.parity()];
+        const int gt = w.idx() * 32 + lane, gn = w.of() * 32;
+        for (int i = gt; i < kMapRows; i += gn) map[i] = 0;
+        group_sync<Shared::kMaxWarps>(w);
+        for (int i = gt; i < s.num(f - 4); i += gn) mark_map(ev, s, map, f - 2, f - 4, i);
+      }
+      group_sync<Shared::kMaxWarps>(w);
+      if constexpr (kPlainGeometry) {
+        seed_pairs<kMode, true>(ev, s, w, f);
+      } else {
+        if (kMode == kPlain && ev.tame)
+          seed_pairs<kPlain, false>(ev, s, w, f);
+        else
+          seed_module<kMode, kLanes>(ev, s, w, f, seed_lanes_of(kLanes, (uint32_t)ev.y_lanes));
+      }
+      group_sync<Shared::kMaxWarps>(w);
+    }
+    if (step == 1 || f == 4) __syncthreads();
+  }
+  return w;
+}
+
+// For the events that the kernel's own loop is not made for, out of line: it
+// then costs that loop no registers.
+template <int kMode, int kLanes, bool kPlainGeometry, class Shared>
+__device__ __noinline__ Worker module_loop_any(const EventView ev, Shared& s, Worker w) {
+  return module_loop<kMode, kLanes, kPlainGeometry>(ev, s, w);
+}
+
 // ---------------------------------------------------------------------------
 template <int kMode, int kLanes, class Shared>
 __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* dyn, const MlpFrag* mlp_smem) {
@@ -1335,11 +1511,18 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
   ev.P = L.y;
   ev.event = e;
   ev.mlp = mlp_smem;
+  ev.tracklets = reinterpret_cast<uint4*>(p.tracklets);
+  ev.tracks = p.tracks;
+  ev.weak = p.weak;
+  ev.entry_words = reinterpret_cast<uint4*>(p.entry_words);
+  ev.entry_lines = reinterpret_cast<float4*>(p.entry_lines);
+  ev.y_lanes = p.y_lanes;
+  ev.narrow = p.narrow;
 
   // stage the event; the module table must tile [0, H) in order (the host
   // checked only the header and the blob's length)
   bool bad = tid == 0 && S == 0 && H != 0;
-  bool wild = !ev.p->narrow;   // the event does not take the pair seeding
+  bool wild = !ev.narrow;   // the event does not take the pair seeding
   for (int m = tid; m < S; m += nt) {
     const int32_t st = gstart[m], nm = gnum[m];
     const int64_t expect = m == 0 ? 0 : (int64_t)gstart[m - 1] + (int64_t)gnum[m - 1];
@@ -1353,15 +1536,30 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
   // only after the sort)
   const uint32_t* gid = reinterpret_cast<const uint32_t*>(gnum + S);
   uint32_t* ids = reinterpret_cast<uint32_t*>(ev.wins());
-  for (int i = tid; i < H; i += nt) {
-    const float xv = gx[i], yv = gy[i], zv = gz[i];
-    bad |= !(isfinite(xv) && isfinite(yv) && isfinite(zv));
-    ev.xs()[i] = xv;
-    ev.ys()[i] = yv;
-    ev.zs()[i] = zv;
-    wild |= fmaxf(fabsf(xv), fmaxf(fabsf(yv), fabsf(zv))) > kMaxCoordinate;
-    if (p.sort_events) ids[i] = gid[i];
+  // x, y and z lie one after another: copied as one array, a warp to whole
+  // 128-byte lines of it and several lines in flight (events read in place
+  // come over the host link, where a request for part of a line costs a line)
+  const int values = 3 * H;
+  for (int i0 = tid - (int)((reinterpret_cast<uintptr_t>(gx) >> 2) & 31u); i0 < values; i0 += kStageWords * nt) {
+    float v[kStageWords];
+#pragma unroll
+    for (int k = 0; k < kStageWords; ++k) {
+      const int i = i0 + k * nt;
+      v[k] = i >= 0 && i < values ? gx[i] : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < kStageWords; ++k) {
+      const int i = i0 + k * nt;
+      bad |= !(fabsf(v[k]) <= FLT_MAX);
+      wild |= fabsf(v[k]) > kMaxCoordinate;
+      if (i >= 0 && i < values) {
+        const int a = (i >= H) + (i >= 2 * H);   // which array
+        *reinterpret_cast<float*>(ev.arena + (uint32_t)a * ev.P + 4u * (uint32_t)(i - a * H)) = v[k];
+      }
+    }
   }
+  if (p.sort_events)
+    for (int i = tid; i < H; i += nt) ids[i] = gid[i];
   if (tid == 0) {
     s.start[S] = H;
     s.status = 0;
@@ -1395,20 +1593,45 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
   VELO_PHASE(0);
 
   // per-module z range, x-sortedness and hit flags (one warp per module)
+  // The first hits of a warp's next module are loaded while it goes over one.
+  float x_next = 0.f, z_next = 0.f;
+  auto load_module = [&](int m) {
+    if (m < S && lane < s.num(m)) {
+      x_next = ev.xs()[s.start[m] + lane];
+      z_next = ev.zs()[s.start[m] + lane];
+    }
+  };
+  load_module(warp);
   for (int m = warp; m < S; m += nwarps) {
     const int st = s.start[m], n = s.num(m);
-    float zmn = FLT_MAX, zmx = -FLT_MAX;
+    float x = x_next, z = z_next;
+    load_module(m + nwarps);
+    float zmn = FLT_MAX, zmx = -FLT_MAX, x_before = -FLT_MAX;
     bool sorted = true;
-    for (int i = lane; i < n; i += 32) {
-      const float z = ev.zs()[st + i];
-      zmn = fminf(zmn, z);
-      zmx = fmaxf(zmx, z);
-      if (i + 1 < n && !(ev.xs()[st + i] <= ev.xs()[st + i + 1])) sorted = false;
+    for (int i0 = 0; i0 < n; i0 += 32) {   // warp-uniform
+      const int i = i0 + lane;
+      if (i0 > 0 && i < n) {
+        x = ev.xs()[st + i];
+        z = ev.zs()[st + i];
+      }
+      const float left = __shfl_up_sync(kFull, x, 1);
+      if (i < n) {
+        sorted &= (lane > 0 ? left : x_before) <= x;
+        zmn = fminf(zmn, z);
+        zmx = fmaxf(zmx, z);
+      }
+      x_before = __shfl_sync(kFull, x, 31);
     }
+    const float z0 = __shfl_sync(kFull, zmn, 0);   // lane 0 has a hit if any has
+    if (__all_sync(kFull, zmn > zmx || (zmn == z0 && zmx == z0))) {
+      zmn = z0;
+      zmx = n > 0 ? z0 : -FLT_MAX;
+    } else {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      zmn = fminf(zmn, __shfl_xor_sync(kFull, zmn, o));
-      zmx = fmaxf(zmx, __shfl_xor_sync(kFull, zmx, o));
+      for (int o = 16; o > 0; o >>= 1) {
+        zmn = fminf(zmn, __shfl_xor_sync(kFull, zmn, o));
+        zmx = fmaxf(zmx, __shfl_xor_sync(kFull, zmx, o));
+      }
     }
     sorted = __all_sync(kFull, sorted);
     wild |= !sorted;
@@ -1420,12 +1643,18 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
     }
   }
   ev.tame = !__syncthreads_or(wild);
+  // the modules' z ascend, empty modules apart
+  bool odd = false;
+  for (int m = tid; m < S; m += nt)
+    if (s.num(m) > 0) {
+      int q = m - 1;
+      while (q >= 0 && s.num(q) == 0) --q;
+      odd |= s.zmin[m] != s.zmax[m] || (q >= 0 && !(fsub(s.zmin[m], s.zmax[q]) > kMinGap));
+    }
+  ev.plain = !__syncthreads_or(odd) && ev.tame;
   VELO_PHASE(1);
 
   bool learned = kMode == kLearned && (p.learned_max_hits == 0 || (uint32_t)H <= p.learned_max_hits);
-  // per-lane constants of the learned seeding's ballots
-  SeedLanes sl{};
-  if constexpr (kMode == kLearned) sl = seed_lanes_of(kLanes, (uint32_t)ev.p->y_lanes);
   // candidate windows for the seedings that read them
   if (kMode != kPlain || !ev.tame) {
     fill_windows(ev, s);
@@ -1447,41 +1676,21 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
       w.n = w.tracklets = w.tracks = w.weak = 0;
       __syncthreads();
     }
-    const bool pairs = kMode == kPlain && ev.tame;
-    // module loop, Kernel.cl:671-767 (see Worker for the order of the warps)
-    for (int f = S - 1; f >= 4; --f) {
-      forward(ev, s, w, f);
-      VELO_PHASE(3);
-      const int step = (S - 1 - f) & 1;
-      if (w.alone() || step == w.parity()) {
-        if (pairs) {
-          uint32_t* map = s.seed.map[w.parity()];
-          const int gt = w.idx() * 32 + lane, gn = w.of() * 32;
-          for (int i = gt; i < kMapRows; i += gn) map[i] = 0;
-          group_sync<Shared::kMaxWarps>(w);
-          if (map_valid(s, f - 2, f - 4))
-            for (int i = gt; i < s.num(f - 4); i += gn) mark_map(ev, s, map, f - 2, f - 4, i);
-          group_sync<Shared::kMaxWarps>(w);
-          seed_pairs(ev, s, w, f);
-        } else {
-          group_sync<Shared::kMaxWarps>(w);
-          if (kMode == kLearned && learned)
-            seed_module<kLearned, kLanes>(ev, s, w, f, sl);
-          else
-            w = seed_windows<kMode == kDump ? kDump : kPlain, kLanes>(ev, s, w, f);
-        }
-        group_sync<Shared::kMaxWarps>(w);
-      }
-      if (step == 1 || f == 4) __syncthreads();
-      VELO_PHASE(4);
-    }
+    constexpr int kOther = kMode == kDump ? kDump : kPlain;
+    if (kMode == kDump || !ev.plain)
+      w = learned ? module_loop_any<kMode, kLanes, false>(ev, s, w) : module_loop_any<kOther, kLanes, false>(ev, s, w);
+    else if (kMode == kLearned && !learned)
+      w = module_loop_any<kPlain, kLanes, true>(ev, s, w);
+    else if constexpr (kMode != kDump)
+      w = module_loop<kMode, kLanes, true>(ev, s, w);
+    VELO_PHASE(4);
 
     // leftover tracklets become weak (Kernel.cl:771-792)
     if (ev.H > VELO_TTF_MODULO / 2 && lane == 0) atomicAdd(&s.inflight[3], min(w.n, kInflightMax));
     for (uint32_t i0 = 0; i0 < w.n; i0 += 32) {   // warp-uniform
-      const uint32_t v = i0 + lane < w.n ? ev.entry_words()[w.row + i0 + lane].x : 0u;
+      const uint32_t v = i0 + lane < w.n ? ev.entry_words[w.row + i0 + lane].x : 0u;
       const unsigned m = __ballot_sync(kFull, (v & kTrackletFlag) != 0);
-      if (v & kTrackletFlag) ev.weak()[w.row + w.weak + (uint32_t)__popc(m & lanemask_lt())] = v & kEntryNumber;
+      if (v & kTrackletFlag) ev.weak[w.row + w.weak + (uint32_t)__popc(m & lanemask_lt())] = v & kEntryNumber;
       w.weak += __popc(m);
     }
     __syncwarp();
@@ -1490,13 +1699,13 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
       uint4 t = make_uint4(0, 0, 0, 0);
       bool take = false;
       if (i0 + lane < w.weak) {
-        t = ev.tracklets()[w.row + ev.weak()[w.row + i0 + lane]];
+        t = ev.tracklets[w.row + ev.weak[w.row + i0 + lane]];
         take = ((ev.useds()[t.x] | ev.useds()[t.y] | ev.useds()[t.z]) & kUsed) == 0;
       }
       const unsigned m = __ballot_sync(kFull, take);
       if (take) {
         uint32_t* wr =
-            reinterpret_cast<uint32_t*>(&ev.tracks()[w.row + w.tracks + (uint32_t)__popc(m & lanemask_lt())]);
+            reinterpret_cast<uint32_t*>(&ev.tracks[w.row + w.tracks + (uint32_t)__popc(m & lanemask_lt())]);
         wr[0] = 3; wr[1] = t.x; wr[2] = t.y; wr[3] = t.z;
       }
       w.tracks += __popc(m);
@@ -1539,11 +1748,24 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
     const unsigned long long first = s.out_first + before;
     const unsigned long long room = first < p.out_capacity ? p.out_capacity - first : 0ull;
     const uint32_t words = (uint32_t)min((unsigned long long)w.tracks, room) * 25u;
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(ev.tracks() + w.row);
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(ev.tracks + w.row);
     uint32_t* dst = reinterpret_cast<uint32_t*>(p.out_tracks + first);
-    for (uint32_t i = lane; i < words; i += 32) {   // words past a track's last hit are zero
-      const uint32_t t = i / 25u;
-      dst[i] = i - 25u * t <= src[25u * t] ? src[i] : 0u;
+    // whole 128-byte lines per warp, as in the staging
+    const int count_words = (int)words;
+    const int skew = count_words > 0 ? (int)((reinterpret_cast<uintptr_t>(dst) >> 2) & 31u) : 0;   // none: no pass
+    for (int i0 = lane - skew; i0 < count_words; i0 += 32 * kCopyWords) {
+      uint32_t v[kCopyWords], hits[kCopyWords];
+#pragma unroll
+      for (int k = 0; k < kCopyWords; ++k) {
+        const uint32_t i = (uint32_t)min(max(i0 + 32 * k, 0), count_words - 1);
+        v[k] = src[i];
+        hits[k] = src[i / 25u * 25u];
+      }
+#pragma unroll
+      for (int k = 0; k < kCopyWords; ++k) {   // words past a track's last hit are zero
+        const int i = i0 + 32 * k;
+        if (i >= 0 && i < count_words) dst[i] = (uint32_t)i % 25u <= hits[k] ? v[k] : 0u;
+      }
     }
   }
   if (p.results) {   // streaming: the tracks first, then the record
@@ -1558,11 +1780,10 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
 // Builds: up to 256 threads per CTA with registers budgeted for 4 or for 5
 // resident 256-thread CTAs per SM (velo_options.register_ctas 4 / 5: 64 / 48
 // registers), 64-thread CTAs with 56 registers (18 CTAs per SM,
-// register_ctas 18), and 512-thread CTAs; the learned mode in the 64-register
-// build of up to 256 threads (a 56-register 64-thread learned build measured
-// slower: more of its registers spill around the scorer's calls); each for
-// one seeding width kLanes (lanes per h0), so that a kernel holds one copy of
-// the seeding loop.
+// register_ctas 18), and 512-thread CTAs; the learned mode in a build of up to
+// 256 threads with 80 registers (3 resident CTAs: 5,000 events 2.76 ms; with 64
+// registers, spilled around the scorer's calls, 3.28 ms); each for one seeding
+// width kLanes (lanes per h0 where the windows are walked).
 template <int kMaxThreads, int kMinCtas, int kMode, int kMods, int kLanes>
 __global__ void __launch_bounds__(kMaxThreads, kMinCtas) search_kernel(const __grid_constant__ SearchParams p) {
   extern __shared__ __align__(16) uint8_t dyn_smem_raw[];
@@ -1601,9 +1822,9 @@ struct SearchBuilds {
   static int launch(const SearchParams& p, int grid, int block, uint32_t smem, cudaStream_t st, int reg_ctas,
                     bool compact) {
     if (p.mlp && compact)
-      search_kernel<256, 4, kLearned, kCompactModules, G><<<grid, min(block, 256), smem, st>>>(p);
+      search_kernel<256, 3, kLearned, kCompactModules, G><<<grid, min(block, 256), smem, st>>>(p);
     else if (p.mlp)
-      search_kernel<256, 4, kLearned, kFullModules, G><<<grid, min(block, 256), smem, st>>>(p);
+      search_kernel<256, 3, kLearned, kFullModules, G><<<grid, min(block, 256), smem, st>>>(p);
     else if (G == 32 && p.dump_features)
       search_kernel<256, 4, kDump, kFullModules, 32><<<grid, min(block, 256), smem, st>>>(p);
     else if (block > 256)
@@ -1634,8 +1855,8 @@ struct SearchBuilds {
     VELO_LIMIT(search_kernel<64, 18, kPlain, kFullModules, G>);
     VELO_LIMIT(search_kernel<64, 18, kPlain, kCompactModules, G>);
     VELO_LIMIT(search_kernel<512, 1, kPlain, kFullModules, G>);
-    VELO_LIMIT(search_kernel<256, 4, kLearned, kFullModules, G>);
-    VELO_LIMIT(search_kernel<256, 4, kLearned, kCompactModules, G>);
+    VELO_LIMIT(search_kernel<256, 3, kLearned, kFullModules, G>);
+    VELO_LIMIT(search_kernel<256, 3, kLearned, kCompactModules, G>);
     if (G == 32) VELO_LIMIT(search_kernel<256, 4, kDump, kFullModules, 32>);
 #undef VELO_LIMIT
     return (int)e;
@@ -1644,9 +1865,9 @@ struct SearchBuilds {
   static int occupancy(int block, uint32_t smem, int reg_ctas, int mode, bool compact, int* ctas) {
     if (mode == kModeLearned)
       return compact ? (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                           ctas, search_kernel<256, 4, kLearned, kCompactModules, G>, min(block, 256), smem)
+                           ctas, search_kernel<256, 3, kLearned, kCompactModules, G>, min(block, 256), smem)
                      : (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                           ctas, search_kernel<256, 4, kLearned, kFullModules, G>, min(block, 256), smem);
+                           ctas, search_kernel<256, 3, kLearned, kFullModules, G>, min(block, 256), smem);
     if (mode == kModeDump)
       return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, search_kernel<256, 4, kDump, kFullModules, 32>,
                                                                 min(block, 256), smem);

@@ -88,3 +88,27 @@ def test_general_path_beside_it(gpu_ctx, oracle_lib):
     for threads in (32, 64, 128):
         compared, tracks = _check(gpu_ctx, oracle_lib, blobs, 4, threads_per_event=threads)
         assert compared == len(blobs) and tracks > 0
+
+
+@pytest.mark.parametrize("y, min_window", [(4, 0), (4, 3), (3, 0), (1, 2)])
+def test_learned_pairs(gpu_ctx, y, min_window):
+    """Doublets scored in the queue's batches against doublets scored where the
+    windows are walked (narrow_windows = 0): with a window margin beyond the
+    exact cut the network only prunes, so both keep the same doublets, and the
+    keep-rate guard, which counts every scored one, sends the same events back."""
+    from cl_forward_gb300 import generator, learned, native
+    blobs = [native.sort_by_x(b) for b in generator.generate(range(5200, 5216))[0]]
+    blobs += [_event(9500 + k, 33, "one") for k in range(4)] + [_event(9600, 20, "two")]
+    w = learned.init_weights(11)
+    ds = learned.build_dataset(gpu_ctx, blobs[:16])
+    logits = native.mlp_forward(w, ds.x)[:, 0]
+    threshold = float(np.quantile(logits, 0.4))
+    opts = dict(learned=1, y_lanes=y, learned_min_window=min_window)
+    for guard in (0.0, 0.6, 1.0):
+        gpu_ctx.set_mlp(w, threshold, 100.0, guard)
+        got, status = gpu_ctx.search(blobs, native.default_options(**opts))
+        walked, wstatus = gpu_ctx.search(blobs, native.default_options(narrow_windows=0, **opts))
+        assert np.array_equal(status, wstatus)
+        for e in range(len(blobs)):
+            assert index_lists(got[e]) == index_lists(walked[e]), f"event {e}, guard {guard}"
+    assert np.any(status & native.EVENT_LEARNED_FALLBACK)
