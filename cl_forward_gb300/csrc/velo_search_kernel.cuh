@@ -71,15 +71,19 @@ constexpr uint8_t kSorted = 1, kDeadTail = 2;
 // occupancy map of the h2 module.  kOwn: the h0s a warp seeds at once.
 constexpr int kMapRows = 64;          // 64 rows x 32 columns of cells
 constexpr int kQueue = 32;            // pairs a warp holds for the exact fits
-template <int kWarps, int kOwn>
+template <int kWarps, int kOwn, int kList>
 struct SeedShared {
-  float4 h0[kWarps][kOwn];            // x, y, z, first h1 - first pair (int bits)
+  float4 h0[kWarps][kOwn];            // x, y, z, first h1's place - first pair (int bits)
   float2 reach[kWarps][kOwn];         // the h0's y cut, and in plain geometry (z2 - z0) / (z1 - z0)
   unsigned long long best[kWarps][kOwn];   // the h0's best (fit, Y-lane, h1, h2) so far
   uint32_t map[2][kMapRows];
   std::conditional_t<(kOwn > 4), uint32_t, uint16_t> queue[kWarps][kQueue];   // h0 << 14 | h1 in its module
   uint16_t first[kWarps][kOwn];       // the h0's first h1 in its module
-  uint8_t active[kWarps][32];         // the warp's unused h0s of a block of 32 hits
+  // by parity: the usable h1s (unused, with an h2 window) of a module of up to
+  // kList hits; per 32 hits their lanes and their number before
+  uint2 usable[2][kList / 32 + 1];
+  uint8_t list[2][kList];
+  uint8_t active[2][32];              // by parity: unused h0s of a block of 32 hits, by rank
 };
 
 // Per-CTA shared state for events of up to kMods modules.  Launches whose
@@ -92,7 +96,8 @@ struct SharedT {
   // more than 16 unused; the others keep the static state below 8 KB
   static constexpr int kOwn = kWarps <= 2 ? 16 : kMods <= kCompactModules ? 64 / kWarps : 16 / kWarps + (kWarps <= 8) * 2;
   static constexpr int kMaxWarps = kWarps;
-  SeedShared<kWarps, kOwn> seed;
+  static constexpr int kList = kMods <= kCompactModules ? 256 : 64;
+  SeedShared<kWarps, kOwn, kList> seed;
   int32_t start[kMods];       // [S] = H
   int32_t sz[kMods];
   float zmin[kMods];
@@ -406,7 +411,8 @@ constexpr uint32_t kInflightMax = 2 * VELO_TTF_MODULO;
 
 // The unused h0s of hits [block, block + 32) of module f (Kernel.cl:720-764)
 // are dealt by rank to the warps of the module's parity; their number for
-// this warp, the hits (relative to block) in `active`.
+// this warp; its c-th is hit block + active[idx + c of].  A warp writes and
+// reads its own ranks only.
 __device__ __forceinline__ int active_h0s(const EventView& ev, const Worker& w, int st0, int n0, int block,
                                           uint8_t* active) {
   __syncwarp();   // the previous block's list has been read
@@ -414,7 +420,7 @@ __device__ __forceinline__ int active_h0s(const EventView& ev, const Worker& w, 
   const bool unused = block + lane < n0 && !(ev.useds()[st0 + block + lane] & kUsed);
   const unsigned m = __ballot_sync(kFull, unused);
   const int rank = __popc(m & lanemask_lt()), total = __popc(m);
-  if (unused && (rank & (w.of() - 1)) == w.idx()) active[rank / w.of()] = (uint8_t)lane;
+  if (unused && (rank & (w.of() - 1)) == w.idx()) active[rank] = (uint8_t)lane;
   __syncwarp();
   return (total + w.of() - 1 - w.idx()) / w.of();
 }
@@ -679,9 +685,9 @@ __device__ __forceinline__ SeedLanes seed_lanes_of(int G, uint32_t Y) {
 
 // Features and MLP of the learned seeding for the warp's doublets: lanes
 // with score == false pass zeros and ignore the result.  All 32 lanes call it
-// together.  Kept out of line, so that the seeding loop keeps the plain
-// method's registers wherever nothing is scored.
-static __device__ __noinline__ float2 score_doublets(const MlpFrag* mlp, bool score, float h0x, float h0y, float h0z,
+// together.  score_doublets keeps it out of line where the windows are walked,
+// so that the loop keeps its registers wherever nothing is scored.
+static __device__ __forceinline__ float2 score_batch(const MlpFrag* mlp, bool score, float h0x, float h0y, float h0z,
                                               float h1x, float h1y, float h1z, float dz_inv, float zmid4,
                                               int h2_window, int f, int n_modules, float dymax) {
   float feat[kMlpIn];
@@ -695,6 +701,12 @@ static __device__ __noinline__ float2 score_doublets(const MlpFrag* mlp, bool sc
   float logit, width;
   mlp_eval_warp(*mlp, feat, &logit, &width);
   return make_float2(logit, width);
+}
+
+static __device__ __noinline__ float2 score_doublets(const MlpFrag* mlp, bool score, float h0x, float h0y, float h0z,
+                                              float h1x, float h1y, float h1z, float dz_inv, float zmid4,
+                                              int h2_window, int f, int n_modules, float dymax) {
+  return score_batch(mlp, score, h0x, h0y, h0z, h1x, h1y, h1z, dz_inv, zmid4, h2_window, f, n_modules, dymax);
 }
 
 // Seeding of module f: h0 on f, h1 on f-2, h2 on f-4 (Kernel.cl:392-568
@@ -730,13 +742,13 @@ __device__ void seed_module(const EventView& ev, Shared& s, Worker& w, int f, co
   uint32_t zk0 = 0x7fc00001u, zk1 = 0x7fc00001u;
   float dz_inv_cached = 0.f;
 
-  uint8_t* active = s.seed.active[w.warp()];
+  uint8_t* active = s.seed.active[w.parity()];
   for (int block = 0; block < n0; block += 32)                    // warp-uniform
   for (int c0 = 0, mine = active_h0s(ev, w, st0, n0, block, active); c0 < mine; c0 += kGroups) {
     int h0 = 0, n1 = 0;
     uint32_t f1 = 0;
     if (c0 + lane / G < mine) {
-      h0 = st0 + block + active[c0 + lane / G];
+      h0 = st0 + block + active[w.idx() + (c0 + lane / G) * w.of()];
       const uint32_t w0 = ev.wins()[h0].x;
       f1 = w0 & 0xffffu;
       if (f1 != kNone16) n1 = (int)(w0 >> 16) - (int)f1;
@@ -1087,6 +1099,24 @@ __device__ __forceinline__ Fit pair_fit_any(const EventView& ev, const Shared& s
   return fit;
 }
 
+// The usable h1s of module s1, for the seeding of its parity (one warp).  Half
+// of a module's hits are used or without an h2 window by then: pairs with them
+// are not formed (see seed_pairs).  Larger modules are paired hit by hit.
+template <class Shared>
+__device__ __forceinline__ void list_h1s(const EventView& ev, Shared& s, const Worker& w, int s1) {
+  const int lane = threadIdx.x & 31, st1 = s.start[s1], n1 = s.num(s1);
+  if (n1 > Shared::kList) return;
+  int before = 0;
+  for (int i0 = 0; i0 <= n1; i0 += 32) {   // n1 itself has a place too: the end of a window
+    const int i = i0 + lane;
+    const bool usable = i < n1 && ev.useds()[st1 + i] == 0;
+    const unsigned m = __ballot_sync(kFull, usable);
+    if (lane == 0) s.seed.usable[w.parity()][i0 >> 5] = make_uint2(m, (unsigned)before);
+    if (usable) s.seed.list[w.parity()][before + __popc(m & lanemask_lt())] = (uint8_t)i;
+    before += __popc(m);
+  }
+}
+
 template <int kMode, bool kPlainGeometry, class Shared>
 __device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Worker& w, int f) {
   constexpr int kOwn = Shared::kOwn;
@@ -1096,6 +1126,8 @@ __device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Worke
   const int st0 = s.start[f], n0 = s.num(f), st1 = s.start[s1], st4 = s.start[m4], n4 = s.num(m4);
   const float zmin1 = s.zmin[s1], zmin4 = s.zmin[m4];
   const uint32_t* map = sd.map[w.parity()];
+  const bool listed = s.num(s1) <= Shared::kList;   // list_h1s has run
+  const uint8_t* list = sd.list[w.parity()];
   float4* own_h0 = sd.h0[w.warp()];
   float2* own_reach = sd.reach[w.warp()];
   unsigned long long* own_best = sd.best[w.warp()];
@@ -1110,17 +1142,23 @@ __device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Worke
   const float s1_z = ev.zs()[st1];   // Kernel.cl:420
 
   for (int block = 0; block < n0; block += 32)   // warp-uniform
-  for (int c0 = 0, mine = active_h0s(ev, w, st0, n0, block, sd.active[w.warp()]); c0 < mine; c0 += kOwn) {
-    int h0 = 0, first = 0, count = 0;
+  for (int c0 = 0, mine = active_h0s(ev, w, st0, n0, block, sd.active[w.parity()]); c0 < mine; c0 += kOwn) {
+    int h0 = 0, first = 0, count = 0, from = 0;
     float h0x = 0.f, h0y = 0.f, h0z = 0.f;
     if (lane < kOwn && c0 + lane < mine) {
-      h0 = st0 + block + sd.active[w.warp()][c0 + lane];
+      h0 = st0 + block + sd.active[w.parity()][w.idx() + (c0 + lane) * w.of()];
       h0x = ev.xs()[h0];
       h0y = ev.ys()[h0];
       h0z = ev.zs()[h0];
       int last;
       h1_window(ev, s, s1, h0x, h0z, &first, &last);
       count = max(last - first, 0);
+      from = first;
+      if (listed && count > 0) {   // the window's usable h1s
+        const uint2 u = sd.usable[w.parity()][first >> 5], v = sd.usable[w.parity()][last >> 5];
+        from = (int)(u.y + __popc(u.x & ((1u << (first & 31)) - 1u)));
+        count = (int)(v.y + __popc(v.x & ((1u << (last & 31)) - 1u))) - from;
+      }
     }
     // the pairs of the warp's h0s, end to end
     int end = count;
@@ -1136,7 +1174,7 @@ __device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Worke
     const int slot = __popc(om & lanemask_lt());
     __syncwarp();   // the previous round's lists have been read
     if (count > 0) {
-      own_h0[slot] = make_float4(h0x, h0y, h0z, __int_as_float(st1 + first - begin));
+      own_h0[slot] = make_float4(h0x, h0y, h0z, __int_as_float(from - begin));
       own_reach[slot] = make_float2(fmul(kMaxYSlope, fabsf(fsub(s1_z, h0z))),
                                    fmul(fsub(zmin4, h0z), fdiv(1.f, fsub(zmin1, h0z))));
       own_best[slot] = ~0ull;
@@ -1158,10 +1196,11 @@ __device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Worke
         if (base + lane < total) {
           const float4 q = own_h0[o];
           const float2 r = own_reach[o];
-          h1 = __float_as_int(q.w) + base + lane;
-          const uint8_t u1 = ev.useds()[h1];
+          const int at = __float_as_int(q.w) + base + lane;
+          h1 = st1 + (listed ? (int)list[at] : at);
+          const bool usable = listed || ev.useds()[h1] == 0;
           const float h1x = ev.xs()[h1], h1y = ev.ys()[h1];
-          pass = u1 == 0 && fabsf(fsub(h1y, q.y)) < r.x;
+          pass = usable && fabsf(fsub(h1y, q.y)) < r.x;
           if (kPlainGeometry && kMode == kPlain && pass) {   // the fit's own predicted point
             const float px = fadd(q.x, fmul(fsub(h1x, q.x), r.y));
             const float py = fadd(q.y, fmul(fsub(h1y, q.y), r.y));
@@ -1199,7 +1238,7 @@ __device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Worke
           const bool score = reached && b - a >= ev.p->learned_min_window;
           bool keep = true;
           if (__any_sync(kFull, score)) {
-            const float2 r = score_doublets(ev.mlp, score, q.x, q.y, q.z, h1x, h1y, zmin1,
+            const float2 r = score_batch(ev.mlp, score, q.x, q.y, q.z, h1x, h1y, zmin1,
                                             fdiv(1.f, fsub(zmin1, q.z)), 0.5f * (zmin4 + zmin4), b - a, f, ev.S,
                                             reached ? own_reach[own].x : 0.f);
             if (score) {
@@ -1448,18 +1487,22 @@ __device__ __forceinline__ Worker module_loop(const EventView& ev, Shared& s, Wo
     forward<kPlainGeometry>(ev, s, w, f);
     const int step = (S - 1 - f) & 1;
     if (w.alone() || step == w.parity()) {
-      if (kMode != kDump && kPlainGeometry) {
-        uint32_t* map = s.seed.map[w.parity()];
-        const int gt = w.idx() * 32 + lane, gn = w.of() * 32;
+      const bool by_pairs = kPlainGeometry || (kMode == kPlain && ev.tame);
+      uint32_t* map = s.seed.map[w.parity()];
+      const int gt = w.idx() * 32 + lane, gn = w.of() * 32;
+      if (kPlainGeometry)
         for (int i = gt; i < kMapRows; i += gn) map[i] = 0;
-        group_sync<Shared::kMaxWarps>(w);
-        for (int i = gt; i < s.num(f - 4); i += gn) mark_map(ev, s, map, f - 2, f - 4, i);
-      }
       group_sync<Shared::kMaxWarps>(w);
+      if (by_pairs) {
+        if (w.idx() == 0) list_h1s(ev, s, w, f - 2);
+        if (kPlainGeometry)   // from the group's last warp on
+          for (int i = gn - 1 - gt; i < s.num(f - 4); i += gn) mark_map(ev, s, map, f - 2, f - 4, i);
+        group_sync<Shared::kMaxWarps>(w);
+      }
       if constexpr (kPlainGeometry) {
         seed_pairs<kMode, true>(ev, s, w, f);
       } else {
-        if (kMode == kPlain && ev.tame)
+        if (by_pairs)
           seed_pairs<kPlain, false>(ev, s, w, f);
         else
           seed_module<kMode, kLanes>(ev, s, w, f, seed_lanes_of(kLanes, (uint32_t)ev.y_lanes));
