@@ -669,9 +669,8 @@ velo_status check_options(velo_ctx* c, const velo_options* opts, velo_options* o
     c->err = "seed_lanes below 32 must be a multiple of y_lanes";
     return VELO_ERR_INVALID_ARGUMENT;
   }
-  if (o->register_ctas == 0) o->register_ctas = o->threads_per_event <= 64 ? 18 : 5;
-  if (o->register_ctas != 4 && o->register_ctas != 5 && o->register_ctas != 18) {
-    c->err = "register_ctas must be 4, 5 or 18";
+  if (o->register_ctas != 0 && o->register_ctas != 4 && o->register_ctas != 5 && o->register_ctas != 18) {
+    c->err = "register_ctas must be 0, 4, 5 or 18";
     return VELO_ERR_INVALID_ARGUMENT;
   }
   if (o->register_ctas == 18 && o->threads_per_event > 64) {
@@ -691,6 +690,33 @@ velo_status check_options(velo_ctx* c, const velo_options* opts, velo_options* o
     o->use_graph = 0;
   }
   return VELO_OK;
+}
+
+// The launch that automatic options stand for, on the staged batch.  A
+// persistent launch of 64-thread CTAs is the fastest for large batches, but
+// it leaves a small one waiting for its largest event: with the automatic
+// register build, CTAs are widened while the batch takes few rounds of them.
+// Milliseconds with 64 / 128 / 256 / 512 threads (events of 1,160 hits; of
+// 4,550 hits):
+//     100 events  0.41  0.30  0.25  0.25    2.7  1.5  1.0  0.8
+//   1,003         0.85  0.60  0.45  1.08    4.8  2.9  1.9  3.3
+//   2,500         0.96  0.70  0.94  2.6     6.0  3.4  3.5  8.1
+//   4,000         1.04  0.97  1.44  4.2     5.9  4.0  4.9  12.8
+//   7,000         1.23  1.61  2.49  7.2
+// Resident CTAs per SM: 16, 8, 4 and 1 (learned: 12, 6 and 3).
+void resolve_launch(const velo_ctx* c, velo_options* o) {
+  const bool learned = o->learned != 0;
+  if (o->register_ctas == 0 && o->threads_per_event == 64 && o->launch_mode == VELO_LAUNCH_PERSISTENT &&
+      o->ctas_per_sm <= 0 && !c->dump_armed) {
+    const int64_t n = c->n, sms = c->sm_count;
+    if (n <= sms && !learned)
+      o->threads_per_event = 512;
+    else if (n <= (learned ? 6 : 8) * sms)
+      o->threads_per_event = 256;
+    else if (n <= (learned ? 18 : 24) * sms)
+      o->threads_per_event = 128;
+  }
+  if (o->register_ctas == 0) o->register_ctas = o->threads_per_event > 256 ? 5 : 4;
 }
 
 // Grid of the launch (the occupancy query stays outside any stream capture).
@@ -830,6 +856,7 @@ velo_status velo_run(velo_ctx* c, const velo_options* opts) {
   velo_options o;
   velo_status st = check_options(c, opts, &o);
   if (st != VELO_OK) return st;
+  resolve_launch(c, &o);
   VELO_CUDA(c, cudaSetDevice(c->device));
   uint32_t smem = 0;
   if ((st = prepare_launch(c, o, &smem)) != VELO_OK) return st;
@@ -1444,6 +1471,7 @@ velo_status velo_time_runs(velo_ctx* c, const velo_options* opts, int32_t warmup
   velo_options o;
   velo_status st = check_options(c, opts, &o);
   if (st != VELO_OK) return st;
+  resolve_launch(c, &o);
   VELO_CUDA(c, cudaSetDevice(c->device));
   uint32_t smem = 0;
   if ((st = prepare_launch(c, o, &smem)) != VELO_OK) return st;

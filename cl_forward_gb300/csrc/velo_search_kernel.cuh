@@ -1101,7 +1101,9 @@ __device__ __forceinline__ Fit pair_fit_any(const EventView& ev, const Shared& s
 
 // The usable h1s of module s1, for the seeding of its parity (one warp).  Half
 // of a module's hits are used or without an h2 window by then: pairs with them
-// are not formed (see seed_pairs).  Larger modules are paired hit by hit.
+// are not formed (6,950 -> 3,930 pairs an event of 1,160 hits, 103,000 ->
+// 54,000 of 4,400: 10,000 uneven events 5.3 -> 4.5 ms, 4,000 dense ones 6.7 ->
+// 6.2 ms).  Larger modules are paired hit by hit.
 template <class Shared>
 __device__ __forceinline__ void list_h1s(const EventView& ev, Shared& s, const Worker& w, int s1) {
   const int lane = threadIdx.x & 31, st1 = s.start[s1], n1 = s.num(s1);
@@ -1822,10 +1824,11 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
 
 // Builds: up to 256 threads per CTA with registers budgeted for 4 or for 5
 // resident 256-thread CTAs per SM (velo_options.register_ctas 4 / 5: 64 / 48
-// registers), 64-thread CTAs with 56 registers (18 CTAs per SM,
-// register_ctas 18), and 512-thread CTAs; the learned mode in a build of up to
-// 256 threads with 80 registers (3 resident CTAs: 5,000 events 2.76 ms; with 64
-// registers, spilled around the scorer's calls, 3.28 ms); each for one seeding
+// registers; of up to 64 threads in a build with the seeding state of two
+// warps), 64-thread CTAs with 56 registers (18 CTAs per SM, register_ctas 18),
+// and 512-thread CTAs; the learned mode in a build of up to
+// 256 threads with 80 registers (3 resident CTAs; 2.76 against 3.28 ms with 64
+// for 5,000 events with the scorer out of line, 2.02 ms with it inlined); each for one seeding
 // width kLanes (lanes per h0 where the windows are walked).
 template <int kMaxThreads, int kMinCtas, int kMode, int kMods, int kLanes>
 __global__ void __launch_bounds__(kMaxThreads, kMinCtas) search_kernel(const __grid_constant__ SearchParams p) {
@@ -1876,6 +1879,10 @@ struct SearchBuilds {
       search_kernel<64, 18, kPlain, kCompactModules, G><<<grid, block, smem, st>>>(p);
     else if (reg_ctas == 18)
       search_kernel<64, 18, kPlain, kFullModules, G><<<grid, block, smem, st>>>(p);
+    else if (reg_ctas == 4 && block <= 64 && compact)
+      search_kernel<64, 16, kPlain, kCompactModules, G><<<grid, block, smem, st>>>(p);
+    else if (reg_ctas == 4 && block <= 64)
+      search_kernel<64, 16, kPlain, kFullModules, G><<<grid, block, smem, st>>>(p);
     else if (reg_ctas == 4 && compact)
       search_kernel<256, 4, kPlain, kCompactModules, G><<<grid, block, smem, st>>>(p);
     else if (reg_ctas == 4)
@@ -1897,6 +1904,8 @@ struct SearchBuilds {
     VELO_LIMIT(search_kernel<256, 5, kPlain, kCompactModules, G>);
     VELO_LIMIT(search_kernel<64, 18, kPlain, kFullModules, G>);
     VELO_LIMIT(search_kernel<64, 18, kPlain, kCompactModules, G>);
+    VELO_LIMIT(search_kernel<64, 16, kPlain, kFullModules, G>);
+    VELO_LIMIT(search_kernel<64, 16, kPlain, kCompactModules, G>);
     VELO_LIMIT(search_kernel<512, 1, kPlain, kFullModules, G>);
     VELO_LIMIT(search_kernel<256, 3, kLearned, kFullModules, G>);
     VELO_LIMIT(search_kernel<256, 3, kLearned, kCompactModules, G>);
@@ -1922,6 +1931,11 @@ struct SearchBuilds {
                            ctas, search_kernel<64, 18, kPlain, kCompactModules, G>, block, smem)
                      : (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                            ctas, search_kernel<64, 18, kPlain, kFullModules, G>, block, smem);
+    if (reg_ctas == 4 && block <= 64)
+      return compact ? (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                           ctas, search_kernel<64, 16, kPlain, kCompactModules, G>, block, smem)
+                     : (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                           ctas, search_kernel<64, 16, kPlain, kFullModules, G>, block, smem);
     if (reg_ctas == 4)
       return compact ? (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                            ctas, search_kernel<256, 4, kPlain, kCompactModules, G>, block, smem)

@@ -171,8 +171,9 @@ extern "C" velo_status velo_search_device_static(const uint8_t* d_input, const u
   const uint32_t smem = arena_layout(max_event_hits, M, (uint32_t)y_lanes).total;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return VELO_ERR_CUDA;
-  int optin = 0;
-  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+  int optin = 0, sms = 0;
+  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return VELO_ERR_CUDA;
   if (smem > (uint32_t)(optin > 8192 ? optin - 8192 : 0)) return VELO_ERR_CAPACITY;   // event too large to stage
   void* base = nullptr;
@@ -224,6 +225,8 @@ extern "C" velo_status velo_search_device_static(const uint8_t* d_input, const u
   p.out_status = d_status;
   p.out_cursor = v.cursor;
   p.work_counter = v.work;
-  if (launch_search(p, n_events, 256, smem, s, 5, false) != 0) return VELO_ERR_CUDA;
+  // wide CTAs while there is at most one per SM, as velo_run's automatic launch
+  const int threads = n_events <= sms ? 512 : n_events <= 8 * sms ? 256 : 128;
+  if (launch_search(p, n_events, threads, smem, s, 4, false) != 0) return VELO_ERR_CUDA;
   return VELO_OK;
 }

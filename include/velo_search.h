@@ -92,7 +92,9 @@ typedef struct velo_options {
   int32_t register_ctas;      /* 4 or 5: kernel build whose registers fit that many 256-thread
                                  CTAs per SM (64 or 48 registers); 18: the 64-thread build with
                                  56 registers (18 CTAs per SM; threads_per_event <= 64 only);
-                                 0 = 18 for <= 64 threads, else 5 */
+                                 0 = automatic: 4, and a persistent launch of 64 threads with
+                                 automatic ctas_per_sm widens its CTAs (up to 512 threads) for
+                                 batches that are small for the device */
   int32_t learned;            /* 1: seeding prunes doublets with the MLP set by velo_set_mlp
                                  (approximate; no counterpart in the reference) */
   int32_t pipeline_events;    /* velo_search / velo_search_packed: > 0 cuts a batch of more than
