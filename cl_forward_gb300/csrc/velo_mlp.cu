@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include <algorithm>
 #include <cstring>
 #include <vector>
 
@@ -301,20 +302,28 @@ __global__ void __launch_bounds__(256) mlp_forward_kernel(const float* __restric
 
 namespace {
 
+// The device arrays of one call, in one allocation (each cudaMalloc / cudaFree
+// pair takes 70 us): reserve them all, then allocate.
 struct DevArrays {
-  std::vector<void*> ptrs;
-  cudaStream_t stream = nullptr;
+  uint8_t* base = nullptr;
+  size_t total = 0;
+  cudaStream_t stream = nullptr, aux = nullptr;
   ~DevArrays() {
     if (stream) cudaStreamSynchronize(stream);
-    for (void* p : ptrs) cudaFree(p);
+    if (aux) cudaStreamSynchronize(aux);
+    if (base) cudaFree(base);
     if (stream) cudaStreamDestroy(stream);
+    if (aux) cudaStreamDestroy(aux);
   }
   template <typename T>
-  cudaError_t alloc(T** p, size_t count) {
-    cudaError_t e = cudaMalloc((void**)p, sizeof(T) * (count ? count : 1));
-    if (e == cudaSuccess) ptrs.push_back(*p);
-    return e;
+  size_t reserve(size_t count) {
+    const size_t at = total;
+    total += (sizeof(T) * (count ? count : 1) + 255) & ~(size_t)255;
+    return at;
   }
+  cudaError_t allocate() { return cudaMalloc(reinterpret_cast<void**>(&base), total); }
+  template <typename T>
+  T* at(size_t offset) const { return reinterpret_cast<T*>(base + offset); }
 };
 
 #define MLP_CHECK(call)                      \
@@ -347,13 +356,27 @@ cudaError_t launch_step(cudaStream_t stream, bool follows, const float* w, const
                             adam);
 }
 
-// splitmix64 for the host-side batch sampling
-uint64_t mix(uint64_t& s) {
-  uint64_t z = (s += 0x9E3779B97F4A7C15ull);
+// splitmix64: the k-th value (k from 1) of the sequence that starts at `seed`.
+__host__ __device__ __forceinline__ uint64_t splitmix(uint64_t seed, uint64_t k) {
+  uint64_t z = seed + k * 0x9E3779B97F4A7C15ull;
   z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
   z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
   return z ^ (z >> 31);
 }
+
+// The draws of `count` places of the epochs' shuffles from place `first` on:
+// an epoch swaps element i (n-1 down to 1) with element value % (i + 1).  The
+// 64-bit remainder took the host 5.4 ns a draw, four times the swap itself.
+__global__ void shuffle_draws_kernel(uint64_t seed, uint64_t n, uint64_t first, uint64_t count,
+                                     uint32_t* __restrict__ out) {
+  for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < count; k += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t i = n - 1 - (first + k) % (n - 1);
+    out[k] = (uint32_t)(splitmix(seed, first + k + 1) % (i + 1));
+  }
+}
+
+// Draws made per launch: enough epochs to make the launch worth it.
+constexpr uint64_t kDrawsAtOnce = 1u << 20;
 
 }  // namespace
 }  // namespace velo
@@ -364,13 +387,12 @@ extern "C" velo_status velo_mlp_grad(const float* weights, const float* x, const
                                      int64_t n, float* grad_out, float* loss_out) {
   if (!weights || !x || !label || !target || n <= 0 || !grad_out) return VELO_ERR_INVALID_ARGUMENT;
   DevArrays d;
-  float *dw, *dx, *dl, *dt, *dg, *dloss;
-  MLP_CHECK(d.alloc(&dw, VELO_MLP_PARAMS));
-  MLP_CHECK(d.alloc(&dx, (size_t)n * kMlpIn));
-  MLP_CHECK(d.alloc(&dl, (size_t)n));
-  MLP_CHECK(d.alloc(&dt, (size_t)n));
-  MLP_CHECK(d.alloc(&dg, VELO_MLP_PARAMS));
-  MLP_CHECK(d.alloc(&dloss, 1));
+  const size_t ow = d.reserve<float>(VELO_MLP_PARAMS), ox = d.reserve<float>((size_t)n * kMlpIn),
+               ol = d.reserve<float>((size_t)n), ot = d.reserve<float>((size_t)n),
+               og = d.reserve<float>(VELO_MLP_PARAMS), oloss = d.reserve<float>(1);
+  MLP_CHECK(d.allocate());
+  float *dw = d.at<float>(ow), *dx = d.at<float>(ox), *dl = d.at<float>(ol), *dt = d.at<float>(ot),
+        *dg = d.at<float>(og), *dloss = d.at<float>(oloss);
   MLP_CHECK(cudaMemcpy(dw, weights, sizeof(float) * VELO_MLP_PARAMS, cudaMemcpyHostToDevice));
   MLP_CHECK(cudaMemcpy(dx, x, sizeof(float) * n * kMlpIn, cudaMemcpyHostToDevice));
   MLP_CHECK(cudaMemcpy(dl, label, sizeof(float) * n, cudaMemcpyHostToDevice));
@@ -386,10 +408,10 @@ extern "C" velo_status velo_mlp_grad(const float* weights, const float* x, const
 extern "C" velo_status velo_mlp_forward(const float* weights, const float* x, int64_t n, float* out) {
   if (!weights || !x || n <= 0 || !out) return VELO_ERR_INVALID_ARGUMENT;
   DevArrays d;
-  float *dw, *dx, *dout;
-  MLP_CHECK(d.alloc(&dw, VELO_MLP_PARAMS));
-  MLP_CHECK(d.alloc(&dx, (size_t)n * kMlpIn));
-  MLP_CHECK(d.alloc(&dout, (size_t)n * 2));
+  const size_t ow = d.reserve<float>(VELO_MLP_PARAMS), ox = d.reserve<float>((size_t)n * kMlpIn),
+               oo = d.reserve<float>((size_t)n * 2);
+  MLP_CHECK(d.allocate());
+  float *dw = d.at<float>(ow), *dx = d.at<float>(ox), *dout = d.at<float>(oo);
   MLP_CHECK(cudaMemcpy(dw, weights, sizeof(float) * VELO_MLP_PARAMS, cudaMemcpyHostToDevice));
   MLP_CHECK(cudaMemcpy(dx, x, sizeof(float) * n * kMlpIn, cudaMemcpyHostToDevice));
   mlp_forward_kernel<<<(int)((n + 255) / 256), 256>>>(dw, dx, n, dout);
@@ -403,50 +425,74 @@ extern "C" velo_status velo_mlp_train(const float* x, const float* label, const 
                                       float* loss_per_step) {
   if (!x || !label || !target || n <= 0 || steps <= 0 || batch <= 0 || !weights_inout)
     return VELO_ERR_INVALID_ARGUMENT;
-  std::vector<int64_t> order((size_t)n), idx((size_t)steps * batch);   // outlive the copies on d.stream
+  const uint64_t places = (uint64_t)steps * (uint64_t)batch;   // samples drawn in all
+  std::vector<int64_t> idx((size_t)places);   // outlives the copies on d.stream
+  std::vector<int64_t> order((size_t)n);
+  std::vector<uint32_t> draws;
   DevArrays d;
-  float *dw, *dx, *dl, *dt, *dg, *dm, *dv, *dloss;
-  int64_t* didx;
-  unsigned int* ddone;
+  const bool device_draws = n > 1 && n <= (int64_t)0xffffffff;
+  const uint64_t swaps = (uint64_t)n - 1;   // draws of an epoch
+  const uint64_t epochs = (places + (uint64_t)n - 1) / (uint64_t)n;
+  const uint64_t epochs_at_once =
+      device_draws ? std::min(epochs, std::max<uint64_t>(1, kDrawsAtOnce / swaps)) : 1;
+  const size_t ow = d.reserve<float>(VELO_MLP_PARAMS), ox = d.reserve<float>((size_t)n * kMlpIn),
+               ol = d.reserve<float>((size_t)n), ot = d.reserve<float>((size_t)n),
+               og = d.reserve<float>(VELO_MLP_PARAMS), om = d.reserve<float>(VELO_MLP_PARAMS),
+               ov = d.reserve<float>(VELO_MLP_PARAMS), oloss = d.reserve<float>((size_t)steps),
+               odone = d.reserve<unsigned int>(1), oi = d.reserve<int64_t>((size_t)places),
+               od = d.reserve<uint32_t>(device_draws ? (size_t)(epochs_at_once * swaps) : 1);
+  MLP_CHECK(d.allocate());
+  float *dw = d.at<float>(ow), *dx = d.at<float>(ox), *dl = d.at<float>(ol), *dt = d.at<float>(ot),
+        *dg = d.at<float>(og), *dm = d.at<float>(om), *dv = d.at<float>(ov), *dloss = d.at<float>(oloss);
+  int64_t* didx = d.at<int64_t>(oi);
+  unsigned int* ddone = d.at<unsigned int>(odone);
   MLP_CHECK(cudaStreamCreateWithFlags(&d.stream, cudaStreamNonBlocking));
-  MLP_CHECK(d.alloc(&dw, VELO_MLP_PARAMS));
-  MLP_CHECK(d.alloc(&dx, (size_t)n * kMlpIn));
-  MLP_CHECK(d.alloc(&dl, (size_t)n));
-  MLP_CHECK(d.alloc(&dt, (size_t)n));
-  MLP_CHECK(d.alloc(&dg, VELO_MLP_PARAMS));
-  MLP_CHECK(d.alloc(&dm, VELO_MLP_PARAMS));
-  MLP_CHECK(d.alloc(&dv, VELO_MLP_PARAMS));
-  MLP_CHECK(d.alloc(&dloss, (size_t)steps));
-  MLP_CHECK(d.alloc(&didx, (size_t)steps * batch));
-  MLP_CHECK(d.alloc(&ddone, 1));
+  MLP_CHECK(cudaStreamCreateWithFlags(&d.aux, cudaStreamNonBlocking));
   MLP_CHECK(cudaMemcpyAsync(dw, weights_inout, sizeof(float) * VELO_MLP_PARAMS, cudaMemcpyHostToDevice, d.stream));
   MLP_CHECK(cudaMemcpyAsync(dx, x, sizeof(float) * n * kMlpIn, cudaMemcpyHostToDevice, d.stream));
   MLP_CHECK(cudaMemcpyAsync(dl, label, sizeof(float) * n, cudaMemcpyHostToDevice, d.stream));
   MLP_CHECK(cudaMemcpyAsync(dt, target, sizeof(float) * n, cudaMemcpyHostToDevice, d.stream));
-  MLP_CHECK(cudaMemsetAsync(dm, 0, sizeof(float) * VELO_MLP_PARAMS, d.stream));
-  MLP_CHECK(cudaMemsetAsync(dv, 0, sizeof(float) * VELO_MLP_PARAMS, d.stream));
-  MLP_CHECK(cudaMemsetAsync(dg, 0, sizeof(float) * VELO_MLP_PARAMS, d.stream));
-  MLP_CHECK(cudaMemsetAsync(dloss, 0, sizeof(float) * steps, d.stream));
-  MLP_CHECK(cudaMemsetAsync(ddone, 0, sizeof(unsigned int), d.stream));
-  // epoch-wise shuffled sample order
+  // gradient, moments (adjacent), losses and the counter start at zero
+  MLP_CHECK(cudaMemsetAsync(dg, 0, oi - og, d.stream));
   for (int64_t i = 0; i < n; ++i) order[(size_t)i] = i;
-  uint64_t s = seed;
-  int64_t pos = n;
-  for (size_t k = 0; k < idx.size(); ++k) {
-    if (pos == n) {
-      for (int64_t i = n - 1; i > 0; --i) std::swap(order[(size_t)i], order[(size_t)(mix(s) % (uint64_t)(i + 1))]);
-      pos = 0;
-    }
-    idx[k] = order[(size_t)pos++];
-  }
-  MLP_CHECK(cudaMemcpyAsync(didx, idx.data(), sizeof(int64_t) * idx.size(), cudaMemcpyHostToDevice, d.stream));
   const float beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
   double p1 = 1.0, p2 = 1.0;
-  for (int32_t t = 0; t < steps; ++t) {
-    p1 *= beta1;
-    p2 *= beta2;
-    MLP_CHECK(launch_step(d.stream, t > 0, dw, dx, dl, dt, didx + (size_t)t * batch, batch, dg, dloss + t, ddone,
-                          AdamStep{dw, dm, dv, lr, beta1, beta2, eps, (float)(1.0 - p1), (float)(1.0 - p2)}));
+  int32_t t = 0;
+  uint64_t filled = 0, sent = 0;
+  // epoch-wise shuffled sample order: each epoch shuffles the one before it.
+  // The steps whose samples are known are launched while the host goes on.
+  for (uint64_t e = 0; e < epochs; ++e) {
+    if (device_draws && e % epochs_at_once == 0) {
+      const uint64_t count = std::min(epochs_at_once, epochs - e) * swaps;
+      draws.resize((size_t)count);
+      const unsigned blocks = (unsigned)std::min<uint64_t>((count + 255) / 256, 4096);
+      shuffle_draws_kernel<<<blocks, 256, 0, d.aux>>>(seed, (uint64_t)n, e * swaps, count, d.at<uint32_t>(od));
+      MLP_CHECK(cudaGetLastError());
+      MLP_CHECK(cudaMemcpyAsync(draws.data(), d.at<uint32_t>(od), sizeof(uint32_t) * count, cudaMemcpyDeviceToHost,
+                                d.aux));
+      MLP_CHECK(cudaStreamSynchronize(d.aux));
+    }
+    const uint32_t* draw = draws.data() + (e % epochs_at_once) * swaps;
+    uint64_t k = e * swaps;
+    for (int64_t i = n - 1; i > 0; --i) {
+      ++k;
+      const uint64_t j = device_draws ? *draw++ : splitmix(seed, k) % (uint64_t)(i + 1);
+      std::swap(order[(size_t)i], order[(size_t)j]);
+    }
+    const uint64_t take = std::min<uint64_t>((uint64_t)n, places - filled);
+    std::copy(order.begin(), order.begin() + (ptrdiff_t)take, idx.begin() + (ptrdiff_t)filled);
+    filled += take;
+    const uint64_t ready = filled / (uint64_t)batch;   // steps
+    if (ready < (uint64_t)steps && filled - sent < kDrawsAtOnce) continue;
+    MLP_CHECK(cudaMemcpyAsync(didx + sent, idx.data() + sent, sizeof(int64_t) * (filled - sent),
+                              cudaMemcpyHostToDevice, d.stream));
+    sent = filled;
+    for (bool first = true; (uint64_t)t < ready; ++t, first = false) {
+      p1 *= beta1;
+      p2 *= beta2;
+      MLP_CHECK(launch_step(d.stream, !first, dw, dx, dl, dt, didx + (size_t)t * batch, batch, dg, dloss + t, ddone,
+                            AdamStep{dw, dm, dv, lr, beta1, beta2, eps, (float)(1.0 - p1), (float)(1.0 - p2)}));
+    }
   }
   MLP_CHECK(cudaStreamSynchronize(d.stream));
   MLP_CHECK(cudaMemcpy(weights_inout, dw, sizeof(float) * VELO_MLP_PARAMS, cudaMemcpyDeviceToHost));

@@ -482,6 +482,6 @@ def mlp_grad(weights: np.ndarray, x: np.ndarray, label: np.ndarray, target: np.n
 def mlp_forward(weights: np.ndarray, x: np.ndarray) -> np.ndarray:
     w = np.ascontiguousarray(weights, np.float32)
     x = np.ascontiguousarray(x, np.float32)
-    out = np.zeros((len(x), 2), np.float32)
+    out = np.empty((len(x), 2), np.float32)   # the call fills it
     _check_free(load().velo_mlp_forward(_p(w), _p(x), len(x), _p(out)), "velo_mlp_forward")
     return out

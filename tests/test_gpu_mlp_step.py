@@ -98,3 +98,20 @@ def test_steps(native_lib, n, batch, steps):
     off = np.abs(got - w)
     assert off.max() <= 4 * lr * steps
     assert np.mean(off > 1e-2 * lr * steps) < 0.01
+
+
+@pytest.mark.parametrize("n, batch, steps", [(2, 3, 50), (3, 1, 40), (257, 256, 30), (5000, 8192, 135)])
+def test_sample_order(native_lib, n, batch, steps):
+    """With a learning rate of 0 each step's loss is that of its samples under
+    the initial weights: every sample of every epoch shows, also where the
+    draws are made in several launches (the last case: over 2^20 of them)."""
+    from cl_forward_gb300 import learned, native
+    x, y, t = _data(n, n)
+    w = learned.init_weights(9)
+    got, losses = native.mlp_train(x, y, t, w, steps, batch, 0.0, 123)
+    assert np.array_equal(got, w)
+    o = learned.forward_np(w, x)
+    z, wd = o[:, 0], o[:, 1]
+    per_sample = np.maximum(z, 0) - z * y + np.log1p(np.exp(-np.abs(z))) + y * learned.WIDTH_WEIGHT * (wd - t) ** 2
+    want = per_sample[_order(n, steps * batch, 123)].reshape(steps, batch).mean(1)
+    assert np.all(np.abs(losses - want) <= ROUNDINGS * (1 + np.abs(want)))
