@@ -695,25 +695,28 @@ velo_status check_options(velo_ctx* c, const velo_options* opts, velo_options* o
 // The launch that automatic options stand for, on the staged batch.  A
 // persistent launch of 64-thread CTAs is the fastest for large batches, but
 // it leaves a small one waiting for its largest event: with the automatic
-// register build, CTAs are widened while the batch takes few rounds of them.
-// Milliseconds with 64 / 128 / 256 / 512 threads (events of 1,160 hits; of
-// 4,550 hits):
-//     100 events  0.41  0.30  0.25  0.25    2.7  1.5  1.0  0.8
-//   1,003         0.85  0.60  0.45  1.08    4.8  2.9  1.9  3.3
-//   2,500         0.96  0.70  0.94  2.6     6.0  3.4  3.5  8.1
-//   4,000         1.04  0.97  1.44  4.2     5.9  4.0  4.9  12.8
-//   7,000         1.23  1.61  2.49  7.2
-// Resident CTAs per SM: 16, 8, 4 and 1 (learned: 12, 6 and 3).
+// register build, CTAs are widened while the batch takes few rounds of them;
+// events of thousands of hits keep four warps busy for longer.
+// Milliseconds with 64 / 128 / 256 threads, by mean hits:
+//               310 hits           1,160              4,550
+//   1,003   0.25  0.23  0.23   0.67  0.53  0.41   4.0  2.6  1.6
+//   1,216   0.27  0.25  0.25   0.70  0.54  0.46   3.9  2.5  1.6
+//   2,000   0.31  0.27  0.38   0.79  0.56  0.76   4.1  2.6  2.4
+//   3,000   0.33  0.38  0.57   0.82  0.72  1.07   4.9  3.1  3.5
+//   4,000   0.35  0.46  0.74   0.86  0.94  1.40   4.9  3.6  4.5
+//   6,000   0.47  0.68  1.09   1.00  1.35  2.08   5.4  5.2  6.7
+// (2,440 hits cross where 1,160 do.)  512 threads, one CTA per SM, take up to
+// one event per SM: 100 events of 1,160 hits 0.25 ms, 0.27 with 256 threads.
 void resolve_launch(const velo_ctx* c, velo_options* o) {
-  const bool learned = o->learned != 0;
   if (o->register_ctas == 0 && o->threads_per_event == 64 && o->launch_mode == VELO_LAUNCH_PERSISTENT &&
-      o->ctas_per_sm <= 0 && !c->dump_armed) {
+      o->ctas_per_sm <= 0 && !c->dump_armed && c->n > 0) {
     const int64_t n = c->n, sms = c->sm_count;
-    if (n <= sms && !learned)
+    const bool large = c->total_hits / (uint64_t)n >= 3000;
+    if (n <= sms && !o->learned)   // no learned build of 512
       o->threads_per_event = 512;
-    else if (n <= (learned ? 6 : 8) * sms)
+    else if (n <= 8 * sms)
       o->threads_per_event = 256;
-    else if (n <= (learned ? 18 : 24) * sms)
+    else if (n <= (large ? 36 : 20) * sms)
       o->threads_per_event = 128;
   }
   if (o->register_ctas == 0) o->register_ctas = o->threads_per_event > 256 ? 5 : 4;

@@ -69,14 +69,13 @@ constexpr uint8_t kSorted = 1, kDeadTail = 2;
 
 // Seeding state per CTA: each warp's lists, and per module parity the
 // occupancy map of the h2 module.  kOwn: the h0s a warp seeds at once.
-constexpr int kMapRows = 64;          // 64 rows x 32 columns of cells
 constexpr int kQueue = 32;            // pairs a warp holds for the exact fits
-template <int kWarps, int kOwn, int kList>
+template <int kWarps, int kOwn, int kList, int kMapRows>
 struct SeedShared {
   float4 h0[kWarps][kOwn];            // x, y, z, first h1's place - first pair (int bits)
   float2 reach[kWarps][kOwn];         // the h0's y cut, and in plain geometry (z2 - z0) / (z1 - z0)
   unsigned long long best[kWarps][kOwn];   // the h0's best (fit, Y-lane, h1, h2) so far
-  uint32_t map[2][kMapRows];
+  alignas(16) uint32_t map[2][kMapRows];   // rows of 32 cells
   std::conditional_t<(kOwn > 4), uint32_t, uint16_t> queue[kWarps][kQueue];   // h0 << 14 | h1 in its module
   uint16_t first[kWarps][kOwn];       // the h0's first h1 in its module
   // by parity: the usable h1s (unused, with an h2 window) of a module of up to
@@ -97,7 +96,8 @@ struct SharedT {
   static constexpr int kOwn = kWarps <= 2 ? 16 : kMods <= kCompactModules ? 64 / kWarps : 16 / kWarps + (kWarps <= 8) * 2;
   static constexpr int kMaxWarps = kWarps;
   static constexpr int kList = kMods <= kCompactModules ? 256 : 64;
-  SeedShared<kWarps, kOwn, kList> seed;
+  static constexpr int kMapRows = kMods <= kCompactModules ? 256 : 64;
+  SeedShared<kWarps, kOwn, kList, kMapRows> seed;
   int32_t start[kMods];       // [S] = H
   int32_t sz[kMods];
   float zmin[kMods];
@@ -952,9 +952,19 @@ __device__ __noinline__ void fill_windows(const EventView ev, const Shared& s) {
 // The windows need no table.  An h0's h1 window is bisected when the h0 is
 // seeded (most hits never are); whether an h1 has an h2 window is the flag
 // kDead; the h2 window itself is only tested on an h2 that passed the cuts.
-constexpr float kCellInv = 1.f / 1.3125f;   // cells of 1.3 mm: 32 columns span half a module's width, 64 rows its height
+// 32 columns of 1.3 mm span half a module's width, the rows its height.  With
+// 256 rows instead of 64 half as many pairs pass that no hit is near (of 54,000
+// pairs in an event of 4,400 hits 2,850 instead of 6,000, 800 of them met).
+__device__ __forceinline__ int map_column(float x) { return __float2int_rd(fmul(x, 1.f / 1.3125f)); }
+template <class Shared>
+__device__ __forceinline__ int map_row(float y) {
+  return __float2int_rd(fmul(y, (float)Shared::kMapRows / 84.f));
+}
 
-__device__ __forceinline__ int map_cell(float v) { return __float2int_rd(fmul(v, kCellInv)); }
+template <class Shared>
+__device__ __forceinline__ bool map_marked(const uint32_t* map, float x, float y) {
+  return (map[map_row<Shared>(y) & (Shared::kMapRows - 1)] >> (map_column(x) & 31)) & 1u;
+}
 
 // Marks the cells from which hit i of module m4 could be met: a pair whose
 // fit passes lies within 0.004 |z2 - z1| of it, and within kTolerance.  A
@@ -967,8 +977,9 @@ __device__ __forceinline__ void mark_map(const EventView& ev, const Shared& s, u
   const float reach = fadd(fminf(kTolerance, fmul(kScatterReach, dz)), 0.01f);
   const float x = ev.xs()[s.start[m4] + i], y = ev.ys()[s.start[m4] + i];
   uint32_t bits = 0;
-  for (int c = map_cell(fsub(x, reach)); c <= map_cell(fadd(x, reach)); ++c) bits |= 1u << (c & 31);
-  for (int r = map_cell(fsub(y, reach)); r <= map_cell(fadd(y, reach)); ++r) atomicOr(&map[r & (kMapRows - 1)], bits);
+  const int c_end = map_column(fadd(x, reach)), r_end = map_row<Shared>(fadd(y, reach));
+  for (int c = map_column(fsub(x, reach)); c <= c_end; ++c) bits |= 1u << (c & 31);
+  for (int r = map_row<Shared>(fsub(y, reach)); r <= r_end; ++r) atomicOr(&map[r & (Shared::kMapRows - 1)], bits);
 }
 
 // The bounds of an h1's h2 window (Kernel.cl:85-102) for h1 at (x, z) on
@@ -1165,11 +1176,11 @@ __device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Worke
     // the pairs of the warp's h0s, end to end
     int end = count;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
+    for (int o = 1; o < kOwn; o <<= 1) {
       const int v = __shfl_up_sync(kFull, end, o);
       if (lane >= o) end += v;
     }
-    const int total = __shfl_sync(kFull, end, 31);
+    const int total = __shfl_sync(kFull, end, kOwn - 1);
     if (total == 0) continue;
     const int begin = end - count;
     const unsigned om = __ballot_sync(kFull, count > 0);
@@ -1206,7 +1217,7 @@ __device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Worke
           if (kPlainGeometry && kMode == kPlain && pass) {   // the fit's own predicted point
             const float px = fadd(q.x, fmul(fsub(h1x, q.x), r.y));
             const float py = fadd(q.y, fmul(fsub(h1y, q.y), r.y));
-            pass = (map[map_cell(py) & (kMapRows - 1)] >> (map_cell(px) & 31)) & 1u;
+            pass = map_marked<Shared>(map, px, py);
           }
         }
       }
@@ -1273,7 +1284,7 @@ __device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Worke
                 lt = fmaxf(lt, l);
                 ht = fminf(ht, h);
               }
-              if (!((map[map_cell(py) & (kMapRows - 1)] >> (map_cell(px) & 31)) & 1u)) b = a;   // no hit in reach
+              if (!map_marked<Shared>(map, px, py)) b = a;   // no hit in reach
             }
             for (int k = first_gt(x4, a, b, lt); k < b; ++k) {
               const float h2x = x4[k];
@@ -1490,24 +1501,21 @@ __device__ __forceinline__ Worker module_loop(const EventView& ev, Shared& s, Wo
     const int step = (S - 1 - f) & 1;
     if (w.alone() || step == w.parity()) {
       const bool by_pairs = kPlainGeometry || (kMode == kPlain && ev.tame);
-      uint32_t* map = s.seed.map[w.parity()];
       const int gt = w.idx() * 32 + lane, gn = w.of() * 32;
-      if (kPlainGeometry)
-        for (int i = gt; i < kMapRows; i += gn) map[i] = 0;
+      if (kPlainGeometry) {
+        uint4* map = reinterpret_cast<uint4*>(s.seed.map[w.parity()]);
+        for (int i = gt; i < Shared::kMapRows / 4; i += gn) map[i] = make_uint4(0, 0, 0, 0);
+      }
       group_sync<Shared::kMaxWarps>(w);
       if (by_pairs) {
         if (w.idx() == 0) list_h1s(ev, s, w, f - 2);
         if (kPlainGeometry)   // from the group's last warp on
-          for (int i = gn - 1 - gt; i < s.num(f - 4); i += gn) mark_map(ev, s, map, f - 2, f - 4, i);
+          for (int i = gn - 1 - gt; i < s.num(f - 4); i += gn)
+            mark_map(ev, s, s.seed.map[w.parity()], f - 2, f - 4, i);
         group_sync<Shared::kMaxWarps>(w);
-      }
-      if constexpr (kPlainGeometry) {
-        seed_pairs<kMode, true>(ev, s, w, f);
-      } else {
-        if (by_pairs)
-          seed_pairs<kPlain, false>(ev, s, w, f);
-        else
-          seed_module<kMode, kLanes>(ev, s, w, f, seed_lanes_of(kLanes, (uint32_t)ev.y_lanes));
+        seed_pairs<kPlainGeometry ? kMode : kPlain, kPlainGeometry>(ev, s, w, f);
+      } else if constexpr (!kPlainGeometry) {
+        seed_module<kMode, kLanes>(ev, s, w, f, seed_lanes_of(kLanes, (uint32_t)ev.y_lanes));
       }
       group_sync<Shared::kMaxWarps>(w);
     }
@@ -1828,7 +1836,8 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
 // warps), 64-thread CTAs with 56 registers (18 CTAs per SM, register_ctas 18),
 // and 512-thread CTAs; the learned mode in a build of up to
 // 256 threads with 80 registers (3 resident CTAs; 2.76 against 3.28 ms with 64
-// for 5,000 events with the scorer out of line, 2.02 ms with it inlined); each for one seeding
+// for 5,000 events with the scorer out of line, 2.02 ms with it inlined) and
+// one of up to 64 threads (1.92 ms); each for one seeding
 // width kLanes (lanes per h0 where the windows are walked).
 template <int kMaxThreads, int kMinCtas, int kMode, int kMods, int kLanes>
 __global__ void __launch_bounds__(kMaxThreads, kMinCtas) search_kernel(const __grid_constant__ SearchParams p) {
@@ -1867,7 +1876,9 @@ template <int G>
 struct SearchBuilds {
   static int launch(const SearchParams& p, int grid, int block, uint32_t smem, cudaStream_t st, int reg_ctas,
                     bool compact) {
-    if (p.mlp && compact)
+    if (p.mlp && compact && block <= 64)
+      search_kernel<64, 12, kLearned, kCompactModules, G><<<grid, block, smem, st>>>(p);
+    else if (p.mlp && compact)
       search_kernel<256, 3, kLearned, kCompactModules, G><<<grid, min(block, 256), smem, st>>>(p);
     else if (p.mlp)
       search_kernel<256, 3, kLearned, kFullModules, G><<<grid, min(block, 256), smem, st>>>(p);
@@ -1909,12 +1920,16 @@ struct SearchBuilds {
     VELO_LIMIT(search_kernel<512, 1, kPlain, kFullModules, G>);
     VELO_LIMIT(search_kernel<256, 3, kLearned, kFullModules, G>);
     VELO_LIMIT(search_kernel<256, 3, kLearned, kCompactModules, G>);
+    VELO_LIMIT(search_kernel<64, 12, kLearned, kCompactModules, G>);
     if (G == 32) VELO_LIMIT(search_kernel<256, 4, kDump, kFullModules, 32>);
 #undef VELO_LIMIT
     return (int)e;
   }
 
   static int occupancy(int block, uint32_t smem, int reg_ctas, int mode, bool compact, int* ctas) {
+    if (mode == kModeLearned && compact && block <= 64)
+      return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+          ctas, search_kernel<64, 12, kLearned, kCompactModules, G>, block, smem);
     if (mode == kModeLearned)
       return compact ? (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                            ctas, search_kernel<256, 3, kLearned, kCompactModules, G>, min(block, 256), smem)
