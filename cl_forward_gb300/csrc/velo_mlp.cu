@@ -27,10 +27,10 @@ namespace velo {
 
 constexpr float kWidthWeight = 0.1f;
 constexpr int kTile = 32;             // samples of a CTA's pass: one per lane
-constexpr int kTrainWarps = 8;        // each warp owns 4 of the 32 units of a layer
+constexpr int kTrainWarps = 16;       // each warp owns 2 of the 32 units of a layer
 constexpr int kTrainThreads = 32 * kTrainWarps;
 constexpr int kUnits = kMlpHidden / kTrainWarps;
-static_assert(kUnits == 4 && kMlpOut == 2, "the tile below is laid out for 8 x 4 units and 2 outputs");
+static_assert(kUnits == 2 && kMlpOut == 2, "the tile below is laid out for 16 x 2 units and 2 outputs");
 // a unit's row over the tile's samples: 36 floats apart, so that 8 lanes
 // reading 16 bytes of 8 rows meet no bank twice
 constexpr int kRow = kTile + 4;
@@ -60,46 +60,46 @@ struct AdamStep {
   float lr, beta1, beta2, eps, c1, c2;
 };
 
+// Floats between two CTAs' rows of partial sums: the gradient, then the loss.
+constexpr int kPartialRow = (VELO_MLP_PARAMS + 1 + 31) & ~31;
+
 __device__ __forceinline__ float lane_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
-// Gradient of the mean loss over n samples (through `index` when given) and,
-// with adam.w, the Adam update: one launch per training step.
+// Gradient of the mean loss over n samples (through `index` when given): each
+// CTA's share of it, row blockIdx.x of `partial`.
 //
 // A CTA passes over tiles of 32 samples, one per lane; warp k computes units
-// 4k..4k+3 of each layer, weights broadcast from shared memory, activations
+// 2k and 2k+1 of each layer, weights broadcast from shared memory, activations
 // exchanged through it by unit and sample.  Bias and output-layer gradients
 // are summed per lane and reduced once at the end; the two weight matrices
 // are products over the tile's samples, each thread holding the same outputs
-// for every tile.  A CTA adds its sums to the global gradient once, and the
-// last CTA to do so updates the parameters and clears the gradient for the
-// next launch.
+// for every tile.
 //
 // The step's floor is 3,904 multiply-adds a sample, 0.2 us for a batch of
-// 4,096 on the whole chip; what bounds it is the chain of launch, gather, five
-// exchanges, reduction and update.  The kernel before it (a thread per sample,
-// every product added by a shared-memory atomic that all lanes of a warp aimed
-// at one address, a memset and a separate Adam kernel) took 1.47 ms a step.
+// 4,096 on the whole chip; what bounds it is the chain of launches, gather, five
+// exchanges and reduction.  A thread per sample with every product added by a
+// shared-memory atomic, which all lanes of a warp aimed at one address, took
+// 1.47 ms a step; this tile with its sums added to the gradient by atomics and
+// the update in the last CTA 20.8 us (128 CTAs waiting on their atomics and a
+// counter); rows of partial sums and a second kernel 10.7 us.
 __global__ void __launch_bounds__(kTrainThreads) mlp_step_kernel(const float* w,
                                                                  const float* __restrict__ x,
                                                                  const float* __restrict__ label,
                                                                  const float* __restrict__ target,
                                                                  const int64_t* __restrict__ index, int64_t n,
-                                                                 float scale, float* grad, float* loss_sum,
-                                                                 unsigned int* done, AdamStep adam) {
+                                                                 float scale, float* __restrict__ partial) {
   __shared__ __align__(16) GradTile t;
-  __shared__ bool last;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, u0 = kUnits * warp;
-  const int j2 = tid >> 3, i2 = tid & 7;   // this thread's outputs of W2's gradient: row j2, columns i2 + 8 q
-  float gw2[4] = {}, gw1[2] = {}, gw3[kMlpOut][kUnits] = {}, gb1[kUnits] = {}, gb2[kUnits] = {}, gb3[kMlpOut] = {};
+  const int j2 = tid >> 4, i2 = tid & 15;   // this thread's outputs of W2's gradient: row j2, columns i2 + 16 q
+  float gw2[2] = {}, gw1 = 0.f, gw3[kMlpOut][kUnits] = {}, gb1[kUnits] = {}, gb2[kUnits] = {}, gb3[kMlpOut] = {};
   float loss = 0.f;
 
   // the samples do not depend on the launch before this one, the weights do
   const int64_t tiles = (n + kTile - 1) / kTile;
-  cudaTriggerProgrammaticLaunchCompletion();
   for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int64_t base = tile * kTile;
     if (tile != blockIdx.x) __syncthreads();   // the tile before has been read
@@ -127,6 +127,7 @@ __global__ void __launch_bounds__(kTrainThreads) mlp_step_kernel(const float* w,
 #pragma unroll
       for (int u = 0; u < kUnits; ++u) a1[u] = __fmaf_rn(t.w[kMlpW1 + (u0 + u) * kMlpIn + i], v, a1[u]);
     }
+    if (tile == blockIdx.x) cudaTriggerProgrammaticLaunchCompletion();   // the reduction may be set up
 #pragma unroll
     for (int u = 0; u < kUnits; ++u) {
       a1[u] = a1[u] > 0.f ? a1[u] : 0.f;
@@ -193,11 +194,9 @@ __global__ void __launch_bounds__(kTrainThreads) mlp_step_kernel(const float* w,
 #pragma unroll 8
     for (int j = 0; j < kMlpHidden; ++j) {
       const float v = t.d2[j][lane];
-      const float4 c = *reinterpret_cast<const float4*>(&t.w[kMlpW2 + j * kMlpHidden + u0]);
+      const float2 c = *reinterpret_cast<const float2*>(&t.w[kMlpW2 + j * kMlpHidden + u0]);
       d1[0] = __fmaf_rn(c.x, v, d1[0]);
       d1[1] = __fmaf_rn(c.y, v, d1[1]);
-      d1[2] = __fmaf_rn(c.z, v, d1[2]);
-      d1[3] = __fmaf_rn(c.w, v, d1[3]);
     }
 #pragma unroll
     for (int u = 0; u < kUnits; ++u) {
@@ -210,74 +209,84 @@ __global__ void __launch_bounds__(kTrainThreads) mlp_step_kernel(const float* w,
     for (int k = 0; k < kTile; k += 4) {
       const float4 d = *reinterpret_cast<const float4*>(&t.d2[j2][k]);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float4 a = *reinterpret_cast<const float4*>(&t.a1[i2 + 8 * q][k]);
+      for (int q = 0; q < 2; ++q) {
+        const float4 a = *reinterpret_cast<const float4*>(&t.a1[i2 + 16 * q][k]);
         gw2[q] = __fmaf_rn(d.w, a.w, __fmaf_rn(d.z, a.z, __fmaf_rn(d.y, a.y, __fmaf_rn(d.x, a.x, gw2[q]))));
       }
     }
     __syncthreads();
     // W1's gradient: 320 outputs, d1[j] x[i]
+    if (tid < kMlpHidden * kMlpIn) {
+      const float* d = t.d1[tid / kMlpIn];
+      const float* v = t.x[tid % kMlpIn];
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int o = tid + q * kTrainThreads;
-      if (o < kMlpHidden * kMlpIn) {
-        const float* d = t.d1[o / kMlpIn];
-        const float* v = t.x[o % kMlpIn];
-#pragma unroll
-        for (int k = 0; k < kTile; k += 4) {
-          const float4 a = *reinterpret_cast<const float4*>(&d[k]), b = *reinterpret_cast<const float4*>(&v[k]);
-          gw1[q] = __fmaf_rn(a.w, b.w, __fmaf_rn(a.z, b.z, __fmaf_rn(a.y, b.y, __fmaf_rn(a.x, b.x, gw1[q]))));
-        }
+      for (int k = 0; k < kTile; k += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(&d[k]), b = *reinterpret_cast<const float4*>(&v[k]);
+        gw1 = __fmaf_rn(a.w, b.w, __fmaf_rn(a.z, b.z, __fmaf_rn(a.y, b.y, __fmaf_rn(a.x, b.x, gw1))));
       }
     }
   }
 
-  // one addition per CTA and parameter
+  float* row = partial + (size_t)blockIdx.x * kPartialRow;
 #pragma unroll
-  for (int q = 0; q < 4; ++q) atomicAdd(&grad[kMlpW2 + j2 * kMlpHidden + i2 + 8 * q], gw2[q]);
-#pragma unroll
-  for (int q = 0; q < 2; ++q)
-    if (tid + q * kTrainThreads < kMlpHidden * kMlpIn) atomicAdd(&grad[kMlpW1 + tid + q * kTrainThreads], gw1[q]);
-  float mine = 0.f;   // lanes 0-3: b1, 4-7: b2, 8-11 and 12-15: W3's rows, 16 and 17: b3, 18: the loss
+  for (int q = 0; q < 2; ++q) row[kMlpW2 + j2 * kMlpHidden + i2 + 16 * q] = gw2[q];
+  if (tid < kMlpHidden * kMlpIn) row[kMlpW1 + tid] = gw1;
+  float mine = 0.f;   // lanes 0, 1: b1; 2, 3: b2; 4, 5 and 6, 7: W3's rows; 8, 9: b3; 10: the loss
 #pragma unroll
   for (int u = 0; u < kUnits; ++u) {
     const float v1 = lane_sum(gb1[u]), v2 = lane_sum(gb2[u]), v3 = lane_sum(gw3[0][u]), v4 = lane_sum(gw3[1][u]);
     if (lane == u) mine = v1;
-    if (lane == 4 + u) mine = v2;
-    if (lane == 8 + u) mine = v3;
-    if (lane == 12 + u) mine = v4;
+    if (lane == 2 + u) mine = v2;
+    if (lane == 4 + u) mine = v3;
+    if (lane == 6 + u) mine = v4;
   }
   const float vb0 = lane_sum(gb3[0]), vb1 = lane_sum(gb3[1]), vl = lane_sum(loss);
-  if (lane == 16) mine = vb0;
-  if (lane == 17) mine = vb1;
-  if (lane == 18) mine = vl;
-  const int u = lane & 3;
-  float* to = lane < 4    ? grad + kMlpB1 + u0 + u
-              : lane < 8  ? grad + kMlpB2 + u0 + u
-              : lane < 12 ? grad + kMlpW3 + u0 + u
-              : lane < 16 ? grad + kMlpW3 + kMlpHidden + u0 + u
-              : lane < 18 ? grad + kMlpB3 + (lane - 16)
-                          : loss_sum;
-  // every warp has the outputs' sums: warp 0 adds them
-  if (lane < 16 || (warp == 0 && lane < 19 && to)) atomicAdd(to, mine);
+  if (lane == 8) mine = vb0;
+  if (lane == 9) mine = vb1;
+  if (lane == 10) mine = vl;
+  const int u = lane & 1;
+  const int to = lane < 2   ? kMlpB1 + u0 + u
+                 : lane < 4 ? kMlpB2 + u0 + u
+                 : lane < 6 ? kMlpW3 + u0 + u
+                 : lane < 8 ? kMlpW3 + kMlpHidden + u0 + u
+                            : kMlpB3 + lane - 8;   // the loss after the parameters
+  // every warp has the outputs' sums: warp 0 writes them
+  if (lane < 8 || (warp == 0 && lane < 11)) row[to] = mine;
+}
+static_assert(kMlpB3 + 2 == VELO_MLP_PARAMS, "the loss follows the output biases");
 
-  if (!adam.w) return;
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  for (int i = tid; i < VELO_MLP_PARAMS; i += kTrainThreads) {
-    const float gi = __ldcg(grad + i);
-    const float mi = adam.beta1 * __ldcg(adam.m + i) + (1.f - adam.beta1) * gi;
-    const float vi = adam.beta2 * __ldcg(adam.v + i) + (1.f - adam.beta2) * gi * gi;
-    adam.m[i] = mi;
-    adam.v[i] = vi;
-    adam.w[i] = __ldcg(adam.w + i) - adam.lr * (mi / adam.c1) / (sqrtf(vi / adam.c2) + adam.eps);
-    grad[i] = 0.f;
+// Sums the rows of `partial`, in a fixed order: the gradient (to `grad` when
+// given) and the mean loss, and with adam.w the Adam update.  32 parameters
+// per CTA, 8 rows at a time.
+__global__ void __launch_bounds__(256) mlp_reduce_kernel(const float* __restrict__ partial, int rows, float* grad,
+                                                         float* loss, AdamStep adam) {
+  __shared__ float sums[8][32];
+  const int lane = threadIdx.x & 31, group = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();   // the next step may gather its samples
+  float v = 0.f;
+  if (i <= VELO_MLP_PARAMS) {
+#pragma unroll 4
+    for (int r = group; r < rows; r += 8) v += __ldcg(partial + (size_t)r * kPartialRow + i);
   }
-  if (tid == 0) *done = 0u;
+  sums[group][lane] = v;
+  __syncthreads();
+  if (group != 0 || i > VELO_MLP_PARAMS) return;
+  float gi = 0.f;
+#pragma unroll
+  for (int g = 0; g < 8; ++g) gi += sums[g][lane];
+  if (i == VELO_MLP_PARAMS) {
+    if (loss) *loss = gi;
+    return;
+  }
+  if (grad) grad[i] = gi;
+  if (!adam.w) return;
+  const float mi = adam.beta1 * __ldcg(adam.m + i) + (1.f - adam.beta1) * gi;
+  const float vi = adam.beta2 * __ldcg(adam.v + i) + (1.f - adam.beta2) * gi * gi;
+  adam.m[i] = mi;
+  adam.v[i] = vi;
+  adam.w[i] = __ldcg(adam.w + i) - adam.lr * (mi / adam.c1) / (sqrtf(vi / adam.c2) + adam.eps);
 }
 
 // Inference as the learned seeding does it (FP16 tensor-core MMA, one warp
@@ -332,28 +341,38 @@ struct DevArrays {
     if (e_ != cudaSuccess) return VELO_ERR_CUDA; \
   } while (0)
 
-// One CTA per tile of 32 samples while the chip has room, at most two per SM:
-// a CTA's sums go to the global gradient once, whatever its tiles.  With
-// `follows`, the launch may start while the step before it finishes.
-cudaError_t launch_step(cudaStream_t stream, bool follows, const float* w, const float* x, const float* label,
-                        const float* target, const int64_t* index, int64_t n, float* grad, float* loss,
-                        unsigned int* done, AdamStep adam) {
+// CTAs (rows of partial sums) of a step over n samples: one per tile of 32
+// while the chip has room, at most two per SM.
+cudaError_t step_rows(int64_t n, int* rows) {
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess) return e;
   const int64_t tiles = (n + kTile - 1) / kTile;
+  *rows = (int)(tiles < 2 * sms ? tiles : 2 * sms);
+  return e;
+}
+
+// One step: partial gradients, then their sum and the update.  Each kernel may
+// be set up while the one before it finishes; `follows`: so may the first.
+cudaError_t launch_step(cudaStream_t stream, bool follows, const float* w, const float* x, const float* label,
+                        const float* target, const int64_t* index, int64_t n, float* partial, int rows, float* grad,
+                        float* loss, AdamStep adam) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t c{};
-  c.gridDim = dim3((unsigned)(tiles < 2 * sms ? tiles : 2 * sms));
+  c.gridDim = dim3((unsigned)rows);
   c.blockDim = dim3(kTrainThreads);
   c.stream = stream;
   c.attrs = &attr;
   c.numAttrs = follows ? 1 : 0;
-  return cudaLaunchKernelEx(&c, mlp_step_kernel, w, x, label, target, index, n, 1.f / (float)n, grad, loss, done,
-                            adam);
+  cudaError_t e =
+      cudaLaunchKernelEx(&c, mlp_step_kernel, w, x, label, target, index, n, 1.f / (float)n, partial);
+  if (e != cudaSuccess) return e;
+  c.gridDim = dim3((VELO_MLP_PARAMS + 1 + 31) / 32);
+  c.blockDim = dim3(256);
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, mlp_reduce_kernel, (const float*)partial, rows, grad, loss, adam);
 }
 
 // splitmix64: the k-th value (k from 1) of the sequence that starts at `seed`.
@@ -390,16 +409,19 @@ extern "C" velo_status velo_mlp_grad(const float* weights, const float* x, const
   const size_t ow = d.reserve<float>(VELO_MLP_PARAMS), ox = d.reserve<float>((size_t)n * kMlpIn),
                ol = d.reserve<float>((size_t)n), ot = d.reserve<float>((size_t)n),
                og = d.reserve<float>(VELO_MLP_PARAMS), oloss = d.reserve<float>(1);
+  int rows = 0;
+  MLP_CHECK(step_rows(n, &rows));
+  const size_t op = d.reserve<float>((size_t)rows * kPartialRow);
   MLP_CHECK(d.allocate());
   float *dw = d.at<float>(ow), *dx = d.at<float>(ox), *dl = d.at<float>(ol), *dt = d.at<float>(ot),
         *dg = d.at<float>(og), *dloss = d.at<float>(oloss);
-  MLP_CHECK(cudaMemcpy(dw, weights, sizeof(float) * VELO_MLP_PARAMS, cudaMemcpyHostToDevice));
-  MLP_CHECK(cudaMemcpy(dx, x, sizeof(float) * n * kMlpIn, cudaMemcpyHostToDevice));
-  MLP_CHECK(cudaMemcpy(dl, label, sizeof(float) * n, cudaMemcpyHostToDevice));
-  MLP_CHECK(cudaMemcpy(dt, target, sizeof(float) * n, cudaMemcpyHostToDevice));
-  MLP_CHECK(cudaMemset(dg, 0, sizeof(float) * VELO_MLP_PARAMS));
-  MLP_CHECK(cudaMemset(dloss, 0, sizeof(float)));
-  MLP_CHECK(launch_step(nullptr, false, dw, dx, dl, dt, nullptr, n, dg, dloss, nullptr, AdamStep{}));
+  MLP_CHECK(cudaStreamCreateWithFlags(&d.stream, cudaStreamNonBlocking));
+  MLP_CHECK(cudaMemcpyAsync(dw, weights, sizeof(float) * VELO_MLP_PARAMS, cudaMemcpyHostToDevice, d.stream));
+  MLP_CHECK(cudaMemcpyAsync(dx, x, sizeof(float) * n * kMlpIn, cudaMemcpyHostToDevice, d.stream));
+  MLP_CHECK(cudaMemcpyAsync(dl, label, sizeof(float) * n, cudaMemcpyHostToDevice, d.stream));
+  MLP_CHECK(cudaMemcpyAsync(dt, target, sizeof(float) * n, cudaMemcpyHostToDevice, d.stream));
+  MLP_CHECK(launch_step(d.stream, false, dw, dx, dl, dt, nullptr, n, d.at<float>(op), rows, dg, dloss, AdamStep{}));
+  MLP_CHECK(cudaStreamSynchronize(d.stream));
   MLP_CHECK(cudaMemcpy(grad_out, dg, sizeof(float) * VELO_MLP_PARAMS, cudaMemcpyDeviceToHost));
   if (loss_out) MLP_CHECK(cudaMemcpy(loss_out, dloss, sizeof(float), cudaMemcpyDeviceToHost));
   return VELO_OK;
@@ -435,25 +457,25 @@ extern "C" velo_status velo_mlp_train(const float* x, const float* label, const 
   const uint64_t epochs = (places + (uint64_t)n - 1) / (uint64_t)n;
   const uint64_t epochs_at_once =
       device_draws ? std::min(epochs, std::max<uint64_t>(1, kDrawsAtOnce / swaps)) : 1;
+  int rows = 0;
+  MLP_CHECK(step_rows(batch, &rows));
   const size_t ow = d.reserve<float>(VELO_MLP_PARAMS), ox = d.reserve<float>((size_t)n * kMlpIn),
                ol = d.reserve<float>((size_t)n), ot = d.reserve<float>((size_t)n),
-               og = d.reserve<float>(VELO_MLP_PARAMS), om = d.reserve<float>(VELO_MLP_PARAMS),
+               op = d.reserve<float>((size_t)rows * kPartialRow), om = d.reserve<float>(VELO_MLP_PARAMS),
                ov = d.reserve<float>(VELO_MLP_PARAMS), oloss = d.reserve<float>((size_t)steps),
-               odone = d.reserve<unsigned int>(1), oi = d.reserve<int64_t>((size_t)places),
+               oi = d.reserve<int64_t>((size_t)places),
                od = d.reserve<uint32_t>(device_draws ? (size_t)(epochs_at_once * swaps) : 1);
   MLP_CHECK(d.allocate());
   float *dw = d.at<float>(ow), *dx = d.at<float>(ox), *dl = d.at<float>(ol), *dt = d.at<float>(ot),
-        *dg = d.at<float>(og), *dm = d.at<float>(om), *dv = d.at<float>(ov), *dloss = d.at<float>(oloss);
+        *dp = d.at<float>(op), *dm = d.at<float>(om), *dv = d.at<float>(ov), *dloss = d.at<float>(oloss);
   int64_t* didx = d.at<int64_t>(oi);
-  unsigned int* ddone = d.at<unsigned int>(odone);
   MLP_CHECK(cudaStreamCreateWithFlags(&d.stream, cudaStreamNonBlocking));
   MLP_CHECK(cudaStreamCreateWithFlags(&d.aux, cudaStreamNonBlocking));
   MLP_CHECK(cudaMemcpyAsync(dw, weights_inout, sizeof(float) * VELO_MLP_PARAMS, cudaMemcpyHostToDevice, d.stream));
   MLP_CHECK(cudaMemcpyAsync(dx, x, sizeof(float) * n * kMlpIn, cudaMemcpyHostToDevice, d.stream));
   MLP_CHECK(cudaMemcpyAsync(dl, label, sizeof(float) * n, cudaMemcpyHostToDevice, d.stream));
   MLP_CHECK(cudaMemcpyAsync(dt, target, sizeof(float) * n, cudaMemcpyHostToDevice, d.stream));
-  // gradient, moments (adjacent), losses and the counter start at zero
-  MLP_CHECK(cudaMemsetAsync(dg, 0, oi - og, d.stream));
+  MLP_CHECK(cudaMemsetAsync(dm, 0, oloss - om, d.stream));   // both moments
   for (int64_t i = 0; i < n; ++i) order[(size_t)i] = i;
   const float beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
   double p1 = 1.0, p2 = 1.0;
@@ -490,7 +512,7 @@ extern "C" velo_status velo_mlp_train(const float* x, const float* label, const 
     for (bool first = true; (uint64_t)t < ready; ++t, first = false) {
       p1 *= beta1;
       p2 *= beta2;
-      MLP_CHECK(launch_step(d.stream, !first, dw, dx, dl, dt, didx + (size_t)t * batch, batch, dg, dloss + t, ddone,
+      MLP_CHECK(launch_step(d.stream, !first, dw, dx, dl, dt, didx + (size_t)t * batch, batch, dp, rows, nullptr, dloss + t,
                             AdamStep{dw, dm, dv, lr, beta1, beta2, eps, (float)(1.0 - p1), (float)(1.0 - p2)}));
     }
   }
