@@ -555,6 +555,24 @@ velo_status stage_impl(velo_ctx* c, const uint8_t* buf, const uint64_t* offsets,
 
 namespace {
 
+// Work order of events read in place over the host link, from one sorted by
+// size.  In sorted order the resident CTAs start and end their events
+// together: all read from the host at once, then none.  So the largest tenth
+// goes first as it is, the middle is dealt out in steps of the golden section,
+// which spreads the sizes evenly over time, and the smallest third comes last,
+// largest first, to even out the end.  10,000 events of 1,160 hits: 2.02 ->
+// 1.78 ms, 10,000 uneven ones 5.46 -> 5.01, 4,000 of 4,550 hits 4.22 -> 4.07;
+// events in device memory gain 1 % or nothing, learned searches (longer events,
+// the same reads) lose 5 % at their end: both keep the sorted order.
+void interleave_sizes(int32_t* order, int32_t n) {
+  const int32_t a = n / 10, m = n * 2ll / 3 - a;
+  if (m < 3) return;
+  const std::vector<int32_t> middle(order + a, order + a + m);
+  int64_t step = (int64_t)(0.6180339887 * m), at = 0;
+  while (std::gcd(step, (int64_t)m) != 1) ++step;   // every event once
+  for (int32_t i = 0; i < m; ++i, at = (at + step) % m) order[a + i] = middle[(size_t)at];
+}
+
 velo_status prepare_launch(velo_ctx* c, const velo_options& o, uint32_t* smem_out) {
   const uint32_t Y = (uint32_t)o.y_lanes;
   // shared-memory arena size: largest event arena up to the budget
@@ -623,6 +641,7 @@ velo_status prepare_launch(velo_ctx* c, const velo_options& o, uint32_t* smem_ou
       for (int32_t e = 0; e < c->n; ++e) start[kBuckets - 1 - (int)(c->h_hits[e] >> shift) + 1]++;
       for (int b = 0; b < kBuckets; ++b) start[b + 1] += start[b];
       for (int32_t e = 0; e < c->n; ++e) c->h_order[start[kBuckets - 1 - (int)(c->h_hits[e] >> shift)]++] = e;
+      if (c->io_input && !o.learned) interleave_sizes(c->h_order.data(), c->n);
       if ((st = ensure(c, c->d_order, 4ull * c->n, "order")) != VELO_OK) return st;
       if (c->n > 0)
         VELO_CUDA(c, cudaMemcpyAsync(c->d_order.p, c->h_order.data(), 4ull * c->n,
