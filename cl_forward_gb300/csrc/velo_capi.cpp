@@ -731,12 +731,16 @@ void resolve_launch(const velo_ctx* c, velo_options* o) {
       o->ctas_per_sm <= 0 && !c->dump_armed && c->n > 0) {
     const int64_t n = c->n, sms = c->sm_count;
     const bool large = c->total_hits / (uint64_t)n >= 3000;
-    if (n <= sms && !o->learned)   // no learned build of 512
+    if (n <= sms && !o->learned) {   // no learned build of 512
       o->threads_per_event = 512;
-    else if (n <= 8 * sms)
+      // one CTA per SM: room to keep the event in shared memory (one event 0.171
+      // ms instead of 0.179, 100 events 0.238 instead of 0.247)
+      if (o->smem_hits == 50) o->smem_hits = 4000;
+    } else if (n <= 8 * sms) {
       o->threads_per_event = 256;
-    else if (n <= (large ? 36 : 20) * sms)
+    } else if (n <= (large ? 36 : 20) * sms) {
       o->threads_per_event = 128;
+    }
   }
   if (o->register_ctas == 0) o->register_ctas = o->threads_per_event > 256 ? 5 : 4;
 }

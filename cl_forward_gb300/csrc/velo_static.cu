@@ -76,50 +76,52 @@ __host__ __device__ StaticView view_of(uint8_t* base) {
   return v;
 }
 
-// One CTA: validate headers, per-event row offsets (prefix sum of max(H, 1)),
-// and clear the counters.  Events whose rows would pass the scratch end, or
-// the caller's track buffer (row_limit), are marked invalid.
+// One CTA: validate headers and module tables, per-event row offsets (prefix
+// sum of max(H, 1)), and clear the counters.  Events whose rows would pass the
+// scratch end, or the caller's track buffer (row_limit), are marked invalid.
+// A warp checks an event's table at once: walked by one thread it was a chain
+// of 52 reads (5 us of a call on 90 events).
 constexpr int kPrepThreads = 1024;
 
 __global__ void __launch_bounds__(kPrepThreads) static_prep_kernel(const uint8_t* input, const uint64_t* offsets,
                                                                    const uint64_t* sizes, int32_t n,
                                                                    uint32_t max_event_hits, uint64_t row_limit) {
   __shared__ uint64_t part[kPrepThreads];
+  __shared__ uint32_t hits[VELO_STATIC_MAX_EVENTS];   // H, or ~0 for an invalid event
   const StaticView v = view_of(g_velo_static_scratch);
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31;
   if (tid == 0) {
     *v.cursor = 0ull;
     *v.work = 0;
   }
-  const int per = (n + kPrepThreads - 1) / kPrepThreads;
-  const int a = min(n, tid * per), b = min(n, a + per);
-  uint64_t local = 0;
-  for (int e = a; e < b; ++e) {
+  for (int e = tid >> 5; e < n; e += kPrepThreads / 32) {   // warp-uniform
     const uint8_t* blob = input + offsets[e];
     const uint64_t size = sizes[e];
     bool ok = size >= 8 && (offsets[e] & 3u) == 0;
-    int32_t S = 0, H = 0, M = 0;
+    int32_t S = 0, H = 0;
     if (ok) {
       const int32_t* hdr = reinterpret_cast<const int32_t*>(blob);
       S = hdr[0];
       H = hdr[1];
       ok = S >= 0 && S <= VELO_MAX_MODULES && H >= 0 && (uint32_t)H <= max_event_hits &&
-           size >= 8ull + 12ull * (uint64_t)S + 16ull * (uint64_t)H;
-      int64_t acc = 0;
-      for (int m = 0; ok && m < S; ++m) {
+           size >= 8ull + 12ull * (uint64_t)S + 16ull * (uint64_t)H && (S > 0 || H == 0);
+      for (int m = lane; ok && m < S; m += 32) {   // the modules tile [0, H) in order
         const int32_t st = hdr[2 + S + m], nm = hdr[2 + 2 * S + m];
-        ok = nm >= 0 && nm <= VELO_MAX_MODULE_HITS && st == acc;
-        acc += nm;
-        M = max(M, nm);
+        const int64_t expect = m == 0 ? 0 : (int64_t)hdr[2 + S + m - 1] + (int64_t)hdr[2 + 2 * S + m - 1];
+        if (nm < 0 || nm > VELO_MAX_MODULE_HITS || (int64_t)st != expect ||
+            (m == S - 1 && (int64_t)st + (int64_t)nm != (int64_t)H))
+          ok = false;
       }
-      ok = ok && acc == H;
     }
-    v.ev_valid[e] = ok ? 1u : 0u;
-    v.ev_hits[e] = ok ? (uint32_t)H : 0u;
-    v.ev_maxmod[e] = ok ? (uint32_t)M : 0u;
-    v.arena_off[e] = kNoArena;
-    local += ok && H > 0 ? (uint64_t)H : 1ull;
+    ok = __all_sync(0xffffffffu, ok);
+    if (lane == 0) hits[e] = ok ? (uint32_t)H : ~0u;
   }
+  __syncthreads();
+  const int per = (n + kPrepThreads - 1) / kPrepThreads;
+  const int a = min(n, tid * per), b = min(n, a + per);
+  auto rows_of = [&](int e) { return hits[e] == ~0u || hits[e] == 0u ? 1ull : (unsigned long long)hits[e]; };
+  uint64_t local = 0;
+  for (int e = a; e < b; ++e) local += rows_of(e);
   part[tid] = local;
   __syncthreads();
   for (int o = 1; o < kPrepThreads; o <<= 1) {   // inclusive scan of the per-thread row counts
@@ -130,14 +132,13 @@ __global__ void __launch_bounds__(kPrepThreads) static_prep_kernel(const uint8_t
   }
   uint64_t base = part[tid] - local;
   for (int e = a; e < b; ++e) {
-    const uint64_t rows = v.ev_hits[e] > 0 ? v.ev_hits[e] : 1ull;
-    v.hit_base[e] = base;
-    if (base + rows > row_limit) {
-      v.ev_valid[e] = 0u;
-      v.ev_hits[e] = 0u;
-      v.ev_maxmod[e] = 0u;
-      v.hit_base[e] = 0u;
-    }
+    const uint64_t rows = rows_of(e);
+    const bool ok = hits[e] != ~0u && base + rows <= row_limit;
+    v.ev_valid[e] = ok ? 1u : 0u;
+    v.ev_hits[e] = ok ? hits[e] : 0u;
+    v.ev_maxmod[e] = 0u;   // the arena layout depends on H only
+    v.arena_off[e] = kNoArena;
+    v.hit_base[e] = ok || base + rows <= row_limit ? base : 0ull;
     base += rows;
   }
 }
