@@ -955,10 +955,16 @@ __device__ __noinline__ void fill_windows(const EventView ev, const Shared& s) {
 // 32 columns of 1.3 mm span half a module's width, the rows its height.  With
 // 256 rows instead of 64 half as many pairs pass that no hit is near (of 54,000
 // pairs in an event of 4,400 hits 2,850 instead of 6,000, 800 of them met).
-__device__ __forceinline__ int map_column(float x) { return __float2int_rd(fmul(x, 1.f / 1.3125f)); }
+// A cell's number is the scaled coordinate rounded to an integer, taken from
+// the low bits of a sum with 1.5 * 2^23 (one instruction, non-decreasing in the
+// coordinate, and no conversion: those issue at a quarter of the rate).
+__device__ __forceinline__ int map_cell(float v, float scale) {
+  return __float_as_int(__fmaf_rn(v, scale, 12582912.f));
+}
+__device__ __forceinline__ int map_column(float x) { return map_cell(x, 1.f / 1.3125f); }
 template <class Shared>
 __device__ __forceinline__ int map_row(float y) {
-  return __float2int_rd(fmul(y, (float)Shared::kMapRows / 84.f));
+  return map_cell(y, (float)Shared::kMapRows / 84.f);
 }
 
 template <class Shared>
