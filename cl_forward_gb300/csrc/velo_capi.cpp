@@ -300,7 +300,8 @@ void velo_default_options(velo_options* o) {
   std::memset(o, 0, sizeof *o);
   // the fastest configuration measured on GB300 for batches of thousands of
   // events: persistent CTAs of 64 threads, per-event state in L1-cached
-  // global scratch (only events of <= 50 hits in shared memory)
+  // global scratch (only events of <= 50 hits in shared memory); smaller
+  // batches get wider CTAs (resolve_launch)
   o->y_lanes = 4;
   o->threads_per_event = 64;
   o->launch_mode = VELO_LAUNCH_PERSISTENT;

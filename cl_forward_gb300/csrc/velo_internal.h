@@ -25,10 +25,9 @@ constexpr uint32_t kMaxSkippedModules = 3;     // MAX_SKIPPED_MODULES
 constexpr int kMaxModules = VELO_MAX_MODULES;
 constexpr int kMaxModuleHits = VELO_MAX_MODULE_HITS;
 
-// Tracks-to-follow entry bits shared with the reference (Kernel.cl:222-225,
-// 351,566): bit 31 = tracklet, bits 28-30 = skipped modules.
+// Tracks-to-follow entry bit shared with the reference (Kernel.cl:222-225,
+// 351,566): a tracklet.
 constexpr uint32_t kTrackletFlag = 0x80000000u;
-constexpr uint32_t kSkipMask = 0x70000000u;
 constexpr uint64_t kNoArena = ~0ull;
 // Module-table capacity of the compact shared-state build of the search
 // kernel (events with fewer modules; the full build takes kMaxModules).
@@ -63,7 +62,7 @@ constexpr uint32_t kMlpSmemBytes = (sizeof(MlpFrag) + 15) & ~15u;
 // Per-event working set ("arena"): staged in dynamic shared memory when it
 // fits the launch's shared-memory size, else carved from global scratch.
 // Offsets are bytes, each array 16-byte aligned.  21 bytes per hit.  (The
-// tracks-to-follow rings live with the per-row scratch in global memory.)
+// tracks-to-follow entries live with the per-row scratch in global memory.)
 struct ArenaLayout {
   uint32_t x, y, z;              // float[H]    hit coordinates (x-sorted per module)
   uint32_t win;                  // uint2[H]    candidate windows, 16-bit offsets into module f-2
@@ -144,10 +143,10 @@ struct SearchParams {
   int32_t learned_min_window;     // score only doublets with at least this many h2 candidates
 };
 
-// Launches the search kernel (velo_kernels.cu); reg_ctas (4 or 5) picks the
-// register budget of the <= 256-thread build, p.seed_lanes the seeding width.  Returns a cudaError_t value.
-// compact: every event of the launch has fewer than 64 modules (the compact
-// shared-state build).
+// Launches the search kernel (velo_kernels.cu); reg_ctas (4, 5 or 18) picks
+// the register budget of the build, p.seed_lanes the width of the walked
+// seeding.  compact: every event of the launch has fewer than 64 modules (the
+// compact shared-state build).  Returns a cudaError_t value.
 int launch_search(const SearchParams& p, int grid, int block, uint32_t smem_bytes, void* stream, int reg_ctas,
                   bool compact);
 // Sets the kernels' maximum dynamic shared memory.  Returns a cudaError_t value.

@@ -115,12 +115,15 @@ typedef struct velo_options {
   int32_t device_budget_mb;   /* velo_search / velo_search_packed: device memory one call may
                                  use; a batch that needs more (about 275 B per hit) is cut into
                                  pipelined parts that fit.  0 = half the free device memory */
-  int32_t seed_lanes;         /* seeding: lanes given to one h0's h1 candidates, 8, 16 or 32 (a
-                                 warp then seeds 32 / seed_lanes h0s at once); below 32 it must
-                                 be a multiple of y_lanes.  The width of the seeding window a
-                                 warp slides over an h0's h1 candidates (the reference's Y-lanes
-                                 per h0, Kernel.cl:435-436, set how many work-items share one
-                                 h0).  Results do not depend on it.  0 = automatic */
+  int32_t seed_lanes;         /* seeding that walks the candidate windows (unsorted events,
+                                 narrow_windows = 0, the training-data dump, learned seeding of
+                                 modules with several z): lanes given to one h0's h1
+                                 candidates, 8, 16 or 32 (a warp then seeds 32 / seed_lanes h0s
+                                 at once); below 32 it must be a multiple of y_lanes (the
+                                 reference's Y-lanes per h0, Kernel.cl:435-436, set how many
+                                 work-items share one h0).  Other events lay the (h0, h1) pairs
+                                 over whole warps.  Results do not depend on it.
+                                 0 = automatic */
   int32_t learned_min_window; /* learned seeding: only doublets whose exact h2 window holds at
                                  least this many hits are scored; narrower ones are searched
                                  exactly (their search costs less than scoring).  0 = score all */
@@ -146,9 +149,10 @@ typedef struct velo_stats {
 
 typedef struct velo_ctx velo_ctx;
 
-/* Defaults: Y = 4, persistent CTAs of 64 threads, 50-hit shared-memory
- * tile, narrowing on, automatic register build, no graph, no pipelining, no
- * in-place host I/O, plain (not learned) seeding. */
+/* Defaults: Y = 4, persistent CTAs of 64 threads (up to 512 for batches that
+ * are small for the device: register_ctas = 0), 50-hit shared-memory tile,
+ * narrowing on, no graph, no pipelining, no in-place host I/O, plain (not
+ * learned) seeding. */
 void velo_default_options(velo_options* opts);
 const char* velo_status_string(velo_status s);
 
