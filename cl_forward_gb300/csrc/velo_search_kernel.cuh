@@ -1867,11 +1867,12 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
 // resident 256-thread CTAs per SM (velo_options.register_ctas 4 / 5: 64 / 48
 // registers; of up to 64 threads in a build with the seeding state of two
 // warps), 64-thread CTAs with 56 registers (18 CTAs per SM, register_ctas 18),
-// and 512-thread CTAs; the learned mode in a build of up to
-// 256 threads with 80 registers (3 resident CTAs; 2.76 against 3.28 ms with 64
-// for 5,000 events with the scorer out of line, 2.02 ms with it inlined) and
-// one of up to 64 threads (1.92 ms); each for one seeding
-// width kLanes (lanes per h0 where the windows are walked).
+// and 512-thread CTAs; the learned mode in a build of up to 256 threads with
+// 80 registers (3 resident CTAs) and one of up to 64 threads whose bound of 11
+// CTAs leaves the same 80 registers, and 12 CTAs fit (5,000 events 1.43 ms;
+// bounds of 12, 10 and 16: 1.47, 1.47 and 1.61; with the scorer out of line
+// 1.75); each for one seeding width kLanes (lanes per h0 where the windows are
+// walked).
 template <int kMaxThreads, int kMinCtas, int kMode, int kMods, int kLanes>
 __global__ void __launch_bounds__(kMaxThreads, kMinCtas) search_kernel(const __grid_constant__ SearchParams p) {
   extern __shared__ __align__(16) uint8_t dyn_smem_raw[];
@@ -1910,7 +1911,7 @@ struct SearchBuilds {
   static int launch(const SearchParams& p, int grid, int block, uint32_t smem, cudaStream_t st, int reg_ctas,
                     bool compact) {
     if (p.mlp && compact && block <= 64)
-      search_kernel<64, 12, kLearned, kCompactModules, G><<<grid, block, smem, st>>>(p);
+      search_kernel<64, 11, kLearned, kCompactModules, G><<<grid, block, smem, st>>>(p);
     else if (p.mlp && compact)
       search_kernel<256, 3, kLearned, kCompactModules, G><<<grid, min(block, 256), smem, st>>>(p);
     else if (p.mlp)
@@ -1953,7 +1954,7 @@ struct SearchBuilds {
     VELO_LIMIT(search_kernel<512, 1, kPlain, kFullModules, G>);
     VELO_LIMIT(search_kernel<256, 3, kLearned, kFullModules, G>);
     VELO_LIMIT(search_kernel<256, 3, kLearned, kCompactModules, G>);
-    VELO_LIMIT(search_kernel<64, 12, kLearned, kCompactModules, G>);
+    VELO_LIMIT(search_kernel<64, 11, kLearned, kCompactModules, G>);
     if (G == 32) VELO_LIMIT(search_kernel<256, 4, kDump, kFullModules, 32>);
 #undef VELO_LIMIT
     return (int)e;
@@ -1962,7 +1963,7 @@ struct SearchBuilds {
   static int occupancy(int block, uint32_t smem, int reg_ctas, int mode, bool compact, int* ctas) {
     if (mode == kModeLearned && compact && block <= 64)
       return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-          ctas, search_kernel<64, 12, kLearned, kCompactModules, G>, block, smem);
+          ctas, search_kernel<64, 11, kLearned, kCompactModules, G>, block, smem);
     if (mode == kModeLearned)
       return compact ? (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                            ctas, search_kernel<256, 3, kLearned, kCompactModules, G>, min(block, 256), smem)
