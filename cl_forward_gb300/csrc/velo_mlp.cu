@@ -14,10 +14,12 @@
 //   W1[32][10] b1[32] W2[32][32] b2[32] W3[2][32] b3[2]
 // (row-major, out x in).
 #include <cuda_runtime.h>
+#include <float.h>
 #include <math.h>
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "velo_internal.h"
@@ -55,6 +57,16 @@ __device__ __forceinline__ float sample_loss(const float* out, float label, floa
 // more than 2e-5 of the weights' norm away from it (one unit of one sample
 // decided otherwise), with these none.
 __device__ __forceinline__ float mul_add(float a, float b, float c) { return __fadd_rn(c, __fmul_rn(a, b)); }
+
+// The same where the unit's gradient a is not 0: a unit that is not live adds
+// nothing, also where b is infinite or NaN (a feature or a weight is).  kFinite:
+// it is known to be neither.
+template <bool kFinite>
+__device__ __forceinline__ float mul_add_live(float a, float b, float c) {
+  return kFinite || a != 0.f ? mul_add(a, b, c) : c;
+}
+
+__device__ __forceinline__ bool finite(float v) { return fabsf(v) <= FLT_MAX; }
 
 struct GradTile {
   float w[(VELO_MLP_PARAMS + 3) & ~3];
@@ -108,24 +120,31 @@ __global__ void __launch_bounds__(kTrainThreads) mlp_step_kernel(const float* w,
   const int j2 = tid >> 4, i2 = tid & 15;   // this thread's outputs of W2's gradient: row j2, columns i2 + 16 q
   float gw2[2] = {}, gw1 = 0.f, gw3[kMlpOut][kUnits] = {}, gb1[kUnits] = {}, gb2[kUnits] = {}, gb3[kMlpOut] = {};
   float loss = 0.f;
+  bool odd = false;   // a weight is infinite or NaN, or a feature or activation of the tile
 
   // the samples do not depend on the launch before this one, the weights do
   const int64_t tiles = (n + kTile - 1) / kTile;
   for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int64_t base = tile * kTile;
     if (tile != blockIdx.x) __syncthreads();   // the tile before has been read
+    bool odd_tile = false;
     for (int k = tid; k < kTile * kMlpIn; k += kTrainThreads) {
       const int s = k / kMlpIn, i = k % kMlpIn;
       float v = 0.f;
       if (base + s < n) v = x[(index ? index[base + s] : base + s) * kMlpIn + i];
       t.x[i][s] = v;
+      odd_tile |= !finite(v);
     }
     const bool in = base + lane < n;
     const int64_t r = in ? (index ? index[base + lane] : base + lane) : 0;
     const float y = in ? label[r] : 0.f, width = in ? target[r] : 0.f;
     if (tile == blockIdx.x) {
       cudaGridDependencySynchronize();
-      for (int k = tid; k < VELO_MLP_PARAMS; k += kTrainThreads) t.w[k] = __ldcg(w + k);
+      for (int k = tid; k < VELO_MLP_PARAMS; k += kTrainThreads) {
+        const float v = __ldcg(w + k);
+        t.w[k] = v;
+        odd |= !finite(v);
+      }
     }
     __syncthreads();
     // layer 1
@@ -141,10 +160,11 @@ __global__ void __launch_bounds__(kTrainThreads) mlp_step_kernel(const float* w,
     if (tile == blockIdx.x) cudaTriggerProgrammaticLaunchCompletion();   // the reduction may be set up
 #pragma unroll
     for (int u = 0; u < kUnits; ++u) {
-      a1[u] = a1[u] > 0.f ? a1[u] : 0.f;
+      a1[u] = in && a1[u] > 0.f ? a1[u] : 0.f;   // no unit of a missing sample is live
       t.a1[u0 + u][lane] = a1[u];
+      odd_tile |= !finite(a1[u]);
     }
-    __syncthreads();
+    const bool careful = __syncthreads_or(odd || odd_tile);
     // layer 2
 #pragma unroll
     for (int u = 0; u < kUnits; ++u) a2[u] = t.w[kMlpB2 + u0 + u];
@@ -161,7 +181,7 @@ __global__ void __launch_bounds__(kTrainThreads) mlp_step_kernel(const float* w,
     }
 #pragma unroll
     for (int u = 0; u < kUnits; ++u) {
-      a2[u] = a2[u] > 0.f ? a2[u] : 0.f;
+      a2[u] = in && a2[u] > 0.f ? a2[u] : 0.f;
       t.a2_d1[u0 + u][lane] = a2[u];
     }
     __syncthreads();
@@ -196,42 +216,49 @@ __global__ void __launch_bounds__(kTrainThreads) mlp_step_kernel(const float* w,
       t.d2[u0 + u][lane] = g;
     }
     __syncthreads();
-    // layer 1: back through W2
-    float d1[kUnits] = {};
+    auto backward = [&](auto known_finite) {
+      constexpr auto add = mul_add_live<decltype(known_finite)::value>;
+      // layer 1: back through W2
+      float d1[kUnits] = {};
 #pragma unroll 8
-    for (int j = 0; j < kMlpHidden; ++j) {
-      const float v = t.d2[j][lane];
-      const float2 c = *reinterpret_cast<const float2*>(&t.w[kMlpW2 + j * kMlpHidden + u0]);
-      d1[0] = mul_add(c.x, v, d1[0]);
-      d1[1] = mul_add(c.y, v, d1[1]);
-    }
-#pragma unroll
-    for (int u = 0; u < kUnits; ++u) {
-      const float g = a1[u] > 0.f ? d1[u] : 0.f;
-      gb1[u] += g;
-      t.a2_d1[u0 + u][lane] = g;
-    }
-    // W2's gradient: sums over the samples of d2[j] a1[i]
-#pragma unroll
-    for (int k = 0; k < kTile; k += 4) {
-      const float4 d = *reinterpret_cast<const float4*>(&t.d2[j2][k]);
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const float4 a = *reinterpret_cast<const float4*>(&t.a1[i2 + 16 * q][k]);
-        gw2[q] = mul_add(d.w, a.w, mul_add(d.z, a.z, mul_add(d.y, a.y, mul_add(d.x, a.x, gw2[q]))));
+      for (int j = 0; j < kMlpHidden; ++j) {
+        const float v = t.d2[j][lane];
+        const float2 c = *reinterpret_cast<const float2*>(&t.w[kMlpW2 + j * kMlpHidden + u0]);
+        d1[0] = add(v, c.x, d1[0]);
+        d1[1] = add(v, c.y, d1[1]);
       }
-    }
-    __syncthreads();
-    // W1's gradient: 320 outputs, d1[j] x[i]
-    if (tid < kMlpHidden * kMlpIn) {
-      const float* d = t.a2_d1[tid / kMlpIn];
-      const float* v = t.x[tid % kMlpIn];
+#pragma unroll
+      for (int u = 0; u < kUnits; ++u) {
+        const float g = a1[u] > 0.f ? d1[u] : 0.f;
+        gb1[u] += g;
+        t.a2_d1[u0 + u][lane] = g;
+      }
+      // W2's gradient: sums over the samples of d2[j] a1[i]
 #pragma unroll
       for (int k = 0; k < kTile; k += 4) {
-        const float4 a = *reinterpret_cast<const float4*>(&d[k]), b = *reinterpret_cast<const float4*>(&v[k]);
-        gw1 = mul_add(a.w, b.w, mul_add(a.z, b.z, mul_add(a.y, b.y, mul_add(a.x, b.x, gw1))));
+        const float4 d = *reinterpret_cast<const float4*>(&t.d2[j2][k]);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const float4 a = *reinterpret_cast<const float4*>(&t.a1[i2 + 16 * q][k]);
+          gw2[q] = add(d.w, a.w, add(d.z, a.z, add(d.y, a.y, add(d.x, a.x, gw2[q]))));
+        }
       }
-    }
+      __syncthreads();
+      // W1's gradient: 320 outputs, d1[j] x[i]
+      if (tid < kMlpHidden * kMlpIn) {
+        const float* d = t.a2_d1[tid / kMlpIn];
+        const float* v = t.x[tid % kMlpIn];
+#pragma unroll
+        for (int k = 0; k < kTile; k += 4) {
+          const float4 a = *reinterpret_cast<const float4*>(&d[k]), b = *reinterpret_cast<const float4*>(&v[k]);
+          gw1 = add(a.w, b.w, add(a.z, b.z, add(a.y, b.y, add(a.x, b.x, gw1))));
+        }
+      }
+    };
+    if (careful)
+      backward(std::false_type{});
+    else
+      backward(std::true_type{});
   }
 
   float* row = partial + (size_t)blockIdx.x * kPartialRow;
