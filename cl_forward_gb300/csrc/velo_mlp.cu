@@ -19,6 +19,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <exception>
 #include <type_traits>
 #include <vector>
 
@@ -348,6 +349,7 @@ namespace {
 // The device arrays of one call, in one allocation (each cudaMalloc / cudaFree
 // pair takes 70 us): reserve them all, then allocate.
 struct DevArrays {
+  static constexpr size_t kMost = (size_t)1 << 62;
   uint8_t* base = nullptr;
   size_t total = 0;
   cudaStream_t stream = nullptr, aux = nullptr;
@@ -361,10 +363,15 @@ struct DevArrays {
   template <typename T>
   size_t reserve(size_t count) {
     const size_t at = total;
-    total += (sizeof(T) * (count ? count : 1) + 255) & ~(size_t)255;
+    if (count > (kMost - total) / sizeof(T))
+      total = kMost;   // no such allocation: allocate() fails
+    else
+      total += (sizeof(T) * (count ? count : 1) + 255) & ~(size_t)255;
     return at;
   }
-  cudaError_t allocate() { return cudaMalloc(reinterpret_cast<void**>(&base), total); }
+  cudaError_t allocate() {
+    return total >= kMost ? cudaErrorMemoryAllocation : cudaMalloc(reinterpret_cast<void**>(&base), total);
+  }
   template <typename T>
   T* at(size_t offset) const { return reinterpret_cast<T*>(base + offset); }
 };
@@ -476,14 +483,13 @@ extern "C" velo_status velo_mlp_forward(const float* weights, const float* x, in
   return VELO_OK;
 }
 
-extern "C" velo_status velo_mlp_train(const float* x, const float* label, const float* target, int64_t n,
-                                      int32_t steps, int32_t batch, float lr, uint64_t seed, float* weights_inout,
-                                      float* loss_per_step) {
-  if (!x || !label || !target || n <= 0 || steps <= 0 || batch <= 0 || !weights_inout)
-    return VELO_ERR_INVALID_ARGUMENT;
+namespace {
+
+velo_status train(const float* x, const float* label, const float* target, int64_t n, int32_t steps, int32_t batch,
+                  float lr, uint64_t seed, float* weights_inout, float* loss_per_step) {
   const uint64_t places = (uint64_t)steps * (uint64_t)batch;   // samples drawn in all
-  std::vector<int64_t> idx((size_t)places);   // outlives the copies on d.stream
-  std::vector<int64_t> order((size_t)n);
+  std::vector<int64_t> idx;   // outlives the copies on d.stream
+  std::vector<int64_t> order;
   std::vector<uint32_t> draws;
   DevArrays d;
   const bool device_draws = n > 1 && n <= (int64_t)0xffffffff;
@@ -500,6 +506,9 @@ extern "C" velo_status velo_mlp_train(const float* x, const float* label, const 
                oi = d.reserve<int64_t>((size_t)places),
                od = d.reserve<uint32_t>(device_draws ? (size_t)(epochs_at_once * swaps) : 1);
   MLP_CHECK(d.allocate());
+  idx.resize((size_t)places);
+  order.resize((size_t)n);
+  if (device_draws) draws.resize((size_t)(epochs_at_once * swaps));
   float *dw = d.at<float>(ow), *dx = d.at<float>(ox), *dl = d.at<float>(ol), *dt = d.at<float>(ot),
         *dp = d.at<float>(op), *dm = d.at<float>(om), *dv = d.at<float>(ov), *dloss = d.at<float>(oloss);
   int64_t* didx = d.at<int64_t>(oi);
@@ -520,7 +529,6 @@ extern "C" velo_status velo_mlp_train(const float* x, const float* label, const 
   for (uint64_t e = 0; e < epochs; ++e) {
     if (device_draws && e % epochs_at_once == 0) {
       const uint64_t count = std::min(epochs_at_once, epochs - e) * swaps;
-      draws.resize((size_t)count);
       const unsigned blocks = (unsigned)std::min<uint64_t>((count + 255) / 256, 4096);
       shuffle_draws_kernel<<<blocks, 256, 0, d.aux>>>(seed, (uint64_t)n, e * swaps, count, d.at<uint32_t>(od));
       MLP_CHECK(cudaGetLastError());
@@ -554,4 +562,18 @@ extern "C" velo_status velo_mlp_train(const float* x, const float* label, const 
   MLP_CHECK(cudaMemcpy(weights_inout, dw, sizeof(float) * VELO_MLP_PARAMS, cudaMemcpyDeviceToHost));
   if (loss_per_step) MLP_CHECK(cudaMemcpy(loss_per_step, dloss, sizeof(float) * steps, cudaMemcpyDeviceToHost));
   return VELO_OK;
+}
+
+}  // namespace
+
+extern "C" velo_status velo_mlp_train(const float* x, const float* label, const float* target, int64_t n,
+                                      int32_t steps, int32_t batch, float lr, uint64_t seed, float* weights_inout,
+                                      float* loss_per_step) {
+  if (!x || !label || !target || n <= 0 || steps <= 0 || batch <= 0 || !weights_inout)
+    return VELO_ERR_INVALID_ARGUMENT;
+  try {
+    return train(x, label, target, n, steps, batch, lr, seed, weights_inout, loss_per_step);
+  } catch (const std::exception&) {   // the host's sample order does not fit
+    return VELO_ERR_OUT_OF_MEMORY;
+  }
 }
