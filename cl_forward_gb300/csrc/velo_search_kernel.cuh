@@ -138,6 +138,13 @@ struct EventView {
   int y_lanes, narrow;
 };
 
+// Hits of a module that the general seedings look at at once: their loads and
+// distances do not depend on one another.  One after another, with a branch on
+// each, the walk of an unsorted module's windows waits some 100 cycles a hit: 100
+// unsorted events of 1,240 hits 7.0 -> 3.3 ms with 64 threads, 2.3 -> 1.6 ms
+// with 512 (two or eight at once: 4.1 ms with 64 threads).
+constexpr int kAtOnce = 4;
+
 // First index i in [lo, hi) with x[i] > c, for non-decreasing x.
 __device__ __forceinline__ int first_gt(const float* x, int lo, int hi, float c) {
   while (lo < hi) {
@@ -866,20 +873,30 @@ __device__ void seed_module(const EventView& ev, Shared& s, Worker& w, int f, co
       float lbest = FLT_MAX;
       int lk = -1;
       uint32_t zc = 0x7fc00001u;
-      float z2_tz = 0.f, den = 0.f;
-      for (int k = a; k < b; ++k) {
-        const float h2z = z4[k];
-        if (__float_as_uint(h2z) != zc) {   // both factors depend on h2z only (per h0, h1)
-          zc = __float_as_uint(h2z);
-          z2_tz = fmul(fsub(h2z, h0z), dz_inverted);
-          den = fdiv(1.f, fsub(h2z, h1z));
+      float den = 0.f;
+      for (int k0 = a; k0 < b; k0 += kAtOnce) {
+        float dx[kAtOnce], dy[kAtOnce], z2[kAtOnce];
+        uint32_t near = 0;
+#pragma unroll
+        for (int q = 0; q < kAtOnce; ++q) {
+          const int k = min(k0 + q, b - 1);
+          z2[q] = z4[k];
+          const float z2_tz = fmul(fsub(z2[q], h0z), dz_inverted);
+          dx[q] = fsub(fadd(h0x, fmul(ddx, z2_tz)), x4[k]);
+          dy[q] = fsub(fadd(h0y, fmul(ddy, z2_tz)), y4[k]);
+          near |= (uint32_t)(k0 + q < b && fabsf(dx[q]) < kTolerance && fabsf(dy[q]) < kTolerance) << q;
         }
-        const float dx = fsub(fadd(h0x, fmul(ddx, z2_tz)), x4[k]);
-        const float dy = fsub(fadd(h0y, fmul(ddy, z2_tz)), y4[k]);
-        if (fabsf(dx) < kTolerance && fabsf(dy) < kTolerance) {
-          const float scatter = fmul(fmul(fadd(fmul(dx, dx), fmul(dy, dy)), den), den);
+        if (near == 0) continue;
+#pragma unroll
+        for (int q = 0; q < kAtOnce; ++q) {
+          if (!((near >> q) & 1u)) continue;
+          if (__float_as_uint(z2[q]) != zc) {   // the factor depends on z2 only (per h1)
+            zc = __float_as_uint(z2[q]);
+            den = fdiv(1.f, fsub(z2[q], h1z));
+          }
+          const float scatter = fmul(fmul(fadd(fmul(dx[q], dx[q]), fmul(dy[q], dy[q])), den), den);
           if (scatter < kMaxScatter) {
-            if (scatter < lbest) { lbest = scatter; lk = k; }
+            if (scatter < lbest) { lbest = scatter; lk = k0 + q; }
           } else if (!isfinite(scatter)) {
             degenerate = true;
           }
@@ -1042,11 +1059,17 @@ __device__ __forceinline__ void h1_window(const EventView& ev, const Shared& s, 
     auto passes = [&](int e) {
       return fabsf(fsub(x[e], x0)) < fmul(kMaxXSlopeCandidates, fabsf(fsub(z[e], z0)));
     };
-    while (lo < hi && !passes(lo)) ++lo;
-    int end = lo;
-    while (end < hi && passes(end)) ++end;
-    *first = lo;
-    *last = end;
+    auto next = [&](int e, bool what) {   // the first from e on that does so
+      for (; e < hi; e += kAtOnce) {
+        uint32_t m = 0;
+#pragma unroll
+        for (int q = 0; q < kAtOnce; ++q) m |= (uint32_t)(passes(min(e + q, hi - 1)) == what) << q;
+        if (m) return min(e + __ffs(m) - 1, hi);
+      }
+      return hi;
+    };
+    *first = next(lo, true);
+    *last = next(*first, false);
   }
 }
 
@@ -1517,29 +1540,29 @@ static __device__ unsigned long long g_phase_cycles[8];   // one per translation
 #endif
 
 // The module loop, Kernel.cl:671-767 (see Worker for the order of the warps).
-// kMode: the seeding; kPlainGeometry: the event is of plain geometry.
-template <int kMode, int kLanes, bool kPlainGeometry, class Shared>
+// kMode: the seeding; kPlainGeometry: the event is of plain geometry; kPairs:
+// it takes the pair seeding.
+template <int kMode, int kLanes, bool kPlainGeometry, bool kPairs, class Shared>
 __device__ __forceinline__ Worker module_loop(const EventView& ev, Shared& s, Worker w) {
   const int lane = threadIdx.x & 31, S = ev.S;
   for (int f = S - 1; f >= 4; --f) {
     forward<kPlainGeometry>(ev, s, w, f);
     const int step = (S - 1 - f) & 1;
     if (w.alone() || step == w.parity()) {
-      const bool by_pairs = kPlainGeometry || (kMode == kPlain && ev.tame);
       const int gt = w.idx() * 32 + lane, gn = w.of() * 32;
       if (kPlainGeometry) {
         uint4* map = reinterpret_cast<uint4*>(s.seed.map[w.parity()]);
         for (int i = gt; i < Shared::kMapRows / 4; i += gn) map[i] = make_uint4(0, 0, 0, 0);
       }
       group_sync<Shared::kMaxWarps>(w);
-      if (by_pairs) {
+      if constexpr (kPairs) {
         if (w.idx() == 0) list_h1s(ev, s, w, f - 2);
         if (kPlainGeometry)   // from the group's last warp on
           for (int i = gn - 1 - gt; i < s.num(f - 4); i += gn)
             mark_map(ev, s, s.seed.map[w.parity()], f - 2, f - 4, i);
         group_sync<Shared::kMaxWarps>(w);
         seed_pairs<kPlainGeometry ? kMode : kPlain, kPlainGeometry>(ev, s, w, f);
-      } else if constexpr (!kPlainGeometry) {
+      } else {
         seed_module<kMode, kLanes>(ev, s, w, f, seed_lanes_of(kLanes, (uint32_t)ev.y_lanes));
       }
       group_sync<Shared::kMaxWarps>(w);
@@ -1549,11 +1572,24 @@ __device__ __forceinline__ Worker module_loop(const EventView& ev, Shared& s, Wo
   return w;
 }
 
-// For the events that the kernel's own loop is not made for, out of line: it
-// then costs that loop no registers.
-template <int kMode, int kLanes, bool kPlainGeometry, class Shared>
-__device__ __noinline__ Worker module_loop_any(const EventView ev, Shared& s, Worker w) {
-  return module_loop<kMode, kLanes, kPlainGeometry>(ev, s, w);
+// The loops of the events that the kernel's own is not made for: each of its own
+// registers, and behind one call of the kernel, so that what they need is none
+// of the kernel's concern (called from it directly, they moved its spills: 1.67
+// -> 1.73 ms for 10,000 events that never call them).  With the two seedings in
+// one loop, events of several z per module ran 5 to 10 % slower.
+template <int kMode, int kLanes, bool kPlainGeometry, bool kPairs, class Shared>
+__device__ __noinline__ Worker module_loop_any(const EventView& ev, Shared& s, Worker w) {
+  return module_loop<kMode, kLanes, kPlainGeometry, kPairs>(ev, s, w);
+}
+
+template <int kMode, int kLanes, class Shared>
+__device__ __noinline__ Worker module_loop_other(const EventView ev, Shared& s, Worker w, bool learned) {
+  constexpr int kOther = kMode == kDump ? kDump : kPlain;
+  if (kMode == kDump || !ev.tame || (learned && !ev.plain))
+    return learned ? module_loop_any<kMode, kLanes, false, false>(ev, s, w)
+                   : module_loop_any<kOther, kLanes, false, false>(ev, s, w);
+  if (!ev.plain) return module_loop_any<kPlain, kLanes, false, true>(ev, s, w);
+  return module_loop_any<kPlain, kLanes, true, true>(ev, s, w);
 }
 
 // ---------------------------------------------------------------------------
@@ -1758,13 +1794,10 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
       w.n = w.tracklets = w.tracks = w.weak = 0;
       __syncthreads();
     }
-    constexpr int kOther = kMode == kDump ? kDump : kPlain;
-    if (kMode == kDump || !ev.plain)
-      w = learned ? module_loop_any<kMode, kLanes, false>(ev, s, w) : module_loop_any<kOther, kLanes, false>(ev, s, w);
-    else if (kMode == kLearned && !learned)
-      w = module_loop_any<kPlain, kLanes, true>(ev, s, w);
+    if (kMode == kDump || !ev.plain || (kMode == kLearned && !learned))
+      w = module_loop_other<kMode, kLanes>(ev, s, w, learned);
     else if constexpr (kMode != kDump)
-      w = module_loop<kMode, kLanes, true>(ev, s, w);
+      w = module_loop<kMode, kLanes, true, true>(ev, s, w);
     VELO_PHASE(4);
 
     // leftover tracklets become weak (Kernel.cl:771-792)
