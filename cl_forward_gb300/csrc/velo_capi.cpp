@@ -117,6 +117,8 @@ struct velo_ctx {
   velo_stats stats{};
   bool ran = false;
 
+  bool pipelined_part = false;   // a child context: its searches run beside its sibling's
+
   // learned seeding
   DevBuf d_mlp;
   bool mlp_set = false;
@@ -727,19 +729,33 @@ velo_status check_options(velo_ctx* c, const velo_options* opts, velo_options* o
 //   6,000   0.47  0.68  1.09   1.00  1.35  2.08   5.4  5.2  6.7
 // (2,440 hits cross where 1,160 do.)  512 threads, one CTA per SM, take up to
 // one event per SM: 100 events of 1,160 hits 0.25 ms, 0.27 with 256 threads.
+// Learned searches of ordinary events cross earlier, as fewer of their CTAs are
+// resident (80 registers):
+//               250 hits           1,240              4,310
+//     304   0.19  0.18  0.17   0.49  0.40  0.35   8.3  5.0  3.3
+//     608   0.20  0.19  0.22   0.54  0.44  0.48   8.8  5.4  3.8
+//   1,216   0.23  0.26  0.38   0.61  0.61  0.78   9.6  6.3  4.9
+//   2,000   0.27  0.35  0.54   0.73  0.90  1.25  11.1  7.1  7.7
+//   2,500   0.33  0.45  0.67   0.83  1.05  1.53  11.4  8.2  9.6
+// Two parts of a pipelined batch are searched at once, so a part counts twice:
+// whole calls on parts of 1,000 events of 1,240 hits read in place 3.8 / 3.2 /
+// 3.9 ms, of 2,500 events 2.4 / 2.8 / 3.9; 300 events of them 2.7 / 2.3 / 2.1;
+// large events fill the device either way (1,000 events of 4,310 hits 5.6 / 3.8
+// / 3.3).
 void resolve_launch(const velo_ctx* c, velo_options* o) {
   if (o->register_ctas == 0 && o->threads_per_event == 64 && o->launch_mode == VELO_LAUNCH_PERSISTENT &&
       o->ctas_per_sm <= 0 && !c->dump_armed && c->n > 0) {
-    const int64_t n = c->n, sms = c->sm_count;
-    const bool large = c->total_hits / (uint64_t)n >= 3000;
-    if (n <= sms && !o->learned) {   // no learned build of 512
+    const int64_t sms = c->sm_count;
+    const bool large = c->total_hits / (uint64_t)c->n >= 3000;
+    const int64_t n = c->pipelined_part && !large ? 2 * (int64_t)c->n : c->n;
+    if (c->n <= sms && !o->learned) {   // no learned build of 512
       o->threads_per_event = 512;
       // one CTA per SM: room to keep the event in shared memory (one event 0.171
       // ms instead of 0.179, 100 events 0.238 instead of 0.247)
       if (o->smem_hits == 50) o->smem_hits = 4000;
-    } else if (n <= 8 * sms) {
+    } else if (n <= (o->learned && !large ? 3 : 8) * sms) {
       o->threads_per_event = 256;
-    } else if (n <= (large ? 36 : 20) * sms) {
+    } else if (n <= (large ? 36 : o->learned ? 8 : 20) * sms) {
       o->threads_per_event = 128;
     }
   }
@@ -984,6 +1000,7 @@ velo_status search_pipelined(velo_ctx* c, const uint8_t* buf, const uint64_t* of
         c->err = "pipeline context: " + std::string(velo_status_string(st));
         return st;
       }
+      c->pipe[k]->pipelined_part = true;
     }
     if (o.learned && c->pipe_mlp_version[k] != c->mlp_version) {
       velo_status st = velo_set_mlp(c->pipe[k], c->h_mlp.data(), c->keep_threshold, c->window_margin,
@@ -1052,6 +1069,7 @@ velo_status search_pipelined(velo_ctx* c, const uint8_t* buf, const uint64_t* of
     const int32_t a = k * part, b = std::min(n, a + part);
     velo_status st = stage_impl(ch, buf, offsets + a, sizes + a, b - a, o.host_direct != 0);
     if (st == VELO_OK) st = velo_run(ch, &po);
+    if (k == 0) c->stats.block = ch->stats.block;   // the last part may be smaller
     if (st != VELO_OK) {
       c->err = ch->err;
       first_error = st;
