@@ -750,8 +750,10 @@ void resolve_launch(const velo_ctx* c, velo_options* o) {
     const int64_t n = c->pipelined_part && !large ? 2 * (int64_t)c->n : c->n;
     if (c->n <= sms && !o->learned) {   // no learned build of 512
       o->threads_per_event = 512;
-      // one CTA per SM: room to keep the event in shared memory (one event 0.171
-      // ms instead of 0.179, 100 events 0.238 instead of 0.247)
+      // one CTA per SM: room to keep the events in shared memory (one event of
+      // 1,240 hits 0.150 ms, 0.159 from global scratch; 100 events 0.223 and
+      // 0.235, of 4,310 hits, some above the tile, 0.789 and 0.778).  The default
+      // stands for this, as its 64 threads do; other tiles are the caller's.
       if (o->smem_hits == 50) o->smem_hits = 4000;
     } else if (n <= (o->learned && !large ? 3 : 8) * sms) {
       o->threads_per_event = 256;

@@ -85,7 +85,11 @@ typedef struct velo_options {
   int32_t y_lanes;            /* reference local size dim 1 (1..16); its output uses 4 */
   int32_t threads_per_event;  /* 32, 64, 128, 256 or 512 */
   int32_t launch_mode;        /* velo_launch_mode */
-  int32_t smem_hits;          /* largest event (hits) staged in shared memory; 0 = auto */
+  int32_t smem_hits;          /* largest event (hits) staged in shared memory; 0 = auto.  The
+                                 default, 50, is automatic too in an automatic launch
+                                 (register_ctas): CTAs of 512 threads then stage events of up
+                                 to 4,000 hits.  Any other value, or one beside a register
+                                 build of the caller's choice, is taken as it is */
   int32_t narrow_windows;     /* 1: binary-search narrowing of x windows (decisions unchanged) */
   int32_t ctas_per_sm;        /* persistent mode: resident CTAs per SM; 0 = auto */
   int32_t use_graph;          /* 1: capture the launch sequence in a CUDA graph and replay it */
