@@ -226,8 +226,14 @@ extern "C" velo_status velo_search_device_static(const uint8_t* d_input, const u
   p.out_status = d_status;
   p.out_cursor = v.cursor;
   p.work_counter = v.work;
-  // wide CTAs while there is at most one per SM, as velo_run's automatic launch
-  const int threads = n_events <= sms ? 512 : n_events <= 8 * sms ? 256 : 128;
+  // Wide CTAs while they are few for the device; the build with the full module
+  // tables, as the events' module counts are not known here.  Milliseconds a
+  // call with 64 / 128 / 256 / 512 threads, one CTA per event (hits):
+  //   100 (1,240)  0.41  0.31  0.25  0.24     600 (22)  0.135 0.129 0.132 0.20
+  //   152 (250)    0.15  0.14  0.13  0.13   1,216       0.155 0.155 0.193 0.33
+  //   250          0.15  0.15  0.14  0.21   2,500       0.215 0.244 0.305 0.58
+  //   400          0.16  0.16  0.15  0.29   4,096       0.29  0.35  0.45  0.92
+  const int threads = n_events <= sms ? 512 : n_events <= 3 * sms ? 256 : n_events <= 8 * sms ? 128 : 64;
   if (launch_search(p, n_events, threads, smem, s, 4, false) != 0) return VELO_ERR_CUDA;
   return VELO_OK;
 }
