@@ -372,7 +372,7 @@ def profiled_traffic(config: str, n_events: int):
     """DRAM bytes of one launch: the ncu capture's bytes per event x events.
 
     The capture ran on 7,000 events of the same workload (a full 10,000-event
-    capture would exceed the size a 45-pass ncu replay can take in minutes);
+    capture would exceed the size a 16-pass ncu replay can take in minutes);
     DRAM traffic grows in proportion to the events processed, so it scales.
     """
     name = PROFILES.get(config)

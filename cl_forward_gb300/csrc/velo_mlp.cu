@@ -103,13 +103,14 @@ __device__ __forceinline__ float lane_sum(float v) {
 // are products over the tile's samples, each thread holding the same outputs
 // for every tile.
 //
-// The step's floor is 3,904 multiply-adds a sample, 0.2 us for a batch of
-// 4,096 on the whole chip; what bounds it is the chain of launches, gather, five
-// exchanges and reduction.  A thread per sample with every product added by a
-// shared-memory atomic, which all lanes of a warp aimed at one address, took
-// 1.47 ms a step; this tile with its sums added to the gradient by atomics and
-// the update in the last CTA 20.8 us (128 CTAs waiting on their atomics and a
-// counter); rows of partial sums and a second kernel 10.7 us.
+// The step's floor is 3,904 products and sums a sample, 0.8 us for a batch of
+// 4,096 on the whole chip at an instruction each (0.4 if they were fused); what
+// bounds it is the chain of launches, gather, six exchanges and reduction.  A
+// thread per sample with every product added by a shared-memory atomic, which
+// all lanes of a warp aimed at one address, took 1.47 ms a step; this tile with
+// its sums added to the gradient by atomics and the update in the last CTA 20.8
+// us (128 CTAs waiting on their atomics and a counter); rows of partial sums and
+// a second kernel 11.0 us.
 __global__ void __launch_bounds__(kTrainThreads) mlp_step_kernel(const float* w,
                                                                  const float* __restrict__ x,
                                                                  const float* __restrict__ label,

@@ -306,11 +306,11 @@ __device__ void compute_windows(const EventView& ev, const Shared& s, int h, int
 // So the warps meet once per two iterations: when iterations f and f-1 begin,
 // every forwarding down to f+1 has been done by all of them.
 //
-// Before, all warps forwarded and seeded each module together: two barriers
-// per iteration, shared-memory counters, and each module's 4 unused h0s spread
-// over the warps.  With 64 threads the split runs one warp per parity: 173 k ->
-// 142 k warp instructions per event, 10,000 events of 1,160 hits 2.50 -> 1.97
-// ms, one event 0.42 -> 0.29 ms.
+// All warps forwarding and seeding each module together takes two barriers per
+// iteration, shared-memory counters, and spreads each module's 4 unused h0s
+// over the warps.  With 64 threads the split runs one warp per parity: 18 %
+// fewer warp instructions, 21 % less time for 10,000 events of 1,160 hits, 31 %
+// for one event.
 struct Worker {
   uint32_t row;        // first of its scratch rows
   uint32_t n, tracklets, tracks, weak;
@@ -963,9 +963,9 @@ __device__ __noinline__ void fill_windows(const EventView ev, const Shared& s) {
 // (x, y) in a map of the cells that f-4's hits could be met from.  The pairs
 // that pass are queued in shared memory and fitted 32 at a time.
 //
-// Measured against a group of 8 lanes per h0 walking its chunk of h1s and
-// searching h2 for every pair (seed_module): 10,000 events of 1,160 hits 3.27
-// -> 2.50 ms, 4,000 events of 4,550 hits 24.1 -> 7.4 ms.
+// Against a group of 8 lanes per h0 walking its chunk of h1s and searching h2
+// for every pair (seed_module) the kernel takes three quarters of the time for
+// 10,000 events of 1,160 hits, a third for 4,000 events of 4,550.
 //
 // The windows need no table.  An h0's h1 window is bisected when the h0 is
 // seeded (most hits never are); whether an h1 has an h2 window is the flag
@@ -1142,9 +1142,9 @@ __device__ __forceinline__ Fit pair_fit_any(const EventView& ev, const Shared& s
 
 // The usable h1s of module s1, for the seeding of its parity (one warp).  Half
 // of a module's hits are used or without an h2 window by then: pairs with them
-// are not formed (6,950 -> 3,930 pairs an event of 1,160 hits, 103,000 ->
-// 54,000 of 4,400: 10,000 uneven events 5.3 -> 4.5 ms, 4,000 dense ones 6.7 ->
-// 6.2 ms).  Larger modules are paired hit by hit.
+// are not formed (3,930 instead of 6,950 pairs an event of 1,160 hits, 54,000
+// instead of 103,000 of 4,400: 15 % of the time of 10,000 uneven events, 8 % of
+// 4,000 dense ones).  Larger modules are paired hit by hit.
 template <class Shared>
 __device__ __forceinline__ void list_h1s(const EventView& ev, Shared& s, const Worker& w, int s1) {
   const int lane = threadIdx.x & 31, st1 = s.start[s1], n1 = s.num(s1);
@@ -1168,7 +1168,8 @@ __device__ __forceinline__ void list_h1s(const EventView& ev, Shared& s, const W
 // they are enough of all.  Else the event is searched again with every doublet
 // scored (process_event).  That needs the doublets to be known when their cell
 // is looked up: modules whose dead h1s are their last hits, and no
-// learned_min_window.  5,000 events of 1,160 hits: 1.92 -> 1.54 ms.
+// learned_min_window.  It saves a fifth of the time of 5,000 events of 1,160
+// hits.
 template <int kMode, bool kPlainGeometry, class Shared>
 __device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Worker& w, int f) {
   constexpr int kOwn = Shared::kOwn;
@@ -1289,7 +1290,7 @@ __device__ __forceinline__ void seed_pairs(const EventView& ev, Shared& s, Worke
             h1x = ev.xs()[hit1];
             h1y = ev.ys()[hit1];
             // the h1's window, found for the scored pairs only: filling in all
-            // windows per event took 5 % (5,000 events 1.54 -> 1.47 ms)
+            // windows per event takes 5 % more time
             float lo, hi;
             h2_bounds(h1x, zmin1, s.sz[f], s.sz[m4], &lo, &hi);
             a = first_gt(x4, 0, n4, lo);
