@@ -1577,7 +1577,9 @@ __device__ __forceinline__ Worker module_loop(const EventView& ev, Shared& s, Wo
 // registers, and behind one call of the kernel, so that what they need is none
 // of the kernel's concern (called from it directly, they moved its spills: 1.67
 // -> 1.73 ms for 10,000 events that never call them).  With the two seedings in
-// one loop, events of several z per module ran 5 to 10 % slower.
+// one loop, events of several z per module ran 5 to 10 % slower.  (The dump's
+// kernel has the walked loop only, in place: 3,000 events 1.83 ms, 2.21 through
+// these calls.)
 template <int kMode, int kLanes, bool kPlainGeometry, bool kPairs, class Shared>
 __device__ __noinline__ Worker module_loop_any(const EventView& ev, Shared& s, Worker w) {
   return module_loop<kMode, kLanes, kPlainGeometry, kPairs>(ev, s, w);
@@ -1585,11 +1587,12 @@ __device__ __noinline__ Worker module_loop_any(const EventView& ev, Shared& s, W
 
 template <int kMode, int kLanes, class Shared>
 __device__ __noinline__ Worker module_loop_other(const EventView ev, Shared& s, Worker w, bool learned) {
-  constexpr int kOther = kMode == kDump ? kDump : kPlain;
-  if (kMode == kDump || !ev.tame || (learned && !ev.plain))
+  if (!ev.tame || (learned && !ev.plain))
     return learned ? module_loop_any<kMode, kLanes, false, false>(ev, s, w)
-                   : module_loop_any<kOther, kLanes, false, false>(ev, s, w);
+                   : module_loop_any<kPlain, kLanes, false, false>(ev, s, w);
   if (!ev.plain) return module_loop_any<kPlain, kLanes, false, true>(ev, s, w);
+  // the plain search of an event that the learned one gave up (other kernels do
+  // not get here; without the call their registers fall otherwise: +1 %)
   return module_loop_any<kPlain, kLanes, true, true>(ev, s, w);
 }
 
@@ -1795,9 +1798,11 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
       w.n = w.tracklets = w.tracks = w.weak = 0;
       __syncthreads();
     }
-    if (kMode == kDump || !ev.plain || (kMode == kLearned && !learned))
+    if constexpr (kMode == kDump)
+      w = module_loop<kDump, kLanes, false, false>(ev, s, w);
+    else if (!ev.plain || (kMode == kLearned && !learned))
       w = module_loop_other<kMode, kLanes>(ev, s, w, learned);
-    else if constexpr (kMode != kDump)
+    else
       w = module_loop<kMode, kLanes, true, true>(ev, s, w);
     VELO_PHASE(4);
 
