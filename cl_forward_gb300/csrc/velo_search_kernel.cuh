@@ -1585,19 +1585,25 @@ __device__ __noinline__ Worker module_loop_any(const EventView& ev, Shared& s, W
   return module_loop<kMode, kLanes, kPlainGeometry, kPairs>(ev, s, w);
 }
 
-template <int kMode, int kLanes, class Shared>
-__device__ __noinline__ Worker module_loop_other(const EventView ev, Shared& s, Worker w, bool learned) {
-  if (!ev.tame || (learned && !ev.plain))
-    return learned ? module_loop_any<kMode, kLanes, false, false>(ev, s, w)
-                   : module_loop_any<kPlain, kLanes, false, false>(ev, s, w);
+template <int kLanes, class Shared>
+__device__ __noinline__ Worker module_loop_other(const EventView ev, Shared& s, Worker w) {
+  if (!ev.tame) return module_loop_any<kPlain, kLanes, false, false>(ev, s, w);
   if (!ev.plain) return module_loop_any<kPlain, kLanes, false, true>(ev, s, w);
   // never taken; without the call the ordinary loop's registers are dealt out
   // otherwise (10,000 events 1.67 -> 1.69 ms)
   return module_loop_any<kPlain, kLanes, true, true>(ev, s, w);
 }
 
+// The same for the learned build, of plain geometry neither.
+template <int kLanes, class Shared>
+__device__ __noinline__ Worker module_loop_learned(const EventView ev, Shared& s, Worker w, bool learned) {
+  if (learned) return module_loop_any<kLearned, kLanes, false, false>(ev, s, w);
+  return ev.tame ? module_loop_any<kPlain, kLanes, false, true>(ev, s, w)
+                 : module_loop_any<kPlain, kLanes, false, false>(ev, s, w);
+}
+
 // The plain search of an event that the learned one gave up, called directly
-// (5,000 events that all fall back 1.07 ms, 1.15 behind the other call).
+// (5,000 events that all fall back 1.10 ms, 1.15 behind the other call).
 template <int kLanes, class Shared>
 __device__ __noinline__ Worker module_loop_fallback(const EventView ev, Shared& s, Worker w) {
   return module_loop<kPlain, kLanes, true, true>(ev, s, w);
@@ -1809,8 +1815,10 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
       w = module_loop<kDump, kLanes, false, false>(ev, s, w);
     else if (kMode == kLearned && ev.plain && !learned)
       w = module_loop_fallback<kLanes>(ev, s, w);
+    else if (kMode == kLearned && !ev.plain)
+      w = module_loop_learned<kLanes>(ev, s, w, learned);
     else if (!ev.plain)
-      w = module_loop_other<kMode, kLanes>(ev, s, w, learned);
+      w = module_loop_other<kLanes>(ev, s, w);
     else
       w = module_loop<kMode, kLanes, true, true>(ev, s, w);
     VELO_PHASE(4);
@@ -1917,9 +1925,9 @@ __device__ void process_event(const SearchParams& p, int e, Shared& s, uint8_t* 
 // warps), 64-thread CTAs with 56 registers (18 CTAs per SM, register_ctas 18),
 // and 512-thread CTAs; the learned mode in a build of up to 256 threads with
 // 80 registers (3 resident CTAs) and one of up to 64 threads whose bound of 11
-// CTAs leaves the same 80 registers, and 12 CTAs fit (5,000 events 1.43 ms;
-// bounds of 12, 10 and 16: 1.47, 1.47 and 1.61; with the scorer out of line
-// 1.75); each for one seeding width kLanes (lanes per h0 where the windows are
+// CTAs leaves the same 80 registers, and 12 CTAs fit (5,000 events 1.43 ms, 1.44
+// with a bound of 12; a bound of 16 takes an eighth more, the scorer out of line
+// a fifth); each for one seeding width kLanes (lanes per h0 where the windows are
 // walked).
 template <int kMaxThreads, int kMinCtas, int kMode, int kMods, int kLanes>
 __global__ void __launch_bounds__(kMaxThreads, kMinCtas) search_kernel(const __grid_constant__ SearchParams p) {
