@@ -836,7 +836,7 @@ def gpu_arm(args, ranks: Ranks):
                      "algorithmic_bytes": alg_bytes, "peak_source": peak_src,
                      "note": "algorithmic bytes = input blobs + 4 B count + 100 B per track",
                      "limiter": ("not HBM: a latency- and issue-bound search (the ncu capture in "
-                                 "traffic_source: ~64% of issue slots busy, DRAM ~7%, L2 ~11%, L1 hit rate "
+                                 "traffic_source: ~65% of issue slots busy, DRAM ~7%, L2 ~11%, L1 hit rate "
                                  "~73%)")},
         "clocks": clk.summary(),
         "gpu_launches": launches,
