@@ -43,8 +43,9 @@ def _event(seed, n_modules, scale, shift, exact):
     noise = 0.0 if exact else 0.012
     x = scale * (x0[line] + tx[line] * z[m] + rng.normal(0, noise, len(m))) + shift
     y = scale * (y0[line] + ty[line] * z[m] + rng.normal(0, noise, len(m)))
-    ev = Event(np.trunc(z).astype(np.int32), (np.cumsum(num) - num).astype(np.int32), num.astype(np.int32), ((np.arange(len(m)) << 8) | m).astype(np.uint32),
-               x.astype(np.float32), y.astype(np.float32), z[m].astype(np.float32))
+    ev = Event(np.trunc(z).astype(np.int32), (np.cumsum(num) - num).astype(np.int32), num.astype(np.int32),
+               ((np.arange(len(m)) << 8) | m).astype(np.uint32), x.astype(np.float32), y.astype(np.float32),
+               z[m].astype(np.float32))
     return pack_event(ev), line
 
 
